@@ -157,8 +157,6 @@ void compress_pass(Engine &e) {
 // either order give the same list and the same counts.  With profiling on
 // they run one after the other on the step's stream.
 void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
-    stage(e, K_REHASH, [&] { launch_rehash(e, e.stream); });
-    stage(e, K_BEGIN, [&] { launch_begin(e, e.stream); });
     stage(e, K_SWEEP, [&] { launch_sweep(e, e.stream); });
     stage(e, K_EXPAND, [&] { launch_expand(e, e.stream); });
     stage(e, K_SPAWN, [&] { launch_spawn(e, e.stream); });
@@ -784,6 +782,8 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaStreamSynchronize(e.stream));
     int err = 0;
     CK(cudaMemcpy(&err, &e.st.ctl->err, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemset(&e.st.ctl->err, 0, sizeof(int)));
+    e.compact_due = e.rehash_due = false;  // the list and its hash are new
     if (err) return fail(err, "upload: hash table full");
     drop_graphs(e);
     return NECI_GPU_OK;
@@ -881,9 +881,17 @@ static void update_compact_due(Engine &e, const neci_gpu_iter_stats &last) {
     e.compact_due = last.tot_walkers > 4ll * kCompactTile && 2 * last.holes_in_list > last.tot_walkers;
 }
 static void compact_if_due(Engine &e, cudaStream_t s) {
-    if (!e.compact_due) return;
-    stage(e, K_COMPACT, [&] { launch_compact(e, s); });
-    e.compact_due = false;
+    if (e.compact_due) stage(e, K_COMPACT, [&] { launch_compact(e, s); });
+    // after a compaction, or when the last step left the table over its load
+    if (e.compact_due || e.rehash_due) stage(e, K_REHASH, [&] { launch_rehash(e, s); });
+    e.compact_due = e.rehash_due = false;
+}
+
+// The last record of a call: its `reserved` says that the walker hash is to
+// be rebuilt before the next step (the kernels check the device's own flag).
+static void take_rehash(Engine &e, neci_gpu_iter_stats *stats, int n) {
+    e.rehash_due = e.rehash_due || (n > 0 && stats[n - 1].reserved != 0);
+    for (int i = 0; i < n; ++i) stats[i].reserved = 0;
 }
 
 static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_gpu_iter_stats *stats,
@@ -891,6 +899,7 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
     if (const char *why = not_ready(e)) return fail(NECI_GPU_ERR_INVALID, why);
     if (p->tau <= 0.0 || p->av_mc_excits <= 0.0) return fail(NECI_GPU_ERR_INVALID, "tau and AvMCExcits must be positive");
     copy_params(*e.h_params, *p);
+    e.h_params->iter_end = p->iter + n_iter;
     CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e.stream));
     compact_if_due(e, e.stream);
     int done = 0;
@@ -916,6 +925,7 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
             *device_ms += ms;
         }
         std::memcpy(stats + done, e.h_stats, sizeof(neci_gpu_iter_stats) * batch);
+        take_rehash(e, stats + done, batch);
         for (int i = 0; i < batch; ++i)
             if (stats[done + i].err) {
                 done += i + 1;
@@ -971,6 +981,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
     for (int c = 0; c < n_ctx; ++c) {
         Engine &e = ctxs[c]->e;
         copy_params(*e.h_params, params[c]);
+        e.h_params->iter_end = params[c].iter + n_iter;
         const unsigned long long v = e.graph_version * 8 + (e.h_params->precision == NECI_PREC_MIXED ? 4 : 0) +
                                      (sweep_fast(*e.h_params) ? 2 : 0) + (e.st.n_core > 0 ? 1 : 0);
         key.push_back({(const void *)ctxs[c], v});
@@ -1034,6 +1045,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
     for (int c = 0; c < n_ctx; ++c) {
         Engine &e = ctxs[c]->e;
         std::memcpy(stats + (size_t)c * n_iter, e.h_stats, sizeof(neci_gpu_iter_stats) * n_iter);
+        take_rehash(e, stats + (size_t)c * n_iter, n_iter);
         for (int i = 0; i < n_iter && !first_err; ++i) first_err = e.h_stats[i].err;
         if (!first_err) {
             update_fuse_probe(e, e.h_stats[n_iter - 1]);
@@ -1078,6 +1090,7 @@ int32_t neci_gpu_annihilate(neci_gpu_ctx *ctx, const neci_gpu_iter_params *p, co
     CK(cudaStreamSynchronize(e.stream));
     *stats = e.h_stats[0];
     stats->n_spawned = n;
+    take_rehash(e, stats, 1);
     if (stats->err) return fail(stats->err, "device reported an error in the annihilation");
     return NECI_GPU_OK;
 }
@@ -1113,6 +1126,7 @@ int32_t neci_gpu_compress_spawns(neci_gpu_ctx *ctx, const int64_t *spawned, int6
     Control c{};
     CK(cudaMemcpyAsync(&hn, d_n, sizeof(hn), cudaMemcpyDeviceToHost, e.stream));
     CK(cudaMemcpyAsync(&c, e.st.ctl, sizeof(Control), cudaMemcpyDeviceToHost, e.stream));
+    launch_begin(e, e.stream);  // the counters of the next step
     CK(cudaStreamSynchronize(e.stream));
     std::vector<long long> rows((size_t)hn * R);
     if (hn) CK(cudaMemcpyAsync(rows.data(), d_out, (size_t)hn * R * 8, cudaMemcpyDeviceToHost, e.stream));

@@ -66,7 +66,9 @@ struct Control {
     int err;
     int halted;                         // status of a failed step: later steps do nothing until
                                         // the walker list is uploaded again
-    int rehash;                         // rebuild the walker hash at the next step
+    int rehash;                         // rebuild the walker hash before the next step (k_hash_clear,
+                                        // k_hash_fill)
+    int rehash_fill;                    // k_final cleared the walker hash: this step's sweep refills it
     int compact;                        // compact the walker list at the next step
     unsigned long long compact_k;       // occupied slots kept by the compaction
     unsigned long long compact_pos_k;   // occupied slots below compact_k
@@ -289,6 +291,7 @@ struct IterParams {
     float f_tau, f_inv_av, f_cutoff, f_inv_cutoff;
     unsigned long long cutoff_q;  // RealSpawnCutoff in fixed point
     int av_unit;                  // AvMCExcits == 1: the spawn count is split in integers
+    long long iter_end;           // the iteration after the call's last one
 };
 
 // The sweep's fast instance serves steps with real coefficients and

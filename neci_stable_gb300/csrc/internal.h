@@ -53,6 +53,7 @@ struct Engine {
     int sort_bpsm = 2;
     int merge_bpsm = 2;  // merge sweep blocks per SM beside the placement (update_merge_blocks)
     bool compact_due = false;  // the last step left more holes than occupied slots
+    bool rehash_due = false;   // ... or the walker hash over its load
     int core_seg_lane = kCoreSegmentPerLane;  // NECI_OPT_CORE_SEGMENT
     cudaStream_t stream = nullptr;
     IterParams *d_params = nullptr;

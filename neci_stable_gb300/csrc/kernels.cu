@@ -3,8 +3,6 @@
 //
 // Iteration pipeline (all grid-stride, fixed grids, so one iteration is a
 // capturable CUDA graph; counts live in device memory):
-//   k_begin        reset per-step counters; rebuild the walker hash if its
-//                  tombstone load is high
 //   k_sweep        loop_over_determinants (:1294-1758) minus the spawn
 //                  attempts: free slots, initiator flags (CalcParentFlag),
 //                  E_proj sums (SumEContrib), number of spawns
@@ -30,7 +28,9 @@
 //   k_merge_stats  deterministic_annihilation + AnnihilateSpawnedParts
 //                  found branch + CalcHashTableStats (load_balancer.fpp:646)
 //                  in one sweep over the slots
-//   k_final        collect estimators into the step's stats record
+//   k_final        collect estimators into the step's stats record, reset the
+//                  per-step counters, clear the walker hash if its load is
+//                  high (the next sweep refills it)
 #include <cstdio>
 #include <type_traits>
 
@@ -43,31 +43,34 @@
 namespace neci {
 
 // ===========================================================================
-// k_begin: per-step reset (single thread) and optional rehash.
+// The per-step counters.  A step finds them reset: k_final resets them behind
+// every step (one launch fewer than a reset kernel before it, about 4 us of a
+// small system's step), and k_begin for the entry points that end without a
+// k_final.
 // ===========================================================================
+__device__ inline void reset_counters(Control *c) {
+    c->n_free = 0; c->free_taken = 0; c->n_att = 0; c->n_spawned = 0; c->n_cand = 0;
+    c->n_reps = 0; c->n_new = 0; c->n_attempts = 0; c->n_occupied = 0; c->n_holes = 0; c->n_found = 0;
+    c->n_reps_nz = 0;
+    c->n_big = 0;
+    c->n_huge = 0;
+    c->n_long = 0;
+    c->n_place = 0;
+    for (int k = 0; k < 2; ++k) {
+        c->abs_q[k] = 0; c->abs_s[k] = 0;
+        c->nborn[k] = c->ndied[k] = c->nannihil[k] = c->naborted[k] = c->nremoved[k] = 0.0;
+        c->tot_parts[k] = c->tot_parts_old[k] = c->noat_hf[k] = c->hf_cyc[k] = c->enum_cyc[k] = c->norm[k] = 0.0;
+    }
+    c->err = 0;
+}
 __global__ void k_begin(DevState st) {
     Control *c = st.ctl;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !c->halted) {
-        c->n_free = 0; c->free_taken = 0; c->n_att = 0; c->n_spawned = 0; c->n_cand = 0;
-        c->n_reps = 0; c->n_new = 0; c->n_attempts = 0; c->n_occupied = 0; c->n_holes = 0; c->n_found = 0;
-        c->n_reps_nz = 0;
-        c->n_big = 0;
-        c->n_huge = 0;
-        c->n_long = 0;
-        c->n_place = 0;
-        c->n_pre = c->tot_walkers;
-        for (int k = 0; k < 2; ++k) {
-            c->abs_q[k] = 0; c->abs_s[k] = 0;
-            c->nborn[k] = c->ndied[k] = c->nannihil[k] = c->naborted[k] = c->nremoved[k] = 0.0;
-            c->tot_parts[k] = c->tot_parts_old[k] = c->noat_hf[k] = c->hf_cyc[k] = c->enum_cyc[k] = c->norm[k] = 0.0;
-        }
-        c->err = 0;
-        c->rehash = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !c->halted) reset_counters(c);
 }
 
-// Rehash: clear every bucket, then reinsert live slots (run only when the
-// tombstone share is high; the flag is decided on the host from n_tomb).
+// Rebuild of the walker hash between two calls (k_final's rule, or a
+// compaction): clear every bucket, then reinsert the occupied slots.  Within
+// a call k_final clears the table and the next sweep refills it.
 __global__ void k_hash_clear(DevState st) {
     if (halted(st)) return;
     if (!st.ctl->rehash) return;
@@ -91,6 +94,13 @@ __global__ void k_hash_fill(DevSys s, DevState st) {
         NECI_FOR_WORDS(w, s.W) d[w] = (unsigned long long)r[w];
         hash_insert(st, j, neci_hash(d, s.W, sh_rh2), st.ctl);
     }
+}
+// Ends a rebuild (the flag stays up until both kernels have seen it); a
+// refill left to the next sweep is done with it.
+__global__ void k_hash_done(DevState st) {
+    if (threadIdx.x != 0 || halted(st) || !st.ctl->rehash) return;
+    st.ctl->rehash = 0;
+    st.ctl->rehash_fill = 0;
 }
 
 // ===========================================================================
@@ -288,6 +298,16 @@ __device__ __noinline__ double death_integer(double fac, double c, unsigned long
     return idie;
 }
 
+// The sweep's part of a rebuild of the walker hash, in the step after k_final
+// cleared it: a slot that stays occupied is inserted again.  Out of line: it
+// runs about once in hundreds of steps.
+__device__ __noinline__ void sweep_reinsert(const DevSys &s, const DevState &st, long long j) {
+    const long long *r = st.dets + j * s.R;
+    unsigned long long d[kMaxWords];
+    NECI_FOR_WORDS(w, s.W) d[w] = (unsigned long long)r[w];
+    (void)hash_insert(st, j, neci_hash(d, s.W, s.random_hash2), st.ctl);
+}
+
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).  FAST: the
 // instance for real coefficients with AvMCExcits = 1 (sweep_fast).  GB300
 // runs FP64 instructions at about one lane per clock per SM (1/128 of the
@@ -300,6 +320,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     const IterParams p = *pp;
     Control *c = st.ctl;
     const long long n = slots_in_use(st);
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->n_pre = (unsigned long long)n;
+    const bool refill = c->rehash_fill != 0;  // the walker hash is empty
     const int W = s.W, R = s.R;
     constexpr int L = LR;
     double acc_old[2] = {0.0, 0.0}, acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0};
@@ -483,14 +505,17 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                     out_zero = out_zero && abs_bits(cp[k]) == 0;
                 }
             } else {
-                hash_remove(st, j);
-                ++acc_tomb;
+                if (!refill) {
+                    hash_remove(st, j);
+                    ++acc_tomb;
+                }
                 r[W + L] = flags | 1ll;  // flag_removed
                 NECI_FOR_RUNS(k, L) r[W + k] = double_to_word(0.0);
             }
         }
         // the signs just written are all zero
         const bool freed = live && occ && !core && out_zero;
+        if (refill && live && (occ || core) && !freed) sweep_reinsert(s, st, j);
         // The round's three appends, free slots, spawn-attempt entries and
         // k_expand's chunks, with one atomic per counter for the whole block
         // (all issued before any result is read): per-warp atomics on these
@@ -1524,10 +1549,12 @@ __global__ void __launch_bounds__(256) k_rdm_diag(DevSys s, DevState st, int use
 // each step's record lands in its own place.
 // split: the merge sweep counted the slots the step began with less the
 // freed ones; the new determinants are occupied, and the freed slots the
-// placement did not fill are holes.
-__global__ void k_final(DevState st, neci_gpu_iter_stats *base, int *pos, int max_out, IterParams *pp,
-                        int advance_iter, long long n_core, int split) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// placement did not fill are holes.  A walker hash whose live entries and
+// tombstones pass 60% of the buckets is rebuilt between two calls (the host
+// is told in `reserved` of the record); within a call, past 70%, it is
+// cleared here (the return value) and the next step's sweep refills it.
+__device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int *pos, int max_out, IterParams *pp,
+                            int advance_iter, long long n_core, int split) {
     neci_gpu_iter_stats *out = base;
     if (pos) {
         const int k = *pos;
@@ -1540,7 +1567,7 @@ __global__ void k_final(DevState st, neci_gpu_iter_stats *base, int *pos, int ma
         neci_gpu_iter_stats r{};
         r.err = c->halted;
         *out = r;
-        return;
+        return 0;
     }
     if (c->tot_walkers > (unsigned long long)st.max_walkers) c->tot_walkers = (unsigned long long)st.max_walkers;
     if (split) {
@@ -1575,16 +1602,35 @@ __global__ void k_final(DevState st, neci_gpu_iter_stats *base, int *pos, int ma
     r.n_new = (long long)c->n_new;
     r.n_core = n_core;
     r.err = c->err;
-    r.reserved = 0;
+    const long long next = pp->iter + 1;
+    if (advance_iter) pp->iter = next;
+    const unsigned long long used = c->n_occupied + c->n_tomb;
+    const bool more = advance_iter && next < pp->iter_end && !c->err;  // another step of the call follows
+    const bool in_call = more && used * 10ull > st.hash_n * 7ull;
+    c->rehash_fill = in_call ? 1 : 0;
+    c->rehash = !more && used * 10ull > st.hash_n * 6ull ? 1 : 0;
+    if (in_call) c->n_tomb = 0;
+    r.reserved = c->rehash;
     *out = r;
-    if (advance_iter) pp->iter += 1;
-    // rebuild the walker hash before the next step when live entries plus
-    // tombstones pass 70% of the buckets
-    c->rehash = (c->n_occupied + c->n_tomb) * 10ull > st.hash_n * 7ull ? 1 : 0;
-    // compact the list before the next step when holes outnumber occupied slots
+    // compact the list before the next call when holes outnumber occupied slots
     c->compact = (c->tot_walkers > (unsigned long long)(4 * kCompactTile) && c->n_holes * 2ull > c->tot_walkers) ? 1 : 0;
     // a failed step halts the ones after it (in the same graph batch)
     if (c->err) c->halted = c->err;
+    reset_counters(c);
+    return in_call ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats *base, int *pos, int max_out,
+                                                IterParams *pp, int advance_iter, long long n_core, int split) {
+    __shared__ int clear;
+    if (threadIdx.x == 0) clear = final_record(st, base, pos, max_out, pp, advance_iter, n_core, split);
+    __syncthreads();
+    if (!clear) return;
+    // one block: within a call a rebuild is due about once in hundreds of
+    // steps, and a grid-wide kernel would cost an idle launch in each of them
+    uint4 *t = reinterpret_cast<uint4 *>(st.hash);
+    for (unsigned long long b = threadIdx.x; b < st.hash_n / 4; b += blockDim.x)
+        t[b] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
 }
 
 // ===========================================================================
@@ -1616,6 +1662,7 @@ void launch_compact(Engine &e, cudaStream_t s) {
 void launch_rehash(Engine &e, cudaStream_t s) {
     k_hash_clear<<<grid_for(e, 256), 256, 0, s>>>(e.st);
     k_hash_fill<<<grid_for(e, 256), 256, (e.sys.nbasis + 1) * sizeof(int32_t), s>>>(e.sys, e.st);
+    k_hash_done<<<1, 32, 0, s>>>(e.st);
 }
 
 // Dynamic shared memory of the staged sweeps: two stages of a tile.
@@ -1735,7 +1782,7 @@ void launch_rdm(Engine &e, cudaStream_t s) {
 }
 
 void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split) {
-    k_final<<<1, 32, 0, s>>>(e.st, out, pos, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
+    k_final<<<1, 1024, 0, s>>>(e.st, out, pos, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
 }
 
 }  // namespace neci

@@ -1,0 +1,82 @@
+"""GPU parity of the forms a step takes at the edges of their ranges, against
+the CPU oracle, bit for bit: the walker hash kept at a high load, where its
+tombstones pile up and it is rebuilt inside a call (cleared behind one step,
+refilled by the next sweep) and between calls."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from neci_stable_gb300 import capi
+from neci_stable_gb300.engine import Engine
+from oracle.oracle import Oracle
+
+from helpers import canonical, hubbard10, molecule
+
+pytestmark = pytest.mark.gpu
+
+
+def same_list(spec, eng, orc, tag):
+    W, L = spec.W, spec.lenof_sign
+    rg, rc = canonical(eng.download()[0], W), canonical(orc.download()[0], W)
+    assert rg.shape == rc.shape, tag
+    assert np.array_equal(rg[:, :W + L], rc[:, :W + L]), tag
+    assert np.array_equal(rg[:, -1] & ~1, rc[:, -1] & ~1), tag
+
+
+def run_both(spec, eng, orc, calls, tau, seed, shift=0.0):
+    """calls[i] steps in the i-th call of the engine, the lists compared
+    after every call and the counts after every step."""
+    it = 1
+    for n in calls:
+        p = capi.default_params(tau=tau, diag_sft=[shift, shift], seed=seed, iter=it)
+        sg = eng.iterate_n(p, n)
+        for k in range(n):
+            q = capi.default_params(tau=tau, diag_sft=[shift, shift], seed=seed, iter=it + k)
+            sc, rc = orc.iterate(q)
+            assert rc == 0 and sg[k].err == 0 and sg[k].reserved == 0, (it + k, rc, sg[k].err)
+            for f in ("n_attempts", "n_spawned", "n_unique", "n_new", "n_occupied"):
+                assert getattr(sg[k], f) == getattr(sc, f), (f, it + k)
+            assert sg[k].n_occupied + sg[k].holes_in_list == sg[k].tot_walkers
+        it += n
+        same_list(spec, eng, orc, it)
+
+
+@pytest.mark.parametrize("lenof_sign", [1, 2])
+@pytest.mark.parametrize("calls", [(400,), (1,) * 200 + (3,) * 60, (150, 1, 7, 150)])
+def test_walker_hash_at_high_load(lenof_sign, calls):
+    # the table's length is 2 max_walkers (a power of two): the list in use
+    # keeps it 0.4 live, and a turnover of 6% a step piles tombstones up
+    spec = hubbard10(lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 12, 1 << 14)
+    orc = Oracle(spec, 1 << 13, 1 << 15, hii=eng.hii)
+    eng.start_from_reference(initial_part=900.0 if lenof_sign == 1 else 840.0)
+    orc.upload(eng.download()[0])
+    run_both(spec, eng, orc, calls, tau=0.02, seed=5, shift=-5.39 if lenof_sign == 1 else -5.4)
+    eng.close()
+
+
+def test_hash_after_entry_points_between_steps():
+    # the counters and the walker hash an entry point finds between two steps
+    spec = molecule(12, 6)
+    eng = Engine(spec, 1 << 14, 1 << 16)
+    orc = Oracle(spec, 1 << 14, 1 << 16, hii=eng.hii)
+    eng.start_from_reference(initial_part=3000.0)
+    orc.upload(eng.download()[0])
+    run_both(spec, eng, orc, (30,), tau=0.01, seed=9)
+    rows = eng.download()[0]
+    sp = rows[::3].copy()
+    sp[:, spec.W:spec.W + 1] = (-sp[:, spec.W:spec.W + 1].view(np.float64)).view(np.int64)
+    for it in (31, 32, 33):
+        p = capi.default_params(tau=0.01, seed=9, iter=it)
+        sg = eng.annihilate(p, sp)
+        sc, rc = orc.annihilate(p, sp)
+        assert rc == 0 and sg.err == 0
+        same_list(spec, eng, orc, it)
+    out_g, _ = eng.compress_spawns(sp)
+    assert out_g.shape[0] == np.unique(sp[:, 0]).size
+    eng.set_core_space(eng.download()[0][:50, :spec.W])
+    gone = np.setdiff1d(rows[:, 0], eng.download()[0][:, 0])
+    if gone.size:
+        with pytest.raises(capi.NeciGpuError):
+            eng.set_core_space(gone[:1, None])
