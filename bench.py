@@ -782,11 +782,11 @@ def main():
     sort_ms = sum(v["ms"] for v in sort_stages.values())
     sort_bytes = sum(v["algorithmic_bytes"] for v in sort_stages.values())
     ktm = {k: v for k, v in r["ktimes_mixed"].items() if v[1] > 0}
-    # sweep, expand, spawn, compress, decide, place, merge, final; the probe
+    # sweep, spawn, compress, decide, place, merge, final; the probe
     # unless the spawn kernel does it; the core projection and the sum of its
     # long rows (a compaction, when a step leaves more holes than walkers, and
     # a rebuild of the walker hash run between calls)
-    launches_per_step = 8 + (2 if r["last"]["n_core"] > 0 else 0) + (0 if fused else 1)
+    launches_per_step = 7 + (2 if r["last"]["n_core"] > 0 else 0) + (0 if fused else 1)
     line = {
         "metric": METRIC, "value": updates / dev_s, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": 1000.0 * dev_s / args.steps, "higher_is_better": True,

@@ -158,7 +158,6 @@ void compress_pass(Engine &e) {
 // they run one after the other on the step's stream.
 void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
     stage(e, K_SWEEP, [&] { launch_sweep(e, e.stream); });
-    stage(e, K_EXPAND, [&] { launch_expand(e, e.stream); });
     stage(e, K_SPAWN, [&] { launch_spawn(e, e.stream); });
     if (e.st.n_core > 0) stage(e, K_CORE, [&] { launch_core(e, e.stream); });
     const int with_core = e.st.n_core > 0 ? 1 : 0;
@@ -294,9 +293,7 @@ int32_t neci_gpu_init(neci_gpu_ctx **out, const neci_gpu_system *sys, int32_t de
     st.max_walkers = sys->max_walkers;
     st.max_spawned = sys->max_spawned;
     st.max_att = 2 * sys->max_spawned + 1024;
-    // a parent with n attempts (kBigAttempts < n <= kHugeAttempts) takes
-    // ceil(n / kExpandChunk) entries, at most n / kBigAttempts + n / kExpandChunk
-    st.max_big = st.max_att / kBigAttempts + st.max_att / kExpandChunk + 1024;
+    st.max_big = st.max_att / kBigAttempts + 1024;
     st.hash_n = next_pow2(std::max<unsigned long long>((unsigned long long)sys->n_walker_hashes,
                                                        2ull * (unsigned long long)sys->max_walkers));
     st.spawn_hash_n = next_pow2(2ull * (unsigned long long)sys->max_spawned);
@@ -318,7 +315,7 @@ int32_t neci_gpu_init(neci_gpu_ctx **out, const neci_gpu_system *sys, int32_t de
     A(st.spawn, (size_t)st.max_spawned * s.R);
     A(st.att, (size_t)st.max_att);
     A(st.big, (size_t)st.max_big * 3);
-    A(st.huge, (size_t)kMaxHuge * 3);
+    A(st.big_at, (size_t)st.max_att / kBigGranule + 1);
     A(st.acc, (size_t)(st.max_walkers + kStagePad) * s.L);
     A(st.meta, (size_t)(st.max_walkers + kStagePad) * s.L);
     A(st.cand, (size_t)st.max_spawned);

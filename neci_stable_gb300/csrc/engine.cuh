@@ -24,9 +24,15 @@ constexpr int kMaxRuns = 2;  // lenof_sign: one run or a replica pair
 #define NECI_FOR_RUNS(k, L) _Pragma("unroll") for (int k = 0; k < kMaxRuns; ++k) if (k < (L))
 constexpr int kMaxNel = 64;
 constexpr int kMaxNeigh = 8;
-constexpr int kBigAttempts = 32;  // parents with more attempts are expanded by k_expand
-constexpr int kHugeAttempts = 1 << 16;  // ... and with more than this by the whole grid
-constexpr int kExpandChunk = 512;  // k_expand's work item: at most this many attempts of one parent
+// A parent with more attempts than this is handed to the spawn kernel as one
+// record instead of an entry per attempt (see heavy_attempt).
+#ifndef NECI_BIG_ATTEMPTS
+#define NECI_BIG_ATTEMPTS 32
+#endif
+constexpr int kBigAttempts = NECI_BIG_ATTEMPTS;
+constexpr int kBigGranule = 128;  // attempts of heavy parents per entry of DevState::big_at
+constexpr int kBigShift = 36;     // Control::n_big: parents << kBigShift | their attempts
+constexpr int kHugeAttempts = 1 << 16;  // at most kMaxHuge parents may have more attempts than this
 constexpr int kMaxHuge = 4096;
 constexpr int kCompactTile = 1024;        // slots per block of the compaction scans
 constexpr int kProbeLimit = 1 << 16;
@@ -56,8 +62,8 @@ struct Control {
     unsigned long long n_found;         // unique spawned determinants already present, with a
                                         // non-zero summed amplitude
     unsigned long long n_reps_nz;       // unique new determinants with a non-zero summed amplitude
-    unsigned long long n_big;           // parents expanded by k_expand
-    unsigned long long n_huge;          // parents expanded by the whole grid
+    unsigned long long n_big;           // heavy parents << kBigShift | their attempts
+    unsigned long long n_huge;          // parents with more than kHugeAttempts attempts
     unsigned long long n_long;          // sort annihilation: runs of equal keys left to k_sk_long
     unsigned long long n_place;         // new determinants k_ann_decide leaves to k_ann_place
     unsigned long long n_pre;           // slots in use before this step's new determinants
@@ -192,9 +198,11 @@ struct DevState {
     long long max_walkers, max_spawned, max_att;
     long long *spawn;              // spawn records
     unsigned long long *att;       // attempts: slot | run << 32 | neg << 33 | attempt << 34
-    unsigned long long *big;       // chunks of at most kExpandChunk attempts of one parent, as triples:
-                                   // slot | run << 32 | neg << 33 | first attempt << 34, attempts, first entry
-    unsigned long long *huge;      // the same for parents with more than kHugeAttempts attempts
+    // heavy parents as triples: slot | run << 32 | neg << 33, the first of
+    // their attempts in the row of all heavy attempts, their number; and for
+    // every kBigGranule-th attempt of that row the parent it belongs to
+    unsigned long long *big;
+    uint32_t *big_at;
     long long max_big;
     long long *acc;                // per slot*L fixed-point spawn sums (found determinants)
     uint32_t *meta;                // per slot*L spawn counts | initiator bit 31

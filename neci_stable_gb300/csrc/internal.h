@@ -14,9 +14,9 @@ namespace neci {
 enum KernelId {
     K_COMPACT = 0,
     K_REHASH,
-    K_BEGIN,
+    K_BEGIN,   // (no stage of its own any more; the ids are part of the ABI)
     K_SWEEP,
-    K_EXPAND,
+    K_EXPAND,  // (as K_BEGIN)
     K_SPAWN,
     K_CORE,
     K_ANN_PROBE,
@@ -39,7 +39,7 @@ struct Engine {
     int num_sms = 152;
     // resident blocks per SM of the grid-stride spawn-list kernels (their
     // grids fill the GPU once; the latency-bound hash passes want every warp)
-    int occ_probe = 4, occ_compress = 4, occ_insert = 4, occ_place = 8, occ_expand = 4;
+    int occ_probe = 4, occ_compress = 4, occ_insert = 4, occ_place = 8;
     // pass 1 of the annihilation runs inside the spawn kernel (chosen from the
     // last step's spawn rate; see update_fuse_probe)
     bool fuse_probe = false;
@@ -106,7 +106,6 @@ void launch_compact(Engine &e, cudaStream_t s);
 void launch_sweep(Engine &e, cudaStream_t s);
 // sets the per-kernel launch attributes a context needs (non-zero: failure)
 int configure_kernels(Engine &e);
-void launch_expand(Engine &e, cudaStream_t s);
 void launch_spawn(Engine &e, cudaStream_t s);
 void launch_core(Engine &e, cudaStream_t s);
 void launch_ann_probe(Engine &e, cudaStream_t s);

@@ -9,7 +9,6 @@
 //                  (decide_num_to_spawn) emitted as one entry per attempt,
 //                  core vector gather, and the death step
 //                  (perform_death_all_walkers / walker_death)
-//   k_expand       attempt entries of heavily populated parents, a block each
 //   k_spawn        the spawn attempts (generate_excitation, attempt_create,
 //                  create_particle): in spawn.cu
 //   k_core         determ_projection_no_death (semi_stoch_procs.F90:290)
@@ -299,13 +298,19 @@ __device__ __noinline__ double death_integer(double fac, double c, unsigned long
 }
 
 // The sweep's part of a rebuild of the walker hash, in the step after k_final
-// cleared it: a slot that stays occupied is inserted again.  Out of line: it
-// runs about once in hundreds of steps.
-__device__ __noinline__ void sweep_reinsert(const DevSys &s, const DevState &st, long long j) {
-    const long long *r = st.dets + j * s.R;
-    unsigned long long d[kMaxWords];
-    NECI_FOR_WORDS(w, s.W) d[w] = (unsigned long long)r[w];
-    (void)hash_insert(st, j, neci_hash(d, s.W, s.random_hash2), st.ctl);
+// cleared it: before a thread sweeps its slots it inserts the occupied ones
+// again (the same thread, so that a removal of the sweep finds its bucket).
+// Out of line: it runs about once in hundreds of steps.
+__device__ __noinline__ void sweep_refill(const DevSys &s, const DevState &st, long long n) {
+    for (long long j = blockIdx.x * (long long)kStageTile + threadIdx.x; j < n; j += (long long)gridDim.x * kStageTile) {
+        const long long *r = st.dets + j * s.R;
+        bool occ = st.n_core > 0 && is_core_flags(r[s.W + s.L]);
+        NECI_FOR_RUNS(k, s.L) occ = occ || abs_bits(word_to_double(r[s.W + k])) >= dbl_bits(kEps12);
+        if (!occ) continue;
+        unsigned long long d[kMaxWords];
+        NECI_FOR_WORDS(w, s.W) d[w] = (unsigned long long)r[w];
+        (void)hash_insert(st, j, neci_hash(d, s.W, s.random_hash2), st.ctl);
+    }
 }
 
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).  FAST: the
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     Control *c = st.ctl;
     const long long n = slots_in_use(st);
     if (blockIdx.x == 0 && threadIdx.x == 0) c->n_pre = (unsigned long long)n;
-    const bool refill = c->rehash_fill != 0;  // the walker hash is empty
+    if (c->rehash_fill) sweep_refill(s, st, n);  // the walker hash is empty
     const int W = s.W, R = s.R;
     constexpr int L = LR;
     double acc_old[2] = {0.0, 0.0}, acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0};
@@ -336,7 +341,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     __shared__ int stage_ok[2];  // by round parity
     // the round's appends: per-warp counts of free slots and attempts, and
     // the block's first positions
-    __shared__ unsigned int s_wfree[kStageTile / 32], s_watt[kStageTile / 32], s_wbig[kStageTile / 32];
+    __shared__ unsigned int s_wfree[kStageTile / 32], s_watt[kStageTile / 32];
+    __shared__ unsigned long long s_wbig[kStageTile / 32];
     __shared__ unsigned long long s_base_free, s_base_att, s_base_big;
     const size_t stage_bytes = (size_t)kStageTile * (R + 2) * 8;
     if (threadIdx.x == 0) {
@@ -505,43 +511,49 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                     out_zero = out_zero && abs_bits(cp[k]) == 0;
                 }
             } else {
-                if (!refill) {
-                    hash_remove(st, j);
-                    ++acc_tomb;
-                }
+                hash_remove(st, j);
+                ++acc_tomb;
                 r[W + L] = flags | 1ll;  // flag_removed
                 NECI_FOR_RUNS(k, L) r[W + k] = double_to_word(0.0);
             }
         }
         // the signs just written are all zero
         const bool freed = live && occ && !core && out_zero;
-        if (refill && live && (occ || core) && !freed) sweep_reinsert(s, st, j);
         // The round's three appends, free slots, spawn-attempt entries and
-        // k_expand's chunks, with one atomic per counter for the whole block
+        // heavy parents, with one atomic per counter for the whole block
         // (all issued before any result is read): per-warp atomics on these
         // addresses serialise in one L2 slice, tens of thousands to millions
         // per step.  One entry per attempt; a parent with more than
-        // kBigAttempts attempts is handed to k_expand in chunks of at most
-        // kExpandChunk attempts, each written by a warp there.
+        // kBigAttempts attempts is one record, whose attempts the spawn
+        // kernel numbers itself (heavy_attempt).
         {
             const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
             const bool want = hole || freed;
             if (live) st.hole_mark[j] = want ? 1 : 0;
             const unsigned int mf = __ballot_sync(0xffffffffu, want);
-            unsigned int nat = 0, nbig = 0;
+            unsigned int nat = 0;  // attempts written as entries
+            bool heavy = false;
             NECI_FOR_RUNS(k, L) {
-                nat += nsp[k];
-                if (nsp[k] > (unsigned int)kBigAttempts && nsp[k] <= (unsigned int)kHugeAttempts)
-                    nbig += (nsp[k] + kExpandChunk - 1) / kExpandChunk;
+                if (nsp[k] > (unsigned int)kBigAttempts) heavy = true;
+                else nat += nsp[k];
             }
-            unsigned int incl = nat, bincl = nbig;  // inclusive scans of the warp's attempts and chunks
+            unsigned int incl = nat;  // inclusive scan of the warp's entries
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
-                const unsigned int z = __shfl_up_sync(0xffffffffu, bincl, o);
-                if (lane >= o) {
-                    incl += y;
-                    bincl += z;
+                if (lane >= o) incl += y;
+            }
+            const unsigned int mb = __ballot_sync(0xffffffffu, heavy);
+            // heavy runs << kBigShift | their attempts: this lane's, and the
+            // warp's inclusive scan
+            unsigned long long big = 0, bincl = 0;
+            if (mb) {
+                NECI_FOR_RUNS(k, L) if (nsp[k] > (unsigned int)kBigAttempts) big += (1ull << kBigShift) + nsp[k];
+                bincl = big;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long z = __shfl_up_sync(0xffffffffu, bincl, o);
+                    if (lane >= o) bincl += z;
                 }
             }
             if (lane == 31) {
@@ -551,7 +563,8 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             }
             __syncthreads();
             if (threadIdx.x == 0) {
-                unsigned int tf = 0, ta = 0, tb = 0;
+                unsigned int tf = 0, ta = 0;
+                unsigned long long tb = 0;
                 for (int w = 0; w < kStageTile / 32; ++w) {
                     tf += s_wfree[w];
                     ta += s_watt[w];
@@ -559,62 +572,65 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                 }
                 s_base_free = tf ? atomicAdd(&c->n_free, (unsigned long long)tf) : 0ull;
                 s_base_att = ta ? atomicAdd(&c->n_att, (unsigned long long)ta) : 0ull;
-                s_base_big = tb ? atomicAdd(&c->n_big, (unsigned long long)tb) : 0ull;
+                s_base_big = tb ? atomicAdd(&c->n_big, tb) : 0ull;
             }
             __syncthreads();
-            unsigned long long bf = s_base_free, ba = s_base_att, bb = s_base_big;
+            unsigned long long bf = s_base_free, ba = s_base_att;
             for (int w = 0; w < wid; ++w) {
                 bf += s_wfree[w];
                 ba += s_watt[w];
-                bb += s_wbig[w];
             }
             if (want) st.free_list[bf + __popc(mf & ((1u << lane) - 1u))] = (int32_t)j;
-            const unsigned long long base = ba + incl - nat;
-            // this lane's chunks for k_expand: every entry below max_big is
-            // written (with no attempts where the lane's entries do not fit),
-            // so that k_expand reads none from an earlier step
-            if (nbig) {
-                unsigned long long cb = bb + bincl - nbig;
-                const bool fits = base + nat <= (unsigned long long)st.max_att;
-                if (cb + nbig > (unsigned long long)st.max_big) set_err(c, NECI_GPU_ERR_SPAWN_FULL);
-                unsigned long long q = base;
+            if (mb) {
+                // Records and attempts of the heavy parents are counted by
+                // one atomic, so the records lie in the order of their
+                // attempts.  The granules that start in a parent's range are
+                // marked with its record, those of a parent with many by the
+                // whole warp.
+                unsigned long long at = s_base_big + bincl - big;
+                for (int w = 0; w < wid; ++w) at += s_wbig[w];
+                const uint32_t gmax = (uint32_t)((unsigned long long)st.max_att / kBigGranule + 1);
                 NECI_FOR_RUNS(k, L) {
-                    if (nsp[k] > (unsigned int)kBigAttempts && nsp[k] <= (unsigned int)kHugeAttempts) {
-                        const unsigned long long head = (unsigned long long)j | ((unsigned long long)k << 32) |
-                                                        ((unsigned long long)neg[k] << 33);
-                        for (unsigned int a0 = 0; a0 < nsp[k] && cb < (unsigned long long)st.max_big;
-                             a0 += kExpandChunk, ++cb) {
-                            st.big[3 * cb] = head | ((unsigned long long)a0 << 34);
-                            st.big[3 * cb + 1] = fits ? min((unsigned int)kExpandChunk, nsp[k] - a0) : 0u;
-                            st.big[3 * cb + 2] = q + a0;
+                    const bool heavy = nsp[k] > (unsigned int)kBigAttempts;
+                    const unsigned long long rec = at >> kBigShift, first = at & ((1ull << kBigShift) - 1);
+                    uint32_t g0 = 0, g1 = 0;
+                    if (heavy) {
+                        at += (1ull << kBigShift) + nsp[k];
+                        if (rec < (unsigned long long)st.max_big) {
+                            st.big[3 * rec] = (unsigned long long)j | ((unsigned long long)k << 32) |
+                                              ((unsigned long long)neg[k] << 33);
+                            st.big[3 * rec + 1] = first;
+                            st.big[3 * rec + 2] = nsp[k];
+                            g0 = (uint32_t)((first + kBigGranule - 1) / kBigGranule);
+                            g1 = min((uint32_t)((first + nsp[k] + kBigGranule - 1) / kBigGranule), gmax);
+                        } else {
+                            set_err(c, NECI_GPU_ERR_SPAWN_FULL);
                         }
+                        if (nsp[k] > (unsigned int)kHugeAttempts && atomicAdd(&c->n_huge, 1ull) >= kMaxHuge)
+                            set_err(c, NECI_GPU_ERR_SPAWN_FULL);
                     }
-                    q += nsp[k];
+                    const bool many = g1 > g0 + 8;
+                    if (!many)
+                        for (; g0 < g1; ++g0) st.big_at[g0] = (uint32_t)rec;
+                    for (unsigned int m = __ballot_sync(0xffffffffu, many); m; m &= m - 1) {
+                        const int from = __ffs(m) - 1;
+                        const uint32_t e1 = __shfl_sync(0xffffffffu, g1, from);
+                        const uint32_t rr = __shfl_sync(0xffffffffu, (uint32_t)rec, from);
+                        for (uint32_t g = __shfl_sync(0xffffffffu, g0, from) + lane; g < e1; g += 32) st.big_at[g] = rr;
+                    }
                 }
             }
             if (nat) {
-                if (base + nat > (unsigned long long)st.max_att) {
+                unsigned long long q = ba + incl - nat;
+                if (q + nat > (unsigned long long)st.max_att) {
                     set_err(c, NECI_GPU_ERR_SPAWN_FULL);
                 } else {
-                    unsigned long long q = base;
                     NECI_FOR_RUNS(k, L) {
                         const unsigned long long head = (unsigned long long)j | ((unsigned long long)k << 32) |
                                                         ((unsigned long long)neg[k] << 33);
-                        if (nsp[k] > (unsigned int)kHugeAttempts) {
-                            const unsigned long long b = atomicAdd(&c->n_huge, 1ull);
-                            if (b < (unsigned long long)kMaxHuge) {
-                                st.huge[3 * b] = head;
-                                st.huge[3 * b + 1] = nsp[k];
-                                st.huge[3 * b + 2] = q;
-                            } else {
-                                set_err(c, NECI_GPU_ERR_SPAWN_FULL);
-                            }
-                        } else if (nsp[k] > (unsigned int)kBigAttempts) {
-                            // its chunks for k_expand are written above
-                        } else {
-                            for (unsigned int a = 0; a < nsp[k]; ++a) st.att[q + a] = head | ((unsigned long long)a << 34);
-                        }
-                        q += nsp[k];
+                        const unsigned int m = nsp[k] > (unsigned int)kBigAttempts ? 0u : nsp[k];
+                        for (unsigned int a = 0; a < m; ++a) st.att[q + a] = head | ((unsigned long long)a << 34);
+                        q += m;
                     }
                 }
             }
@@ -638,35 +654,6 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             b = y > b ? y : b;
         }
         if ((threadIdx.x & 31) == 0 && b) atomicMax(&c->tau_death, b);
-    }
-}
-
-// ===========================================================================
-// k_expand: attempt entries of heavily populated parents, one warp per chunk
-// of at most kExpandChunk attempts of a parent (the whole grid per parent for
-// the few with more than kHugeAttempts).
-// ===========================================================================
-__global__ void k_expand(DevState st) {
-    if (halted(st)) return;
-    // parents with more than kHugeAttempts attempts: the whole grid per parent
-    const unsigned long long nh = min(st.ctl->n_huge, (unsigned long long)kMaxHuge);
-    for (unsigned long long b = 0; b < nh; ++b) {
-        const unsigned long long head = st.huge[3 * b], n = st.huge[3 * b + 1], base = st.huge[3 * b + 2];
-        for (unsigned long long a = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; a < n;
-             a += (unsigned long long)gridDim.x * blockDim.x)
-            st.att[base + a] = head | (a << 34);
-    }
-    // the others (33 to 65536 attempts): a warp per chunk; the chunk's head
-    // carries its first attempt index, so its entry a is head + (a << 34)
-    const unsigned long long nb = min(st.ctl->n_big, (unsigned long long)st.max_big);
-    const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
-    const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-    const unsigned long long lane = threadIdx.x & 31;
-    for (unsigned long long b = warp; b < nb; b += nwarps) {
-        const unsigned long long head = st.big[3 * b];
-        const unsigned long long n = st.big[3 * b + 1];
-        const unsigned long long base = st.big[3 * b + 2];
-        for (unsigned long long a = lane; a < n; a += 32) st.att[base + a] = head + (a << 34);
     }
 }
 
@@ -1699,7 +1686,6 @@ int configure_kernels(Engine &e) {
     e.occ_compress = occ((const void *)k_ann_compress<1>, (const void *)k_ann_compress<2>, 256, 0);
     e.occ_insert = occ((const void *)k_ann_decide<1>, (const void *)k_ann_decide<2>, 256, 0);
     e.occ_place = occ((const void *)k_ann_place<1>, (const void *)k_ann_place<2>, 128, 0);
-    e.occ_expand = occ((const void *)k_expand, (const void *)k_expand, 256, 0);
     (void)cudaGetLastError();
     return 0;
 }
@@ -1716,7 +1702,6 @@ void launch_sweep(Engine &e, cudaStream_t s) {
         else k_sweep<1, false><<<grid, kStageTile, shm, s>>>(e.sys, e.st, e.d_params);
     }
 }
-void launch_expand(Engine &e, cudaStream_t s) { k_expand<<<grid_spawns(e, 256, e.occ_expand), 256, 0, s>>>(e.st); }
 template <int G>
 static void launch_core_g(Engine &e, cudaStream_t s) {
     const int grid = clamp_grid(e.st.n_core_seg * G / 256 + 1, e.num_sms * 8);

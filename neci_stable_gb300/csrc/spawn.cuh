@@ -102,6 +102,24 @@ __device__ inline Stream attempt_stream(const DevState &st, const IterParams &p,
     return Stream(st.dkey[j], p.iter, P_ATTEMPT, (uint32_t)((w0 >> 32) & 1ull), (uint32_t)(w0 >> 34));
 }
 
+// Attempt v of the row of all attempts of heavy parents, as an entry: its
+// parent is the one noted for its granule or one of the next few (a heavy
+// parent has more than kBigAttempts attempts).  The parents with hundreds or
+// thousands of attempts so cost one record each, not an entry per attempt
+// written and read, and no kernel to write them (that kernel took 19 us of
+// 906 per step at n = 24 with 1e7 walkers, and 5 us of an idle step).
+__device__ inline unsigned long long heavy_attempt(const DevState &st, unsigned long long v) {
+    const unsigned long long n_big = min(st.ctl->n_big >> kBigShift, (unsigned long long)st.max_big);
+    const unsigned long long *b = st.big + 3ull * st.big_at[v / kBigGranule], *last = st.big + 3 * n_big - 3;
+    while (b < last && v - b[1] >= b[2]) b += 3;
+    return b[0] + ((v - b[1]) << 34);
+}
+// The entry of attempt q: the sweep's n_entry entries come first, then the
+// heavy parents' attempts.
+__device__ inline unsigned long long attempt_entry(const DevState &st, long long q, const volatile long long &n_entry) {
+    return q < n_entry ? st.att[q] : heavy_attempt(st, (unsigned long long)(q - n_entry));
+}
+
 // Block-local tau-search log of k_spawn: per TauClass the largest gamma (as
 // bits) and the logged count, capped near the reference's threshold.
 struct TauAcc {
@@ -290,6 +308,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     __shared__ int wcnt[2][2][4];
     __shared__ unsigned int ring_tail;
     __shared__ unsigned long long sh_sums[3];
+    __shared__ long long sh_n[2];
     __shared__ TauAcc tacc;
     int32_t *sh_rh2 = sh;
     int32_t *sh_neigh = sh + (s.nbasis + 1);
@@ -304,7 +323,18 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     if (threadIdx.x < 3) sh_sums[threadIdx.x] = 0ull;
     __syncthreads();
     const IterParams p = *pp;
-    const long long nat = (long long)min(st.ctl->n_att, (unsigned long long)st.max_att);
+    // attempts in all; sh_n[0] of them have entries (kept in shared memory:
+    // the loops below are short of registers)
+    if (threadIdx.x == 0) {
+        const unsigned long long na = st.ctl->n_att, cap = (unsigned long long)st.max_att;
+        const unsigned long long nh = st.ctl->n_big & ((1ull << kBigShift) - 1);
+        if (na + nh > cap) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        sh_n[0] = (long long)min(na, cap);
+        sh_n[1] = sh_n[0] + (long long)min(nh, cap);
+    }
+    __syncthreads();
+    const volatile long long &n_entry = sh_n[0];
+    const long long nat = sh_n[1];
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long nround = ((nat + stride - 1) / stride) * stride;
     const int nb = blockDim.x;  // 128: four warps
@@ -322,7 +352,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
             Excit<Real> e;
             e.ok = false;
             if (q < nat) {
-                load_parent<NW, RW>(s, st, p, st.att[q], P);
+                load_parent<NW, RW>(s, st, p, attempt_entry(st, q, n_entry), P);
                 Stream rng(P.key, p.iter, P_ATTEMPT, P.run, P.k);
                 gen_rs_hubbard<Real, NW>(s, P.d, sh_neigh, rng, e);
                 qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, sh_rh2, ovf, &tacc);
@@ -358,7 +388,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                 e.ok = false;
                 long long qv = 0;
                 if (q < nat) {
-                    w0 = st.att[q];
+                    w0 = attempt_entry(st, q, n_entry);
                     load_parent<NW, RW>(s, st, p, w0, P);
                     Stream rng(P.key, p.iter, P_ATTEMPT, P.run, P.k);
                     const unsigned long long r0 = rng.next64();
@@ -414,7 +444,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
             int cls = 0;
             unsigned long long w0 = 0, r1 = 0;
             if (valid) {
-                w0 = st.att[q];
+                w0 = attempt_entry(st, q, n_entry);
                 Stream rng = attempt_stream(st, p, w0);
                 const unsigned long long r0 = rng.next64();
                 r1 = rng.next64();

@@ -1,7 +1,11 @@
 """GPU parity of the forms a step takes at the edges of their ranges, against
-the CPU oracle, bit for bit: the walker hash kept at a high load, where its
-tombstones pile up and it is rebuilt inside a call (cleared behind one step,
-refilled by the next sweep) and between calls."""
+the CPU oracle, bit for bit:
+* the walker hash kept at a high load, where its tombstones pile up and it is
+  rebuilt inside a call (cleared behind one step, refilled by the next sweep)
+  and between calls;
+* heavy parents, whose spawn attempts are numbered by the spawn kernel instead
+  of written as entries: around the limit, around the granules, alone and
+  many side by side."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,7 +15,7 @@ from neci_stable_gb300 import capi
 from neci_stable_gb300.engine import Engine
 from oracle.oracle import Oracle
 
-from helpers import canonical, hubbard10, molecule
+from helpers import canonical, hubbard10, molecule, random_walkers
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +84,23 @@ def test_hash_after_entry_points_between_steps():
     if gone.size:
         with pytest.raises(capi.NeciGpuError):
             eng.set_core_space(gone[:1, None])
+
+
+@pytest.mark.parametrize("name,lenof_sign", [("hub", 1), ("hub", 2), ("mol", 1), ("mol", 2)])
+@pytest.mark.parametrize("signs", [(32.0, 33.0), (33.0,) * 40, (127.5, 128.0, 129.0, 31.0, 1.0), (40.0, 5000.0, 1.5, 70000.0),
+                                   (1.0, 2.0, 31.0)])
+def test_heavy_parents(name, lenof_sign, signs):
+    spec = hubbard10(lenof_sign=lenof_sign) if name == "hub" else molecule(12, 6, lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 15, 1 << 18)
+    orc = Oracle(spec, 1 << 15, 1 << 18, hii=eng.hii)
+    rng = np.random.default_rng(31)
+    rows = random_walkers(spec, 300, rng)
+    W, L = spec.W, spec.lenof_sign
+    v = rows[:, W:W + L].view(np.float64).copy()
+    for k, x in enumerate(signs):  # in both runs, of either sign
+        v[7 * k, 0] = -x if k % 2 else x
+        v[7 * k + 3, L - 1] = x
+    rows[:, W:W + L] = v.view(np.int64)
+    eng.upload(rows)
+    orc.upload(rows)
+    run_both(spec, eng, orc, (1, 2), tau=0.002, seed=17)
