@@ -393,6 +393,86 @@ int32_t neci_gpu_set_random_hash(neci_gpu_ctx *ctx, const int32_t *rh) {
     std::vector<int32_t> h(e.sys.nbasis + 1, 0);
     for (int i = 1; i <= e.sys.nbasis; ++i) h[i] = rh[i - 1];
     CK(cudaMemcpy((void *)e.sys.random_hash2, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    // the table of hash_by_nibbles, where no product of RandomHash2 and an
+    // electron's number leaves 32 bits
+    bool fits = true;
+    for (int i = 1; i <= e.sys.nbasis; ++i)
+        fits = fits && std::llabs((long long)h[i]) * e.sys.nel <= 0x7FFFFFFFll;
+    constexpr unsigned long long kMult = 1099511628211ull;
+    const int nib = hash_nibbles(e.sys.nbasis);
+    std::vector<ulonglong2> tab((size_t)hash_tab_len(e.sys.nbasis));
+    for (int c = 0; c < nib; ++c)
+        for (int v = 0; v < 16; ++v) {
+            unsigned long long a = 0, b = 0;
+            int t = 0;
+            for (int k = 0; k < 4; ++k) {
+                if (!((v >> k) & 1)) continue;
+                const int orb = 4 * c + k + 1;
+                const unsigned long long r = orb <= e.sys.nbasis ? (unsigned long long)(long long)h[orb] : 0ull;
+                ++t;
+                a = kMult * a + r;
+                b = kMult * b + r * (unsigned long long)t;
+            }
+            tab[16 * c + v].x = a;
+            tab[16 * c + v].y = b;
+        }
+    unsigned long long pw[8];
+    pw[0] = 1;
+    for (int n = 1; n < 8; ++n) pw[n] = pw[n - 1] * kMult;
+    std::memcpy(&tab[16 * nib], pw, sizeof(pw));
+    if (!e.hash_tab)
+        if (int r = dalloc(e, &e.hash_tab, tab.size())) return r;
+    CK(cudaMemcpyAsync(e.hash_tab, tab.data(), tab.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice, e.stream));
+    CK(cudaStreamSynchronize(e.stream));
+    e.sys.hash_tab = fits ? e.hash_tab : nullptr;
+    drop_graphs(e);
+    return NECI_GPU_OK;
+}
+
+// The tables of a lattice with one coupling (LatTab), when TMat2D and the
+// lattice are both there: built when every listed neighbour pair of either
+// spin has the same coupling, of at least the generator's 1e-10 floor (the
+// list's total); otherwise the spawn kernel runs the general generator.
+static int derive_lattice_tables(Engine &e) {
+    e.sys.lat = nullptr;
+    const int mn = e.sys.max_neigh, nb = e.sys.nbasis;
+    if (e.sys.system != NECI_SYS_HUBBARD_REAL_SPACE || e.h_tmat.empty() || e.h_neighbours.empty()) return NECI_GPU_OK;
+    double t = 0.0;
+    for (int i = 0; i < e.sys.nsites * mn; ++i) {
+        const int n = e.h_neighbours[i], site = i / mn + 1;
+        if (n <= 0) continue;
+        for (int spin = 0; spin < 2; ++spin) {
+            const int src = 2 * site - spin, orb = 2 * n - spin;
+            const double v = e.h_tmat[(size_t)(orb - 1) * nb + (src - 1)];
+            if (t == 0.0) t = v;
+            if (v != t || !(std::fabs(v) >= 1e-10) || !std::isfinite(v)) return NECI_GPU_OK;
+        }
+    }
+    if (t == 0.0) return NECI_GPU_OK;
+    LatTab h{};
+    h.t = t;
+    double cum[kMaxNeigh + 1] = {0.0};  // the running sums of 1, 2, ... open neighbours
+    for (int m = 1; m <= kMaxNeigh; ++m) cum[m] = cum[m - 1] + std::fabs(t);
+    for (int m = 1; m <= kMaxNeigh; ++m)
+        for (int j = 1; j <= m; ++j) {
+            // the largest 53-bit draw x with (x 2^-53) cum[m] <= cum[j], as rounded
+            unsigned long long lo = 0, hi = (1ull << 53) - 1;
+            while (lo < hi) {
+                const unsigned long long mid = lo + (hi - lo + 1) / 2;
+                const double r = ((double)mid * 0x1.0p-53) * cum[m];
+                if (r <= cum[j]) lo = mid;
+                else hi = mid - 1;
+            }
+            const int i = kMaxNeigh * (m - 1) + (j - 1);
+            const double p_orb = (cum[j] - cum[j - 1]) / cum[m];
+            h.bound[i] = lo;
+            h.invp[i] = 1.0 / ((1.0 / (double)e.sys.nel) * p_orb);
+        }
+    if (!e.lat_tab)
+        if (int r = dalloc(e, &e.lat_tab, 1)) return r;
+    CK(cudaMemcpyAsync(e.lat_tab, &h, sizeof(h), cudaMemcpyHostToDevice, e.stream));
+    CK(cudaStreamSynchronize(e.stream));
+    e.sys.lat = e.lat_tab;
     return NECI_GPU_OK;
 }
 
@@ -411,8 +491,9 @@ int32_t neci_gpu_set_tmat(neci_gpu_ctx *ctx, const double *t) {
     CK(cudaStreamSynchronize(e.stream));
     e.sys.tmat = d;
     e.sys.tmat32 = d32;
+    if (e.sys.system == NECI_SYS_HUBBARD_REAL_SPACE) e.h_tmat.assign(t, t + n);
     drop_graphs(e);
-    return NECI_GPU_OK;
+    return derive_lattice_tables(e);
 }
 
 int32_t neci_gpu_set_umat(neci_gpu_ctx *ctx, const double *u, int64_t len) {
@@ -469,8 +550,9 @@ int32_t neci_gpu_set_lattice(neci_gpu_ctx *ctx, const int32_t *nb, int32_t nsite
     CK(cudaStreamSynchronize(e.stream));
     e.sys.neighbours = d;
     e.sys.nsites = nsites;
+    e.h_neighbours.assign(nb, nb + n);
     drop_graphs(e);
-    return NECI_GPU_OK;
+    return derive_lattice_tables(e);
 }
 
 // Hoisted constants of the excitation generators from pSingles, pParallel

@@ -124,15 +124,31 @@ __device__ inline AliasRec load_alias(const AliasRec *p) {
     return r;
 }
 
+// The rs-Hubbard generator's choices on a lattice whose couplings are all
+// equal (one hopping t between every pair of listed neighbours): with m of a
+// site's neighbours open, the cumulative list holds m equal steps, and the
+// j-th open neighbour is picked when the draw's 53 bits lie above bound
+// j - 1 and not above bound j.  Entries [8 (m - 1) + (j - 1)].
+struct LatTab {
+    unsigned long long bound[kMaxNeigh * kMaxNeigh];  // the largest draw that picks j or an earlier one
+    double invp[kMaxNeigh * kMaxNeigh];               // 1/p_gen of that pick
+    double t;                                         // the coupling
+};
+
 struct DevSys {
     int nel, nbasis, W, L, R, system, excitgen, max_neigh, nsites, nOccAlpha, nOccBeta, nBI;
     double uhub, bhub, ecore, p_singles, p_parallel, hii;
     long long ijMax, abMax;
     unsigned long long ilut_ref[kMaxWords];
     const int32_t *random_hash2;   // [nbasis + 1], 1-based
+    // FindWalkerHash four orbitals at a time (hash_by_nibbles): [place][value],
+    // then the powers of the multiplier; null where RandomHash2 times an
+    // electron's number can overflow its 32 bits
+    const ulonglong2 *hash_tab;
     const double *tmat;            // TMat2D column-major
     const double *umat;            // UMAT, UMatInd - 1
     const int32_t *neighbours;     // [nsites * max_neigh], 1-based site, 0 = none
+    const LatTab *lat;             // lattices with one coupling for all neighbours, else null
     const double *pexch;           // [ijMax]
     const double *alias_bias;      // [(ij-1)*3 + type-1][abMax]
     const int32_t *alias_alias;
@@ -614,6 +630,36 @@ __device__ inline unsigned long long neci_hash(const unsigned long long *d, int 
             const long long term = (long long)(int32_t)(rh2[orb] * i);
             hash = 1099511628211ull * hash + (unsigned long long)term;
             x &= x - 1;
+        }
+    }
+    return hash;
+}
+// The same value four orbitals at a time.  With P the multiplier, the n
+// electrons of a nibble that follow `before` others turn the hash into
+//   hash P^n + sum_t P^(n-t) rh2(orb_t) (before + t) = hash P^n + before a + b,
+// a and b the table's entry for the nibble's place and value (all modulo
+// 2^64; exact while rh2(orb) times the number of electrons fits 32 bits,
+// which the host checks).  A nibble costs about 14 instructions, the same for
+// every lane, and its loads do not wait for one another; the loop over
+// electrons costs about 17 each in one dependent chain, as long as the
+// warp's fullest determinant.  `tab` is in shared memory: from global memory
+// (bytes at a time, 36 KB) the lanes' scattered 16-byte loads made the 6x6
+// lattice's spawn kernel 15% slower than the loop.
+__host__ __device__ inline int hash_nibbles(int nbasis) { return (nbasis + 3) / 4; }
+__host__ __device__ inline int hash_tab_len(int nbasis) { return 16 * hash_nibbles(nbasis) + 4; }
+template <int NW>
+__device__ inline unsigned long long hash_by_nibbles(const unsigned long long *d, int W, int nibbles, const ulonglong2 *tab) {
+    const unsigned long long *pw = reinterpret_cast<const unsigned long long *>(tab + 16 * nibbles);
+    unsigned long long hash = 0;
+    unsigned int before = 0;
+    NECI_FOR_WORDS(w, NW > 0 ? NW : W) {
+#pragma unroll 4
+        for (int c = 0; c < 16; ++c) {
+            if (16 * w + c >= nibbles) break;
+            const unsigned int v = (unsigned int)(d[w] >> (4 * c)) & 15u, n = __popc(v);
+            const ulonglong2 a = tab[16 * (16 * w + c) + v];
+            hash = hash * pw[n] + a.y + a.x * before;
+            before += n;
         }
     }
     return hash;

@@ -156,6 +156,51 @@ __device__ inline void gen_rs_hubbard(const DevSys &s, const unsigned long long 
     e.ok = true;
 }
 
+// gen_rs_hubbard on a lattice with one coupling (DevSys::lat): the same draws,
+// pick, child and probability without FP64 arithmetic.  The generator above
+// issues about 30 FP64 instructions an attempt (running sums, two divisions,
+// the amplitude), which held GB300's FP64 pipe (about one lane per clock per
+// SM) for most of the spawn kernel's time; here the pick is integer compares
+// of the draw with `bound` (LatTab, in shared memory) and the rest follows
+// from the pair (open neighbours m, pick j), whose table index is returned in
+// `cell`.  nb8: the site's neighbours, one byte each (site - 1, 255: none).
+// A draw of zero is left to gen_rs_hubbard (it picks the first entry of the
+// list, open or not): returns false.
+template <int NW>
+__device__ inline bool pick_rs_uniform(const DevSys &s, const unsigned long long *d, const unsigned long long *nb8,
+                                       const unsigned long long *bound, Stream &rng, int &src, int &tgt, int &cell) {
+    rng.fill_pair();  // the pick's two draws and the rounding draw: two Philox blocks side by side
+    src = nth_orbital(d, nwords<NW>(s), kAllBits, 1 + (int)uniform_index(rng, (unsigned)s.nel));
+    const unsigned long long nb = nb8[spat(src) - 1];
+    const int spin = (src - 1) & 1;
+    unsigned int open = 0;
+#pragma unroll
+    for (int k = 0; k < kMaxNeigh; ++k) {
+        if (k >= s.max_neigh) break;
+        const unsigned int n = (unsigned int)(nb >> (8 * k)) & 0xFFu;
+        if (n != 255u && !orb_occ(d, 2 * (int)n + 1 + spin)) open |= 1u << k;
+    }
+    const int m = __popc(open);
+    cell = -1;
+    if (m == 0) return true;
+    const unsigned long long x = rng.next64() >> 11;
+    if (x == 0) return false;
+    const unsigned long long *b = bound + kMaxNeigh * (m - 1);
+    int j = 0;  // earlier open neighbours than the pick
+#pragma unroll
+    for (int k = 0; k < kMaxNeigh - 1; ++k) {
+        if (k >= s.max_neigh - 1) break;
+        if (k < m - 1 && x > b[k]) {
+            ++j;
+            open &= open - 1;
+        }
+    }
+    cell = kMaxNeigh * (m - 1) + j;
+    const int k = __ffs((int)open) - 1;
+    tgt = 2 * (int)((nb >> (8 * k)) & 0xFFu) + 1 + spin;
+    return true;
+}
+
 // The c-th (1-based) unoccupied spin orbital among those of `pattern`, 0 if none.
 template <int NW = 0>
 __device__ inline int nth_unoccupied(const DevSys &s, const unsigned long long *d, unsigned long long pattern, int c) {

@@ -76,6 +76,12 @@ struct Engine {
     cudaEvent_t branch_ev = nullptr, merge_ev = nullptr;
     std::vector<void *> allocs;
     bool have_ref = false, have_pchb = false;
+    // lattices: host copies of TMat2D and the neighbour lists, and the device
+    // table of DevSys::lat derived from them
+    std::vector<double> h_tmat;
+    std::vector<int32_t> h_neighbours;
+    LatTab *lat_tab = nullptr;
+    ulonglong2 *hash_tab = nullptr;  // device table of DevSys::hash_tab
     double *inv_single = nullptr;  // device table of DevSys::inv_single
     float *inv_single32 = nullptr;
     // CUDA graph of one step per precision (FP64, mixed); `graph` is the one

@@ -18,13 +18,30 @@ namespace neci {
 template <typename Real>
 __device__ inline Real prm(double d, float f) { return sizeof(Real) == 8 ? (Real)d : (Real)f; }
 
+// The rounding of a spawned amplitude of magnitude aq in fixed point, with its
+// sign: RealSpawnCutoff rounding (|n| < cutoff -> +-cutoff with probability
+// |n|/cutoff) or stochastic_round (lib/util_mod.fpp:182) to an integer
+// walker, in integer arithmetic.  Returns 0 for no child.
+__device__ inline long long round_amplitude(const IterParams &p, bool negative, unsigned long long aq, Stream &rng) {
+    unsigned long long v = aq;
+    if (p.t_all_real_coeff) {
+        // keep with probability aq / cutoff_q
+        if (p.t_real_spawn_cutoff && aq < p.cutoff_q)
+            v = __umul64hi(rng.next64(), p.cutoff_q) < aq ? p.cutoff_q : 0ull;
+    } else {
+        const unsigned long long whole = aq >> 32, frac = aq & 0xFFFFFFFFull;
+        v = whole;
+        if (frac != 0 && (rng.next64() >> 32) < frac) v += 1;
+        v <<= 32;
+    }
+    return negative ? -(long long)v : (long long)v;
+}
+
 // attempt_create_normal (fcimc_pointed_fns.F90:178-494) for one generated
 // excitation: the child amplitude -tau H_ij sign(C) / (p_gen AvMCExcits),
 // taken as -tau H_ij sign(C) (1/p_gen) (1/AvMCExcits) in precision Real and
-// converted to fixed point, then rounded there in integer arithmetic:
-// RealSpawnCutoff rounding (|n| < cutoff -> +-cutoff with probability
-// |n|/cutoff) or stochastic_round (lib/util_mod.fpp:182) to an integer
-// walker.  Returns 0 for no child.
+// converted to fixed point, then rounded there (round_amplitude).  Returns 0
+// for no child.
 // In FP64 the product is formed as ((tau H_ij) (1/p_gen)) (1/AvMCExcits)
 // and its sign applied afterwards: multiplying by -1, by the walker sign and
 // by 1/AvMCExcits = 1 are exact, so the value is the reference order's, with
@@ -49,19 +66,7 @@ __device__ inline long long spawn_amplitude(const IterParams &p, Real hel, Real 
     }
     const unsigned long long aq = (unsigned long long)(q < 0 ? -q : q);
     aq_out = aq;
-    if (p.t_all_real_coeff) {
-        if (p.t_real_spawn_cutoff && aq < p.cutoff_q) {
-            // keep with probability |q| / cutoff_q
-            const bool keep = __umul64hi(rng.next64(), p.cutoff_q) < aq;
-            return keep ? (q < 0 ? -(long long)p.cutoff_q : (long long)p.cutoff_q) : 0ll;
-        }
-        return q;
-    }
-    const unsigned long long whole = aq >> 32, frac = aq & 0xFFFFFFFFull;
-    unsigned long long m = whole;
-    if (frac != 0 && (rng.next64() >> 32) < frac) m += 1;
-    const long long v = (long long)(m << 32);
-    return q < 0 ? -v : v;
+    return round_amplitude(p, q < 0, aq, rng);
 }
 
 // One spawn attempt's parent, unpacked from its 8-byte attempt entry
@@ -142,21 +147,75 @@ __device__ inline void tau_log(const DevSys &s, const Excit<Real> &e, TauAcc *ac
     if (counts && acc->c[e.cls] <= kTauCntThreshold) atomicAdd(&acc->c[e.cls], 1u);
 }
 
-// attempt_create for a generated excitation: the core -> core filter
-// (is_core_state, semi_stoch_procs.F90:547; those spawns are done by the
-// deterministic projection), the tau-search log and the rounded fixed-point
-// amplitude.
+// Whether a child is a core determinant (is_core_state,
+// semi_stoch_procs.F90:547).
+template <int NW, int RW>
+__device__ inline bool core_child(const DevSys &s, const DevState &st, const unsigned long long *c) {
+    const long long hs = hash_find(st, c, nwords<NW>(s), s.R, neci_hash(c, nwords<NW>(s), s.random_hash2), st.ctl);
+    return hs >= 0 && is_core_flags(st.dets[hs * s.R + rwords<RW>(s) + s.L]);
+}
+
+// A spawned amplitude out of the fixed point's range (spawn_amplitude's ovf),
+// as the amplitude of its child.
+constexpr long long kOverflow = -0x7FFFFFFFFFFFFFFFll - 1;
+
+// attempt_create for a generated excitation: the tau-search log and the
+// rounded fixed-point amplitude.  The reference first filters a core parent's
+// core children (the deterministic projection makes those spawns).  Without
+// the tau search, which logs the attempts that pass, the filter matters only
+// for a child that comes to be, so create_particle applies it: a core
+// parent's attempts are the most numerous of a semistochastic run and few of
+// them spawn.
 template <typename Real, int NW, int RW>
 __device__ inline long long attempt_create(const DevSys &s, const DevState &st, const IterParams &p, const Parent &P,
-                                           Excit<Real> &e, Stream &rng, const int32_t *sh_rh2, int &ovf,
-                                           TauAcc *tacc) {
+                                           Excit<Real> &e, Stream &rng, TauAcc *tacc) {
     if (!e.ok) return 0;
-    if (P.core) {
-        const long long hs = hash_find(st, e.child, nwords<NW>(s), s.R, neci_hash(e.child, nwords<NW>(s), sh_rh2), st.ctl);
-        if (hs >= 0 && is_core_flags(st.dets[hs * s.R + rwords<RW>(s) + s.L])) return 0;
+    if (s.tau_search) {
+        if (P.core && core_child<NW, RW>(s, st, e.child)) return 0;
+        tau_log<Real>(s, e, tacc);
     }
-    if (s.tau_search) tau_log<Real>(s, e, tacc);
-    return spawn_amplitude<Real>(p, e.hel, e.invp, P.neg, rng, ovf, e.aq);
+    int ovf = 0;
+    const long long q = spawn_amplitude<Real>(p, e.hel, e.invp, P.neg, rng, ovf, e.aq);
+    return ovf ? kOverflow : q;
+}
+
+// The attempt of the general lattice generator, as the instance for one
+// coupling runs it: out of line and on copies of its own, since it is met once
+// in 2^53 draws there.
+template <typename Real, int NW, int RW>
+__device__ __noinline__ long long create_general(const DevSys &s, const DevState &st, const IterParams &p,
+                                                 const unsigned long long w0, const int32_t *sh_neigh, TauAcc *tacc,
+                                                 Excit<Real> *e) {
+    Parent P;
+    load_parent<NW, RW>(s, st, p, w0, P);
+    Stream rng(P.key, p.iter, P_ATTEMPT, P.run, P.k);
+    gen_rs_hubbard<Real, NW>(s, P.d, sh_neigh, rng, *e);
+    return attempt_create<Real, NW, RW>(s, st, p, P, *e, rng, tacc);
+}
+
+// The attempt of pick_rs_uniform: finish_single and attempt_create with the
+// amplitude's magnitude taken from the step's table.
+template <typename Real, int NW, int RW>
+__device__ inline long long create_uniform(const DevSys &s, const DevState &st, const IterParams &p, const Parent &P,
+                                           int src, int tgt, int cell, const unsigned long long *sh_aq, Excit<Real> &e,
+                                           Stream &rng, TauAcc *tacc) {
+    NECI_FOR_WORDS(w, nwords<NW>(s)) e.child[w] = P.d[w];
+    flip_orb(e.child, src);
+    flip_orb(e.child, tgt);
+    if (s.tau_search || s.rdm) {
+        e.cls = TC_SING;
+        e.hel = (Real)fabs(s.lat->t);
+        e.invp = (Real)s.lat->invp[cell];
+    }
+    if (s.tau_search) {
+        if (P.core && core_child<NW, RW>(s, st, e.child)) return 0;
+        tau_log<Real>(s, e, tacc);
+    }
+    e.aq = sh_aq[cell];
+    if (e.aq == ~0ull) return kOverflow;
+    // -tau H sign(C): make_single's parity, the coupling's sign, the parent's
+    const bool par = occ_between(P.d, nwords<NW>(s), min(src, tgt), max(src, tgt)) & 1;
+    return round_amplitude(p, !(par ^ (s.lat->t < 0.0) ^ P.neg), e.aq, rng);
 }
 
 // The unbiasing weight of a spawn's parent for the 2-RDM (the role of
@@ -178,44 +237,18 @@ __device__ inline double rdm_parent_weight(const IterParams &p, double invp, uns
     return neg ? -w : w;
 }
 
-// The block's sums of the spawns it created, in shared memory: their number
-// and sum of |amplitude| per run (n_spawned and abs_q of the step).  Kept out
-// of registers, which the spawn loop is short of.
-struct SpawnSums {
-    unsigned long long *sh;  // [3]: number, |amplitude| of run 0, of run 1
-};
-
-// create_particle (fcimc_helper.F90:152-308) with pass 1 of the
-// annihilation done at once: the child is looked up in the walker hash
-// (hash_table_lookup); one that is occupied takes the found branch of
-// AnnihilateSpawnedParts (Annihilation.F90:1000-1140), its fixed-point
-// amplitude, record count and initiator bit added to the slot's spawn sums
-// (acc, meta), while an absent child becomes a candidate record of the
-// compression pass.  The sums are integer atomics, so the order of the spawns
-// does not matter.  Done when `fused` (chosen by the host where spawns are
-// frequent enough to fill the lookup's lanes, and never with 2-RDM sampling,
-// which needs every record and its parent); otherwise every spawn is written
-// and pass 1 runs as its own kernel.  Warp-wide (the appends).
+// create_particle (fcimc_helper.F90:152-308): the child's record, appended
+// warp-wide, after the core filter (see attempt_create).
 template <typename Real, int NW, int RW>
 __device__ inline void create_particle(const DevSys &s, const DevState &st, const IterParams &p, long long qv,
-                                       const Parent &P, const Excit<Real> &e, const int32_t *sh_rh2, const SpawnSums &ss,
-                                       bool fused) {
-    long long slot = -1;
-    unsigned long long h = 0;
-    if (qv != 0 && fused) {
-        h = neci_hash(e.child, nwords<NW>(s), sh_rh2);
-        slot = hash_find(st, e.child, nwords<NW>(s), s.R, h, st.ctl);
-        atomicAdd(&ss.sh[0], 1ull);
-        atomicAdd(&ss.sh[1 + P.run], (unsigned long long)(qv < 0 ? -qv : qv));
+                                       const Parent &P, const Excit<Real> &e) {
+    bool rec = qv != 0;
+    if (rec && P.core && !s.tau_search && core_child<NW, RW>(s, st, e.child)) rec = false;
+    if (rec && qv == kOverflow) {
+        set_err(st.ctl, NECI_GPU_ERR_OVERFLOW);
+        rec = false;
     }
-    if (fused && qv != 0 && slot >= 0) {
-        const long long j = slot * s.L + P.run;
-        atomicAdd((unsigned long long *)&st.acc[j], (unsigned long long)qv);
-        atomicAdd(&st.meta[j], 1u);
-        if (P.pinit) atomicOr(&st.meta[j], 0x80000000u);
-    }
-    const bool rec = qv != 0 && (!fused || slot < 0);
-    const unsigned long long pos = warp_append1(fused ? &st.ctl->n_cand : &st.ctl->n_spawned, rec);
+    const unsigned long long pos = warp_append1(&st.ctl->n_spawned, rec);
     if (!rec) return;
     if (pos >= (unsigned long long)st.max_spawned) {
         set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
@@ -225,11 +258,6 @@ __device__ inline void create_particle(const DevSys &s, const DevState &st, cons
     NECI_FOR_WORDS(w, rwords<RW>(s)) o[w] = w < nwords<NW>(s) ? (long long)e.child[w] : 0ll;
     for (int k2 = 0; k2 < s.L; ++k2) o[rwords<RW>(s) + k2] = (k2 == P.run) ? qv : 0ll;
     o[rwords<RW>(s) + s.L] = P.pinit ? (1ll << init_flag_bit(P.run)) : 0ll;
-    if (fused) {
-        st.cand[pos] = (uint32_t)pos;
-        st.cand_h[pos] = h;
-        return;
-    }
     if (!s.rdm) return;
     // the parent and its unbiased sign for the 2-RDM: sign(C_i) divided
     // by the expected number of non-zero spawns onto this child per unit
@@ -239,13 +267,89 @@ __device__ inline void create_particle(const DevSys &s, const DevState &st, cons
     par[rwords<RW>(s)] = double_to_word(rdm_parent_weight(p, (double)e.invp, e.aq, P.neg));
 }
 
+// Children of a warp waiting for the fused lookup, in shared memory: their
+// words, amplitude and marks.  A warp holds fewer than 32 between rounds.
+constexpr int kWaiting = 64;
+template <int NW>
+struct Waiting {
+    unsigned long long d[NW > 0 ? NW : kMaxWords][kWaiting];
+    long long q[kWaiting];
+    uint32_t mark[kWaiting];  // run | initiator parent << 1 | core parent << 2
+};
+
+// create_particle with pass 1 of the annihilation done at once, for 32 waiting
+// children of a warp (entries first .. first + n - 1): each is looked up in
+// the walker hash (hash_table_lookup); one that is occupied takes the found
+// branch of AnnihilateSpawnedParts (Annihilation.F90:1000-1140), its
+// fixed-point amplitude, record count and initiator bit added to the slot's
+// spawn sums (acc, meta), while an absent child becomes a candidate record of
+// the compression pass, and a core parent's core child is dropped (the
+// deterministic projection makes it).  The sums are integer atomics, so the
+// order of the spawns does not matter.  Done when the host chose the fused
+// lookup (spawns frequent, never with 2-RDM sampling, which needs every
+// record and its parent).  The hash and the two dependent reads of a lookup
+// cost a warp the same for one child as for 32, so the children wait until a
+// warp has 32: looked up round by round, 13 of 32 lanes had one on the 6x6
+// lattice and the lookups took half of the kernel's instructions.
+// sums: the block's spawns, their number and |amplitude| per run (n_spawned
+// and abs_q of the step), a place per thread in shared memory (64-bit shared
+// atomics are compare-and-swap loops, which the lanes of a warp that spawn
+// together go through in turn).
+template <int NW, int RW>
+__device__ inline void look_up(const DevSys &s, const DevState &st, Waiting<NW> &wt, int first, int n,
+                               const ulonglong2 *hash_tab, unsigned long long (*sums)[128]) {
+    const int lane = threadIdx.x & 31, i = first + lane;
+    bool rec = lane < n;
+    unsigned long long c[kMaxWords], h = 0;
+    NECI_FOR_WORDS(w, nwords<NW>(s)) c[w] = 0ull;
+    long long qv = 0;
+    uint32_t mark = 0;
+    if (rec) {
+        NECI_FOR_WORDS(w, nwords<NW>(s)) c[w] = wt.d[w][i];
+        qv = wt.q[i];
+        mark = wt.mark[i];
+        h = s.hash_tab ? hash_by_nibbles<NW>(c, s.W, hash_nibbles(s.nbasis), hash_tab)
+                       : neci_hash(c, nwords<NW>(s), s.random_hash2);
+        const long long slot = hash_find(st, c, nwords<NW>(s), s.R, h, st.ctl);
+        bool drop = (mark & 4u) && slot >= 0 && is_core_flags(st.dets[slot * s.R + rwords<RW>(s) + s.L]);
+        if (!drop && qv == kOverflow) {
+            set_err(st.ctl, NECI_GPU_ERR_OVERFLOW);
+            drop = true;
+        }
+        if (!drop) {
+            const unsigned long long aq = (unsigned long long)(qv < 0 ? -qv : qv);
+            sums[0][threadIdx.x] += 1ull;
+            sums[1 + (mark & 1u)][threadIdx.x] += aq;
+            if (slot >= 0) {
+                const long long j = slot * s.L + (mark & 1u);
+                atomicAdd((unsigned long long *)&st.acc[j], (unsigned long long)qv);
+                atomicAdd(&st.meta[j], 1u);
+                if (mark & 2u) atomicOr(&st.meta[j], 0x80000000u);
+            }
+        }
+        rec = !drop && slot < 0;
+    }
+    const unsigned long long pos = warp_append1(&st.ctl->n_cand, rec);
+    if (!rec) return;
+    if (pos >= (unsigned long long)st.max_spawned) {
+        set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        return;
+    }
+    const int run = (int)(mark & 1u);
+    long long *o = st.spawn + pos * s.R;
+    NECI_FOR_WORDS(w, rwords<RW>(s)) o[w] = w < nwords<NW>(s) ? (long long)c[w] : 0ll;
+    for (int k2 = 0; k2 < s.L; ++k2) o[rwords<RW>(s) + k2] = (k2 == run) ? qv : 0ll;
+    o[rwords<RW>(s) + s.L] = mark & 2u ? (1ll << init_flag_bit(run)) : 0ll;
+    st.cand[pos] = (uint32_t)pos;
+    st.cand_h[pos] = h;
+}
+
 // One attempt of class CLS (0: double, 1: single) whose parent and stream
 // are loaded: the stream stands after its first draw (the singles/doubles
 // choice), so the draws are those of the attempt processed inline.
 template <typename Real, int GEN, int CLS, int NW, int RW>
 __device__ inline void spawn_class(const DevSys &s, const DevState &st, const IterParams &p, bool valid,
-                                   const Parent &P, Stream &rng, const int32_t *sh_rh2, int &ovf, TauAcc *tacc,
-                                   const SpawnSums &ss, bool fused) {
+                                   const Parent &P, Stream &rng, TauAcc *tacc) {
     Excit<Real> e;
     e.ok = false;
     long long qv = 0;
@@ -253,9 +357,9 @@ __device__ inline void spawn_class(const DevSys &s, const DevState &st, const It
         if (CLS == 1) gen_uniform_single<Real, NW>(s, P.d, rng, e);
         else if (GEN == NECI_EXGEN_UNIFORM) gen_uniform_double<Real, NW>(s, P.d, rng, e);
         else gen_pchb_double<Real, NW>(s, P.d, rng, e);
-        qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, sh_rh2, ovf, tacc);
+        qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, tacc);
     }
-    create_particle<Real, NW, RW>(s, st, p, qv, P, e, sh_rh2, ss, fused);
+    create_particle<Real, NW, RW>(s, st, p, qv, P, e);
 }
 
 // The parent and stream of a queued attempt: the stream resumes after its
@@ -296,42 +400,75 @@ __device__ inline Stream load_queued(const DevSys &s, const DevState &st, const 
 template <typename Real, int GEN, int NW, int RW, bool QD>
 __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     k_spawn(DevSys s, DevState st, const IterParams *pp, int fuse_probe) {
-    if (halted(st)) return;
     // lattice systems only: their singles spawn often enough to fill the
     // lookup's lanes; the molecular instances carry no fused code
     const bool fused = GEN == NECI_EXGEN_RS_HUBBARD && fuse_probe != 0 && !s.rdm;
-    extern __shared__ int32_t sh[];
+    extern __shared__ __align__(16) unsigned char sh[];
     // per class: attempt entries and their second draws (at most two
     // rounds' worth are held), and each warp's appends of the round (by
     // round parity)
-    __shared__ unsigned long long sq[2][256], sr1[2][256];
+    __shared__ unsigned long long sq[GEN == NECI_EXGEN_RS_HUBBARD ? 1 : 2][256], sr1[GEN == NECI_EXGEN_RS_HUBBARD ? 1 : 2][256];
     __shared__ int wcnt[2][2][4];
     __shared__ unsigned int ring_tail;
-    __shared__ unsigned long long sh_sums[3];
+    // the fused lookup of lattice systems: sums per thread, waiting children
+    // per warp
+    __shared__ Waiting<GEN == NECI_EXGEN_RS_HUBBARD ? NW : 1> waiting[GEN == NECI_EXGEN_RS_HUBBARD ? 4 : 1];
+    __shared__ unsigned long long sh_sums[GEN == NECI_EXGEN_RS_HUBBARD ? 3 : 1][128];
     __shared__ long long sh_n[2];
+    // the lattice instance for one coupling: the pick's bounds, the step's
+    // amplitude magnitudes, the sites' neighbours
+    constexpr bool uniform = GEN == NECI_EXGEN_RS_HUBBARD && QD;
+    __shared__ unsigned long long sh_bound[uniform ? kMaxNeigh * kMaxNeigh : 1], sh_aq[uniform ? kMaxNeigh * kMaxNeigh : 1];
+    __shared__ unsigned long long sh_nb8[uniform ? 32 * kMaxWords : 1];
     __shared__ TauAcc tacc;
-    int32_t *sh_rh2 = sh;
-    int32_t *sh_neigh = sh + (s.nbasis + 1);
-    for (int i = threadIdx.x; i <= s.nbasis; i += blockDim.x) sh_rh2[i] = s.random_hash2[i];
-    if (GEN == NECI_EXGEN_RS_HUBBARD)
-        for (int i = threadIdx.x; i < s.nsites * s.max_neigh; i += blockDim.x) sh_neigh[i] = s.neighbours[i];
-    if (threadIdx.x < 4) {
-        tacc.g[threadIdx.x] = 0ull;
-        tacc.c[threadIdx.x] = 0u;
-    }
-    if (threadIdx.x == 0) ring_tail = 0u;
-    if (threadIdx.x < 3) sh_sums[threadIdx.x] = 0ull;
-    __syncthreads();
-    const IterParams p = *pp;
     // attempts in all; sh_n[0] of them have entries (kept in shared memory:
     // the loops below are short of registers)
     if (threadIdx.x == 0) {
         const unsigned long long na = st.ctl->n_att, cap = (unsigned long long)st.max_att;
         const unsigned long long nh = st.ctl->n_big & ((1ull << kBigShift) - 1);
-        if (na + nh > cap) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        const bool stop = halted(st);
+        if (!stop && na + nh > cap) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
         sh_n[0] = (long long)min(na, cap);
-        sh_n[1] = sh_n[0] + (long long)min(nh, cap);
+        sh_n[1] = stop ? 0 : sh_n[0] + (long long)min(nh, cap);
     }
+    __syncthreads();
+    // a block with no attempts leaves (the grid is sized to the capacity)
+    if (sh_n[1] <= (long long)blockIdx.x * blockDim.x) return;
+    const IterParams p = *pp;
+    // lattice systems: the hash table of the fused lookup, the neighbour lists
+    ulonglong2 *sh_hash = reinterpret_cast<ulonglong2 *>(sh);
+    int32_t *sh_neigh = reinterpret_cast<int32_t *>(sh_hash + hash_tab_len(s.nbasis));
+    if (fused && s.hash_tab)
+        for (int i = threadIdx.x; i < hash_tab_len(s.nbasis); i += blockDim.x) sh_hash[i] = s.hash_tab[i];
+    if (GEN == NECI_EXGEN_RS_HUBBARD)
+        for (int i = threadIdx.x; i < s.nsites * s.max_neigh; i += blockDim.x) sh_neigh[i] = s.neighbours[i];
+    if (uniform) {
+        // the amplitude depends on the pick's table cell alone: the block
+        // takes the magnitudes of its step once
+        for (int i = threadIdx.x; i < kMaxNeigh * kMaxNeigh; i += blockDim.x) {
+            Stream none(0, 0, 0, 0, 0);
+            unsigned long long aq = 0;
+            int over = 0;
+            (void)spawn_amplitude<Real>(p, (Real)fabs(s.lat->t), (Real)s.lat->invp[i], false, none, over, aq);
+            sh_bound[i] = s.lat->bound[i];
+            sh_aq[i] = over ? ~0ull : aq;
+        }
+        for (int i = threadIdx.x; i < s.nsites; i += blockDim.x) {
+            unsigned long long b = ~0ull;  // the site's neighbours, a byte each (255: none)
+            for (int k = 0; k < s.max_neigh; ++k) {
+                const int n = s.neighbours[i * s.max_neigh + k];
+                if (n > 0) b = (b & ~(0xFFull << (8 * k))) | ((unsigned long long)(n - 1) << (8 * k));
+            }
+            sh_nb8[i] = b;
+        }
+    }
+    if (threadIdx.x < 4) {
+        tacc.g[threadIdx.x] = 0ull;
+        tacc.c[threadIdx.x] = 0u;
+    }
+    if (threadIdx.x == 0) ring_tail = 0u;
+    if (fused)
+        for (int k = 0; k < 3; ++k) sh_sums[k][threadIdx.x] = 0ull;
     __syncthreads();
     const volatile long long &n_entry = sh_n[0];
     const long long nat = sh_n[1];
@@ -340,24 +477,59 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     const int nb = blockDim.x;  // 128: four warps
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int qn[2] = {0, 0};  // queue lengths, the same in every thread
-    int ovf = 0;
-    const SpawnSums ss = {sh_sums};
-    if (GEN == NECI_EXGEN_RS_HUBBARD) {
-        // lattice systems (singles only): one attempt per thread per round
+    if constexpr (GEN == NECI_EXGEN_RS_HUBBARD) {
+        // lattice systems (singles only): one attempt per thread per round.
+        // QD marks the instance for one coupling (DevSys::lat).
+        Waiting<NW> &wt = waiting[wid];
+        int n_wait = 0;  // the warp's waiting children, the same in every lane
         for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nround; q += stride) {
             long long qv = 0;
             Parent P;
             P.run = 0;
             P.pinit = false;
+            P.core = false;
             Excit<Real> e;
             e.ok = false;
             if (q < nat) {
-                load_parent<NW, RW>(s, st, p, attempt_entry(st, q, n_entry), P);
+                const unsigned long long w0 = attempt_entry(st, q, n_entry);
+                load_parent<NW, RW>(s, st, p, w0, P);
                 Stream rng(P.key, p.iter, P_ATTEMPT, P.run, P.k);
-                gen_rs_hubbard<Real, NW>(s, P.d, sh_neigh, rng, e);
-                qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, sh_rh2, ovf, &tacc);
+                if (QD) {
+                    int src, tgt, cell;
+                    if (!pick_rs_uniform<NW>(s, P.d, sh_nb8, sh_bound, rng, src, tgt, cell)) {
+                        Excit<Real> eg;
+                        qv = create_general<Real, NW, RW>(s, st, p, w0, sh_neigh, &tacc, &eg);
+                        e = eg;
+                    } else if (cell >= 0) {
+                        qv = create_uniform<Real, NW, RW>(s, st, p, P, src, tgt, cell, sh_aq, e, rng, &tacc);
+                    }
+                } else {
+                    gen_rs_hubbard<Real, NW>(s, P.d, sh_neigh, rng, e);
+                    qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, &tacc);
+                }
             }
-            create_particle<Real, NW, RW>(s, st, p, qv, P, e, sh_rh2, ss, fused);
+            if (!fused) {
+                create_particle<Real, NW, RW>(s, st, p, qv, P, e);
+                continue;
+            }
+            const unsigned int m = __ballot_sync(0xffffffffu, qv != 0);
+            if (qv != 0) {
+                const int i = n_wait + __popc(m & ((1u << lane) - 1u));
+                NECI_FOR_WORDS(w, nwords<NW>(s)) wt.d[w][i] = e.child[w];
+                wt.q[i] = qv;
+                wt.mark[i] = (uint32_t)P.run | (P.pinit ? 2u : 0u) | (P.core ? 4u : 0u);
+            }
+            n_wait += __popc(m);
+            if (n_wait >= 32) {
+                __syncwarp();
+                n_wait -= 32;
+                look_up<NW, RW>(s, st, wt, n_wait, 32, sh_hash, sh_sums);
+                __syncwarp();
+            }
+        }
+        if (fused) {
+            __syncwarp();
+            look_up<NW, RW>(s, st, wt, 0, n_wait, sh_hash, sh_sums);
         }
     }
     // Molecular systems without QD (singles rare or dominant): a round
@@ -370,7 +542,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // thread.  A full batch (or after the last attempt what is left) is read
     // at once and processed: the next round's appends land at least 128 and
     // less than 512 entries past the head, never on an entry being read.
-    if (GEN != NECI_EXGEN_RS_HUBBARD && !QD) {
+    if constexpr (GEN != NECI_EXGEN_RS_HUBBARD && !QD) {
         unsigned long long *ring = &sq[0][0], *ring_r1 = &sr1[0][0];  // 512 entries each
         unsigned int head = 0;
         int cnt = 0;
@@ -398,10 +570,10 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                     } else {
                         if (GEN == NECI_EXGEN_UNIFORM) gen_uniform_double<Real, NW>(s, P.d, rng, e);
                         else gen_pchb_double<Real, NW>(s, P.d, rng, e);
-                        qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, sh_rh2, ovf, &tacc);
+                        qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, &tacc);
                     }
                 }
-                create_particle<Real, NW, RW>(s, st, p, qv, P, e, sh_rh2, ss, fused);
+                create_particle<Real, NW, RW>(s, st, p, qv, P, e);
             }
             if (single) {
                 const unsigned int t = atomicAdd(&ring_tail, 1u) & 511u;
@@ -418,7 +590,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                 cnt -= take;
                 Parent P;
                 Stream rng = load_queued<NW, RW>(s, st, p, v, a, b, P);
-                spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v, P, rng, sh_rh2, ovf, &tacc, ss, fused);
+                spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v, P, rng, &tacc);
             }
         }
     }
@@ -435,7 +607,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // drains takes a second barrier (its entries visible) and reads its
     // entries at once; the next round writes only after its own first
     // barrier, by which time every thread has read them.
-    if (GEN != NECI_EXGEN_RS_HUBBARD && QD) {
+    if constexpr (GEN != NECI_EXGEN_RS_HUBBARD && QD) {
         long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
         for (int round = 0;; ++round, q += stride) {
             const bool more = q - threadIdx.x < nround;  // the same in the whole block
@@ -500,24 +672,26 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                 if (t0) {
                     Parent P;
                     Stream rng = load_queued<NW, RW>(s, st, p, v0, a0, b0, P);
-                    spawn_class<Real, GEN, 0, NW, RW>(s, st, p, v0, P, rng, sh_rh2, ovf, &tacc, ss, fused);
+                    spawn_class<Real, GEN, 0, NW, RW>(s, st, p, v0, P, rng, &tacc);
                 }
                 if (t1) {
                     Parent P;
                     Stream rng = load_queued<NW, RW>(s, st, p, v1, a1, b1, P);
-                    spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v1, P, rng, sh_rh2, ovf, &tacc, ss, fused);
+                    spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v1, P, rng, &tacc);
                 }
             }
         }
     }
-    if (ovf) set_err(st.ctl, NECI_GPU_ERR_OVERFLOW);
-    // n_spawned and abs_q of the spawns created here (with 2-RDM sampling
-    // pass 1 counts them)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (sh_sums[0]) atomicAdd(&st.ctl->n_spawned, sh_sums[0]);
-        if (sh_sums[1]) atomicAdd(&st.ctl->abs_q[0], sh_sums[1]);
-        if (sh_sums[2]) atomicAdd(&st.ctl->abs_q[1], sh_sums[2]);
+    // n_spawned and abs_q of the spawns created here (otherwise pass 1 counts
+    // them)
+    if (fused) {
+        __syncthreads();
+        if (wid < 3) {
+            unsigned long long t = 0;
+            for (int i = lane; i < 128; i += 32) t += sh_sums[wid][i];
+            t = warp_sum_u(t);
+            if (lane == 0 && t) atomicAdd(wid == 0 ? &st.ctl->n_spawned : &st.ctl->abs_q[wid - 1], t);
+        }
     }
     if (s.tau_search) {
         __syncthreads();
@@ -556,14 +730,18 @@ void launch_spawn_words(Engine &e, cudaStream_t s, int grid, size_t shm) {
 
 template <typename Real, int GEN>
 void launch_spawn_gen(Engine &e, cudaStream_t s, int grid, size_t shm) {
-    if (GEN != NECI_EXGEN_RS_HUBBARD && spawn_queue_doubles(e.sys)) launch_spawn_words<Real, GEN, true>(e, s, grid, shm);
+    const bool qd = GEN == NECI_EXGEN_RS_HUBBARD ? e.sys.lat != nullptr : spawn_queue_doubles(e.sys) != 0;
+    if (qd) launch_spawn_words<Real, GEN, true>(e, s, grid, shm);
     else launch_spawn_words<Real, GEN, false>(e, s, grid, shm);
 }
 
 // The spawn kernel for amplitudes in precision Real.
 template <typename Real>
 void launch_spawn_real(Engine &e, cudaStream_t s) {
-    const size_t shm = (size_t)(e.sys.nbasis + 1 + e.sys.nsites * e.sys.max_neigh) * sizeof(int32_t);
+    const size_t shm = e.sys.excitgen == NECI_EXGEN_RS_HUBBARD
+                           ? (size_t)hash_tab_len(e.sys.nbasis) * sizeof(ulonglong2) +
+                                 (size_t)(e.sys.nsites * e.sys.max_neigh) * sizeof(int32_t)
+                           : 0;
     const int grid = spawn_grid(e, 128);
     if (e.sys.excitgen == NECI_EXGEN_RS_HUBBARD) launch_spawn_gen<Real, NECI_EXGEN_RS_HUBBARD>(e, s, grid, shm);
     else if (e.sys.excitgen == NECI_EXGEN_UNIFORM) launch_spawn_gen<Real, NECI_EXGEN_UNIFORM>(e, s, grid, shm);

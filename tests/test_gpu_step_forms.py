@@ -5,7 +5,10 @@ the CPU oracle, bit for bit:
   and between calls;
 * heavy parents, whose spawn attempts are numbered by the spawn kernel instead
   of written as entries: around the limit, around the granules, alone and
-  many side by side."""
+  many side by side;
+* lattices with one coupling and with several, the lookup of their children
+  in the spawn kernel or behind it, core parents, and walker hashes the
+  spawn kernel's table cannot hold."""
 from __future__ import annotations
 
 import numpy as np
@@ -15,7 +18,7 @@ from neci_stable_gb300 import capi
 from neci_stable_gb300.engine import Engine
 from oracle.oracle import Oracle
 
-from helpers import canonical, hubbard10, molecule, random_walkers
+from helpers import canonical, hubbard10, hubbard_square, molecule, random_walkers
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +107,69 @@ def test_heavy_parents(name, lenof_sign, signs):
     eng.upload(rows)
     orc.upload(rows)
     run_both(spec, eng, orc, (1, 2), tau=0.002, seed=17)
+
+
+def lattice(kind, lenof_sign):
+    """Lattices the spawn kernel takes in its form for one coupling (ring,
+    duplicated neighbours, six neighbours, two words) and in the general one
+    (couplings that differ in size or sign)."""
+    if kind == "ring":
+        return hubbard10(lenof_sign=lenof_sign)
+    if kind == "two-wide":  # left and right neighbour are the same site
+        return hubbard_square(2, 3, 6, lenof_sign)
+    if kind == "6x6":
+        return hubbard_square(6, 6, 35, lenof_sign)
+    spec = hubbard_square(3, 4, 11, lenof_sign)
+    if kind == "triangular":
+        nb = np.zeros((12, 6), dtype=np.int32)
+        for s in range(12):
+            x, y = s % 3, s // 3
+            for k, (dx, dy) in enumerate(((-1, 0), (1, 0), (0, -1), (0, 1), (1, 1), (-1, -1))):
+                nb[s, k] = (y + dy) % 4 * 3 + (x + dx) % 3 + 1
+        nb[5, 2] = 0  # a site with a neighbour less in the middle of its list
+    else:
+        nb = spec.neighbours
+    t = np.zeros((24, 24))
+    rng = np.random.default_rng(3)
+    for s in range(12):
+        for n in nb[s]:
+            if n > s + 1:
+                v = -1.3 if kind == "triangular" else (rng.choice([-1.0, 1.0]) if kind == "signs" else -rng.uniform(0.3, 2.0))
+                for sp in (0, 1):
+                    t[2 * s + sp, 2 * n - 2 + sp] = t[2 * n - 2 + sp, 2 * s + sp] = v
+    spec.neighbours = nb
+    spec.tmat = np.ascontiguousarray(t.T)
+    return spec
+
+
+@pytest.mark.parametrize("kind", ["ring", "two-wide", "6x6", "triangular", "signs", "sizes"])
+@pytest.mark.parametrize("lenof_sign,fuse,core,real,prec", [(1, 1, 0, 1, 1), (1, 1, 40, 1, 0), (2, 1, 40, 0, 0), (2, 0, 40, 1, 0),
+                                                            (1, 0, 0, 0, 1)])
+@pytest.mark.parametrize("big_hash", [False, True])
+def test_lattice_spawn_forms(kind, lenof_sign, fuse, core, real, prec, big_hash):
+    spec = lattice(kind, lenof_sign)
+    if big_hash:  # products with the electron's number leave 32 bits
+        spec.random_hash2 = (spec.random_hash2.astype(np.int64) * 40009 % (1 << 31)).astype(np.int32)
+    eng = Engine(spec, 1 << 15, 1 << 17)
+    orc = Oracle(spec, 1 << 15, 1 << 17, hii=eng.hii)
+    eng.set_option(capi.OPT_FUSE_PROBE, fuse)
+    rows = random_walkers(spec, 400, np.random.default_rng(8))
+    eng.upload(rows)
+    orc.upload(rows)
+    if core:
+        cd = rows[:core, :spec.W]
+        eng.set_core_space(cd)
+        orc.set_core_space(cd)
+    for tau_search in (0, 1):
+        eng.set_tau_search(bool(tau_search))
+        orc.set_tau_search(bool(tau_search))
+        for it in range(1 + 3 * tau_search, 4 + 3 * tau_search):
+            p = capi.default_params(tau=0.01, seed=23, iter=it, t_all_real_coeff=real, precision=prec)
+            sg = eng.perform_fcimc_cyc_par(p)
+            sc, rc = orc.iterate(p)
+            assert rc == 0 and sg.err == 0
+            for f in ("n_attempts", "n_spawned", "n_unique", "n_new", "n_occupied"):
+                assert getattr(sg, f) == getattr(sc, f), (f, it)
+            same_list(spec, eng, orc, it)
+    a, b = eng.tau_stats(), orc.tau_stats()
+    assert a.gamma_sing == b.gamma_sing and a.cnt_sing == b.cnt_sing
