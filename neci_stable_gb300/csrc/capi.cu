@@ -158,6 +158,17 @@ void compress_pass(Engine &e) {
 // they run one after the other on the step's stream.
 void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
     stage(e, K_SWEEP, [&] { launch_sweep(e, e.stream); });
+    // the freed slots' 2-RDM sums: beside the spawn, before the placement
+    if (e.sys.rdm) {
+        if (e.profiling) {
+            stage(e, K_RDM, [&] { launch_rdm_freed(e, e.stream); });
+        } else {
+            cudaEventRecord(e.sweep_ev, e.stream);
+            cudaStreamWaitEvent(e.side, e.sweep_ev, 0);
+            launch_rdm_freed(e, e.side);
+            cudaEventRecord(e.freed_ev, e.side);
+        }
+    }
     stage(e, K_SPAWN, [&] { launch_spawn(e, e.stream); });
     if (e.st.n_core > 0) stage(e, K_CORE, [&] { launch_core(e, e.stream); });
     const int with_core = e.st.n_core > 0 ? 1 : 0;
@@ -172,6 +183,7 @@ void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
         launch_merge_stats(e, e.side, with_core, 1);
         cudaEventRecord(e.merge_ev, e.side);
         compress_pass(e);
+        if (e.sys.rdm) cudaStreamWaitEvent(e.stream, e.freed_ev, 0);
         launch_ann_insert(e, e.stream, 1);
         cudaStreamWaitEvent(e.stream, e.merge_ev, 0);
     }
@@ -349,6 +361,8 @@ int32_t neci_gpu_init(neci_gpu_ctx **out, const neci_gpu_system *sys, int32_t de
         cudaEventCreateWithFlags(&e.join_ev, cudaEventDisableTiming);
         if (cudaEventCreateWithFlags(&e.branch_ev, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&e.merge_ev, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&e.sweep_ev, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&e.freed_ev, cudaEventDisableTiming) != cudaSuccess ||
             cudaStreamCreateWithFlags(&e.side, cudaStreamNonBlocking) != cudaSuccess)
             rc = fail(NECI_GPU_ERR_CUDA, "stream or event creation failed");
         e.graph_version = fresh_graph_version();
@@ -375,6 +389,8 @@ int32_t neci_gpu_free(neci_gpu_ctx *ctx) {
     if (e.join_ev) cudaEventDestroy(e.join_ev);
     if (e.branch_ev) cudaEventDestroy(e.branch_ev);
     if (e.merge_ev) cudaEventDestroy(e.merge_ev);
+    if (e.sweep_ev) cudaEventDestroy(e.sweep_ev);
+    if (e.freed_ev) cudaEventDestroy(e.freed_ev);
     if (e.side) cudaStreamDestroy(e.side);
     for (void *p : e.allocs) cudaFree(p);
     if (e.h_params) cudaFreeHost(e.h_params);
@@ -723,6 +739,7 @@ int32_t neci_gpu_set_rdm_sampling(neci_gpu_ctx *ctx, int32_t on) {
     if (on && !e.st.rdm2) {
         const long long npair = (long long)e.sys.nbasis * (e.sys.nbasis - 1) / 2;
         if (int r = dalloc(e, &e.st.spawn_par, (size_t)e.st.max_spawned * (e.sys.W + 1))) return r;
+        if (int r = dalloc(e, &e.st.rdm_w, (size_t)e.st.max_walkers)) return r;
         if (int r = dalloc(e, &e.st.rdm2, (size_t)npair * npair)) return r;
         CK(cudaStreamSynchronize(e.stream));
         e.sys.npair = npair;
@@ -844,6 +861,8 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaMemsetAsync(e.st.hash, 0, (size_t)e.st.hash_n * 4, e.stream));
     CK(cudaMemsetAsync(e.st.acc, 0, (size_t)e.st.max_walkers * e.sys.L * 8, e.stream));
     CK(cudaMemsetAsync(e.st.meta, 0, (size_t)e.st.max_walkers * e.sys.L * 4, e.stream));
+    // (not zero only behind a failed step)
+    if (e.st.rdm_w) CK(cudaMemsetAsync(e.st.rdm_w, 0, (size_t)e.st.max_walkers * 8, e.stream));
     if (nrows > 0) CK(cudaMemcpyAsync(e.st.dets, ilut, (size_t)nrows * R * 8, cudaMemcpyHostToDevice, e.stream));
     const int compute = (dh && odh) ? 0 : 1;
     if (!compute && nrows > 0) {
@@ -973,13 +992,19 @@ static void take_rehash(Engine &e, neci_gpu_iter_stats *stats, int n) {
     for (int i = 0; i < n; ++i) stats[i].reserved = 0;
 }
 
+// The steps that run before the host looks at the list again: what a step
+// leaves to a later one of them (a refill of the walker hash, the diagonal of
+// the 2-RDM) is done by the last.
+static void set_span(IterParams &p, int n) {
+    p.iter_end = p.iter + n;
+    p.rdm_defer = n > 1;
+}
+
 static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_gpu_iter_stats *stats,
                      double *device_ms = nullptr) {
     if (const char *why = not_ready(e)) return fail(NECI_GPU_ERR_INVALID, why);
     if (p->tau <= 0.0 || p->av_mc_excits <= 0.0) return fail(NECI_GPU_ERR_INVALID, "tau and AvMCExcits must be positive");
     copy_params(*e.h_params, *p);
-    e.h_params->iter_end = p->iter + n_iter;
-    CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e.stream));
     compact_if_due(e, e.stream);
     int done = 0;
     if (device_ms) *device_ms = 0.0;
@@ -987,6 +1012,9 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         if (!e.profiling)
             if (int r = ensure_graph(e)) return r;
         const int batch = std::min(n_iter - done, e.max_stats);
+        e.h_params->iter = p->iter + done;
+        set_span(*e.h_params, batch);
+        CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e.stream));
         CK(cudaMemsetAsync(e.d_stat_pos, 0, sizeof(int), e.stream));
         if (device_ms) CK(cudaEventRecord(e.ev[0], e.stream));
         if (e.profiling) {
@@ -1060,7 +1088,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
     for (int c = 0; c < n_ctx; ++c) {
         Engine &e = ctxs[c]->e;
         copy_params(*e.h_params, params[c]);
-        e.h_params->iter_end = params[c].iter + n_iter;
+        set_span(*e.h_params, n_iter);
         const unsigned long long v = e.graph_version * 8 + (e.h_params->precision == NECI_PREC_MIXED ? 4 : 0) +
                                      (sweep_fast(*e.h_params) ? 2 : 0) + (e.st.n_core > 0 ? 1 : 0);
         key.push_back({(const void *)ctxs[c], v});

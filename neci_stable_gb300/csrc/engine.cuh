@@ -245,6 +245,8 @@ struct DevState {
     // rdm2[pair(p,q) * npair + pair(r,s)] = <a+_p a+_q a_s a_r>, p<q, r<s
     long long *spawn_par;
     double *rdm2;
+    double *rdm_w;                 // per slot: the sum of C^1 C^2 over the call's steps that its determinant has
+                                   // seen, not yet in the 2-RDM's diagonal (zero between calls)
     double *core_x, *core_y;
     float *core_x32;               // core_x rounded to FP32, written in mixed-precision steps
     long long *core_rowptr;
@@ -315,7 +317,9 @@ struct IterParams {
     float f_tau, f_inv_av, f_cutoff, f_inv_cutoff;
     unsigned long long cutoff_q;  // RealSpawnCutoff in fixed point
     int av_unit;                  // AvMCExcits == 1: the spawn count is split in integers
-    long long iter_end;           // the iteration after the call's last one
+    long long iter_end;           // the iteration after the last one of these steps
+    int rdm_defer;                // 2-RDM: the diagonal is summed per slot (DevState::rdm_w) and added
+                                  // behind the last step
 };
 
 // The sweep's fast instance serves steps with real coefficients and

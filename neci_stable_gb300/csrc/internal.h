@@ -74,6 +74,7 @@ struct Engine {
     // the merge sweep), on stream and side
     cudaStream_t side = nullptr;
     cudaEvent_t branch_ev = nullptr, merge_ev = nullptr;
+    cudaEvent_t sweep_ev = nullptr, freed_ev = nullptr;  // around k_rdm_freed, which runs beside the spawn
     std::vector<void *> allocs;
     bool have_ref = false, have_pchb = false;
     // lattices: host copies of TMat2D and the neighbour lists, and the device
@@ -120,6 +121,7 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split);
 void launch_merge_stats(Engine &e, cudaStream_t s, int with_core, int split);
 void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split);
 void launch_rdm(Engine &e, cudaStream_t s);
+void launch_rdm_freed(Engine &e, cudaStream_t s);
 
 // sort form of the annihilation and core selection (sort_kernels.cu)
 constexpr int kSortBins = 256;  // digit values of a radix pass (radix.cuh kRadixBins)

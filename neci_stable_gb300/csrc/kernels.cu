@@ -1066,8 +1066,9 @@ __global__ void __launch_bounds__(256) k_ann_decide(DevSys s, DevState st, const
 // kernel), so their |C| and C^2 (TotParts, norm) and the reference's sign
 // are taken here.
 template <int LR>
-__global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, int split) {
+__global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, const IterParams *pp, int split) {
     if (halted(st)) return;
+    const bool rdm = LR == 2 && split && s.rdm && pp->rdm_defer;
     Control *c = st.ctl;
     double a_tp[2] = {0.0, 0.0}, a_norm[2] = {0.0, 0.0};
     const long long n = (long long)min(c->n_place, (unsigned long long)st.max_spawned);
@@ -1140,6 +1141,7 @@ __global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, int sp
         st.diagH[slot] = dh;
         st.offdiagH[slot] = odh;
         if (st.n_core > 0) st.core_of_slot[slot] = -1;
+        if (rdm) st.rdm_w[slot] = word_to_double(ws[0]) * word_to_double(ws[1]);
         a_tomb -= hash_insert(st, slot, h, c);
         ++a_new;
         if (split) {
@@ -1180,6 +1182,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     const long long n = (long long)min(split ? c->n_pre : c->tot_walkers, (unsigned long long)st.max_walkers);
     const int W = s.W, R = s.R;
     constexpr int L = LR;
+    const bool rdm = LR == 2 && split && s.rdm && p.rdm_defer;
     double a_born[2] = {0, 0}, a_ann[2] = {0, 0}, a_ab[2] = {0, 0}, a_rm[2] = {0, 0};
     double a_tp[2] = {0, 0}, a_norm[2] = {0, 0};
     unsigned long long a_s[2] = {0, 0}, a_occ = 0, a_holes = 0, a_found = 0, a_tomb = 0;
@@ -1316,6 +1319,10 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
             a_tp[k] += abs_dbl(C[k]);
             a_norm[k] = fma(C[k], C[k], a_norm[k]);  // a statistic: one rounding, one FP64 instruction
             if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
+        }
+        if (rdm) {
+            const double w = C[0] * C[1];
+            if (w != 0.0) st.rdm_w[j] += w;
         }
         if (occ || core) {
             ++a_occ;
@@ -1479,18 +1486,19 @@ __global__ void __launch_bounds__(256) k_rdm_core(DevSys s, DevState st) {
     }
 }
 
-// Diagonal terms; per-block sums in shared memory when npair doubles fit.
-// The lanes of a warp hold determinants that share most of their orbitals
-// (those near the reference), so walking their pairs in one order would
-// send all lanes' atomics to the same sum at once; each lane walks the list
-// of electron pairs from its own starting point instead.  (The sums are
-// atomics, whose order is not defined in either case.)
-__global__ void __launch_bounds__(256) k_rdm_diag(DevSys s, DevState st, int use_shared) {
-    if (halted(st)) return;
-    extern __shared__ double sh_diag[];
-    // the electron pairs (a, b), b < a, as a | b << 8
-    __shared__ uint16_t pairs[kMaxNel * (kMaxNel - 1) / 2];
-    const long long npair = s.npair;
+// Diagonal terms: a determinant of weight w adds w to Gamma(pq, pq) of its
+// nel (nel - 1) / 2 occupied pairs; per-block sums in shared memory when
+// npair doubles fit.  The lanes of a warp hold determinants that share most of
+// their orbitals (those near the reference), so walking their pairs in one
+// order would send all lanes' atomics to the same sum at once; each lane walks
+// the list of electron pairs from its own starting point instead.  (The sums
+// are atomics, whose order is not defined in either case.)
+struct DiagSums {
+    const uint16_t *pairs;  // the electron pairs (a, b), b < a, as a | b << 8
+    double *sh;             // npair sums, or null: straight to the 2-RDM
+    int P, start;
+};
+__device__ inline DiagSums diag_begin(const DevSys &s, double *sh, uint16_t *pairs) {
     const int P = s.nel * (s.nel - 1) / 2;
     for (int k = threadIdx.x; k < P; k += blockDim.x) {
         // the largest a with a (a - 1) / 2 <= k, from a float estimate
@@ -1499,33 +1507,75 @@ __global__ void __launch_bounds__(256) k_rdm_diag(DevSys s, DevState st, int use
         while ((a + 1) * a / 2 <= k) ++a;
         pairs[k] = (uint16_t)(a | ((k - a * (a - 1) / 2) << 8));
     }
-    if (use_shared)
-        for (long long k = threadIdx.x; k < npair; k += blockDim.x) sh_diag[k] = 0.0;
+    if (sh)
+        for (long long k = threadIdx.x; k < s.npair; k += blockDim.x) sh[k] = 0.0;
     __syncthreads();
-    const int start = P > 0 ? (int)((threadIdx.x * 7u) % (unsigned)P) : 0;
+    return {pairs, sh, P, P > 0 ? (int)((threadIdx.x * 7u) % (unsigned)P) : 0};
+}
+__device__ inline void diag_add(const DevSys &s, const DevState &st, const DiagSums &ds, const long long *r, double w) {
+    uint8_t nI[kMaxNel];
+    unsigned long long d[kMaxWords];
+    NECI_FOR_WORDS(k, s.W) d[k] = (unsigned long long)r[k];
+    if (decode(d, s.W, nI) != s.nel) return;  // every row holds nel electrons (checked at upload)
+    int k = ds.start;
+    for (int t = 0; t < ds.P; ++t) {
+        const uint32_t ab = ds.pairs[k];
+        const long long pq = rdm_pair(nI[ab >> 8], nI[ab & 0xFFu]);
+        if (ds.sh) atomicAdd(&ds.sh[pq], w);
+        else atomicAdd(&st.rdm2[pq * s.npair + pq], w);
+        if (++k == ds.P) k = 0;
+    }
+}
+__device__ inline void diag_end(const DevSys &s, const DevState &st, const DiagSums &ds) {
+    if (!ds.sh) return;
+    __syncthreads();
+    for (long long k = threadIdx.x; k < s.npair; k += blockDim.x)
+        if (ds.sh[k] != 0.0) atomicAdd(&st.rdm2[k * s.npair + k], ds.sh[k]);
+}
+
+// Every occupied determinant's C^1 C^2 of the step; or, with the weights
+// summed per slot (IterParams::rdm_defer: calls of several steps), those sums
+// behind the last step.  The pair walk issues nel (nel - 1) / 2 shared FP64
+// atomics a determinant, compare-and-swap loops on an FP64 pipe of about one
+// lane per clock per SM: 110 of the 286 us of a step at n = 32 with 2.5e5
+// determinants of 12 electrons.  A determinant that stays for the whole call
+// takes the walk once, and one multiply-add a step in the merge sweep.
+__global__ void __launch_bounds__(256) k_rdm_diag(DevSys s, DevState st, const IterParams *pp, int use_shared) {
+    if (halted(st)) return;
+    const bool defer = pp->rdm_defer != 0;
+    if (defer && pp->iter + 1 < pp->iter_end) return;
+    extern __shared__ double sh_diag[];
+    __shared__ uint16_t pairs[kMaxNel * (kMaxNel - 1) / 2];
+    const DiagSums ds = diag_begin(s, use_shared ? sh_diag : nullptr, pairs);
     const long long n = (long long)min(st.ctl->tot_walkers, (unsigned long long)st.max_walkers);
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
         const long long *r = st.dets + j * s.R;
-        const double prod = word_to_double(r[s.W]) * word_to_double(r[s.W + 1]);
-        if (prod == 0.0) continue;
-        uint8_t nI[kMaxNel];
-        unsigned long long d[kMaxWords];
-        NECI_FOR_WORDS(w, s.W) d[w] = (unsigned long long)r[w];
-        if (decode(d, s.W, nI) != s.nel) continue;  // every row holds nel electrons (checked at upload)
-        int k = start;
-        for (int t = 0; t < P; ++t) {
-            const uint32_t ab = pairs[k];
-            const long long pq = rdm_pair(nI[ab >> 8], nI[ab & 0xFFu]);
-            if (use_shared) atomicAdd(&sh_diag[pq], prod);
-            else atomicAdd(&st.rdm2[pq * npair + pq], prod);
-            if (++k == P) k = 0;
-        }
+        const double w = defer ? st.rdm_w[j] : word_to_double(r[s.W]) * word_to_double(r[s.W + 1]);
+        if (w == 0.0) continue;
+        if (defer) st.rdm_w[j] = 0.0;
+        diag_add(s, st, ds, r, w);
     }
-    if (use_shared) {
-        __syncthreads();
-        for (long long k = threadIdx.x; k < npair; k += blockDim.x)
-            if (sh_diag[k] != 0.0) atomicAdd(&st.rdm2[k * npair + k], sh_diag[k]);
+    diag_end(s, st, ds);
+}
+
+// The sums of the slots this step's sweep freed, before a placement writes
+// another determinant into them.
+__global__ void __launch_bounds__(256) k_rdm_freed(DevSys s, DevState st, const IterParams *pp, int use_shared) {
+    if (halted(st)) return;
+    if (!pp->rdm_defer) return;
+    const long long n = (long long)min(st.ctl->n_free, (unsigned long long)st.max_walkers);
+    if (n <= (long long)blockIdx.x * blockDim.x) return;
+    extern __shared__ double sh_diag[];
+    __shared__ uint16_t pairs[kMaxNel * (kMaxNel - 1) / 2];
+    const DiagSums ds = diag_begin(s, use_shared ? sh_diag : nullptr, pairs);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long j = st.free_list[i];
+        const double w = st.rdm_w[j];
+        if (w == 0.0) continue;
+        st.rdm_w[j] = 0.0;
+        diag_add(s, st, ds, st.dets + j * s.R, w);
     }
+    diag_end(s, st, ds);
 }
 
 // ===========================================================================
@@ -1738,10 +1788,10 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split) {
     const int gp = clamp_grid(e.st.max_spawned / 1024 + 1, e.num_sms * e.occ_place);
     if (e.sys.L == 2) {
         k_ann_decide<2><<<grid_spawns(e, 256, e.occ_insert), 256, 0, s>>>(e.sys, e.st, e.d_params);
-        k_ann_place<2><<<gp, 128, 0, s>>>(e.sys, e.st, split);
+        k_ann_place<2><<<gp, 128, 0, s>>>(e.sys, e.st, e.d_params, split);
     } else {
         k_ann_decide<1><<<grid_spawns(e, 256, e.occ_insert), 256, 0, s>>>(e.sys, e.st, e.d_params);
-        k_ann_place<1><<<gp, 128, 0, s>>>(e.sys, e.st, split);
+        k_ann_place<1><<<gp, 128, 0, s>>>(e.sys, e.st, e.d_params, split);
     }
 }
 // Blocks per SM of the merge sweep when it runs beside the placement
@@ -1754,16 +1804,26 @@ void launch_merge_stats(Engine &e, cudaStream_t s, int with_core, int split) {
     else
         k_merge_stats<1><<<grid, kStageTile, merge_smem_bytes(e), s>>>(e.sys, e.st, e.d_params, with_core, split);
 }
+// Shared memory of the diagonal's block sums: npair doubles, or none where
+// they pass the default dynamic limit.
+static size_t diag_shared(const Engine &e) {
+    const size_t shm = (size_t)e.sys.npair * sizeof(double);
+    return shm <= 48 * 1024 ? shm : 0;
+}
 void launch_rdm(Engine &e, cudaStream_t s) {
     if (!e.sys.rdm) return;
     k_rdm_offdiag<<<grid_spawns(e, 256), 256, (e.sys.nbasis + 1) * sizeof(int32_t), s>>>(e.sys, e.st);
     if (e.st.n_core > 0) k_rdm_core<<<clamp_grid(e.st.n_core_seg / 8 + 1, e.num_sms * 8), 256, 0, s>>>(e.sys, e.st);
-    const size_t shm = (size_t)e.sys.npair * sizeof(double);
-    const int use_shared = shm <= 48 * 1024 ? 1 : 0;  // the default dynamic shared-memory limit
+    const size_t shm = diag_shared(e);
     // at least 64 slots per thread: every block ends by adding its npair
     // shared sums to the global 2-RDM, so the blocks are kept few
     const int grid = clamp_grid(e.st.max_walkers / (256 * 64) + 1, e.num_sms);
-    k_rdm_diag<<<grid, 256, use_shared ? shm : 0, s>>>(e.sys, e.st, use_shared);
+    k_rdm_diag<<<grid, 256, shm, s>>>(e.sys, e.st, e.d_params, shm ? 1 : 0);
+}
+// The slots freed in a step are a few percent of the list: few blocks.
+void launch_rdm_freed(Engine &e, cudaStream_t s) {
+    const size_t shm = diag_shared(e);
+    k_rdm_freed<<<clamp_grid(e.st.max_walkers / (256 * 64) + 1, 32), 256, shm, s>>>(e.sys, e.st, e.d_params, shm ? 1 : 0);
 }
 
 void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split) {
