@@ -139,12 +139,27 @@ void lookup_passes(Engine &e) {
         annihilation_passes(e, 1);
         return;
     }
-    if (!fused_lookup(e)) stage(e, K_ANN_PROBE, [&] { launch_ann_probe(e, e.stream); });
+    if (fused_lookup(e)) return;
+    if (e.gather) stage(e, K_ANN_PROBE, [&] { launch_ann_gather(e, e.stream); });
+    else stage(e, K_ANN_PROBE, [&] { launch_ann_probe(e, e.stream); });
 }
 
-// The compression of the hash form (the sort form has none left).
+// The compression of the hash form (the sort form has none left; for a short
+// list the lookup's kernel does it, and the stage is counted with no time of
+// its own).
 void compress_pass(Engine &e) {
-    if (e.ann_mode != NECI_ANN_SORT) stage(e, K_ANN_COMPRESS, [&] { launch_ann_compress(e, e.stream); });
+    if (e.ann_mode == NECI_ANN_SORT) return;
+    stage(e, K_ANN_COMPRESS, [&] {
+        if (!e.gather || fused_lookup(e)) launch_ann_compress(e, e.stream);
+    });
+}
+
+// The new determinants of a step.
+void insert_pass(Engine &e) {
+    stage(e, K_ANN_INSERT, [&] {
+        if (e.short_list) launch_ann_new(e, e.stream, 1);
+        else launch_ann_insert(e, e.stream, 1);
+    });
 }
 
 // The launch sequence of one PerformFCIMCycPar step.  After the walker-hash
@@ -175,7 +190,7 @@ void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
     lookup_passes(e);
     if (e.profiling) {
         compress_pass(e);
-        stage(e, K_ANN_INSERT, [&] { launch_ann_insert(e, e.stream, 1); });
+        insert_pass(e);
         stage(e, K_MERGE_STATS, [&] { launch_merge_stats(e, e.stream, with_core, 1); });
     } else {
         cudaEventRecord(e.branch_ev, e.stream);
@@ -184,7 +199,7 @@ void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
         cudaEventRecord(e.merge_ev, e.side);
         compress_pass(e);
         if (e.sys.rdm) cudaStreamWaitEvent(e.stream, e.freed_ev, 0);
-        launch_ann_insert(e, e.stream, 1);
+        insert_pass(e);
         cudaStreamWaitEvent(e.stream, e.merge_ev, 0);
     }
     if (e.sys.rdm) stage(e, K_RDM, [&] { launch_rdm(e, e.stream); });
@@ -505,6 +520,13 @@ int32_t neci_gpu_set_tmat(neci_gpu_ctx *ctx, const double *t) {
     if (int r = dalloc(e, &d32, n)) return r;
     CK(cudaMemcpyAsync(d32, t32.data(), n * sizeof(float), cudaMemcpyHostToDevice, e.stream));
     CK(cudaStreamSynchronize(e.stream));
+    std::vector<double> diag(e.sys.nbasis + 1, 0.0);
+    for (int o = 1; o <= e.sys.nbasis; ++o) diag[o] = t[(size_t)(o - 1) * e.sys.nbasis + (o - 1)];
+    double *dd = nullptr;
+    if (int r = dalloc(e, &dd, diag.size())) return r;
+    CK(cudaMemcpyAsync(dd, diag.data(), diag.size() * sizeof(double), cudaMemcpyHostToDevice, e.stream));
+    CK(cudaStreamSynchronize(e.stream));
+    e.sys.tdiag = dd;
     e.sys.tmat = d;
     e.sys.tmat32 = d32;
     if (e.sys.system == NECI_SYS_HUBBARD_REAL_SPACE) e.h_tmat.assign(t, t + n);
@@ -969,6 +991,19 @@ static void update_merge_blocks(Engine &e, const neci_gpu_iter_stats &last) {
     }
 }
 
+// Whether the next steps take the annihilation's kernels of a short spawn list,
+// from the last step's records, with a margin so that the choice does not
+// flap.
+static void update_short_list(Engine &e, const neci_gpu_iter_stats &last) {
+    auto below = [&](bool now, long long line) { return last.n_spawned <= (now ? line : line - line / 4); };
+    const bool gather = below(e.gather, kGatherSpawns), small = below(e.short_list, kShortSpawns);
+    if (gather != e.gather || small != e.short_list) {
+        e.gather = gather;
+        e.short_list = small;
+        drop_graphs(e);
+    }
+}
+
 // Compaction of the walker list runs between calls, before the first step
 // of a call whose last step left more holes than occupied slots (the rule
 // k_final applies to Control::compact; the compaction kernels check that
@@ -1041,6 +1076,7 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         done += batch;
         update_fuse_probe(e, stats[done - 1]);
         update_merge_blocks(e, stats[done - 1]);
+        update_short_list(e, stats[done - 1]);
         update_compact_due(e, stats[done - 1]);
         if (done < n_iter) compact_if_due(e, e.stream);
     }
@@ -1157,6 +1193,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         if (!first_err) {
             update_fuse_probe(e, e.h_stats[n_iter - 1]);
             update_merge_blocks(e, e.h_stats[n_iter - 1]);
+            update_short_list(e, e.h_stats[n_iter - 1]);
             update_compact_due(e, e.h_stats[n_iter - 1]);
         }
     }

@@ -146,6 +146,7 @@ struct DevSys {
     // electron's number can overflow its 32 bits
     const ulonglong2 *hash_tab;
     const double *tmat;            // TMat2D column-major
+    const double *tdiag;           // its diagonal by orbital, 1-based
     const double *umat;            // UMAT, UMatInd - 1
     const int32_t *neighbours;     // [nsites * max_neigh], 1-based site, 0 = none
     const LatTab *lat;             // lattices with one coupling for all neighbours, else null
@@ -741,14 +742,16 @@ __device__ inline double sltcnd_2(const DevSys &s, int i, int j, int a, int b) {
 // nI array: the one-electron sum, then for each electron i the Coulomb sum
 // over j > i added to hel_doub, while the exchange terms of the same pairs,
 // in the same (i, j) order, go to their own sum.
-__device__ inline double sltcnd_0(const DevSys &s, const unsigned long long *d, int W) {
+// jm, km: <ij|ij> and <ij|ji> of the spatial orbitals; hd: <o|h|o> by orbital.
+__device__ inline double sltcnd_0(const unsigned long long *d, int W, int nBI, const double *jm, const double *km,
+                                  const double *hd) {
     double hel_sing = 0.0;
     NECI_FOR_WORDS(w, W) {
         unsigned long long x = d[w];
         while (x) {
             const int o = w * 64 + __ffsll((long long)x);
             x &= x - 1;
-            hel_sing += tmat_el(s, o, o);
+            hel_sing += hd[o];
         }
     }
     double hel_doub = 0.0, hel_tmp = 0.0;
@@ -758,15 +761,15 @@ __device__ inline double sltcnd_0(const DevSys &s, const unsigned long long *d, 
             const int oi = wi * 64 + __ffsll((long long)xi);
             xi &= xi - 1;
             double t = 0.0;
-            const size_t ri = (size_t)(spat(oi) - 1) * s.nBI - 1;
+            const int ri = (spat(oi) - 1) * nBI - 1;
             NECI_FOR_WORDS(wj, W) {
                 if (wj < wi) continue;
                 unsigned long long xj = wj == wi ? xi : d[wj];  // the electrons after i
                 while (xj) {
                     const int oj = wj * 64 + __ffsll((long long)xj);
                     xj &= xj - 1;
-                    t += __ldg(&s.jmat[ri + spat(oj)]);  // <ij|ij>
-                    if (beta(oi) == beta(oj)) hel_tmp -= __ldg(&s.kmat[ri + spat(oj)]);  // <ij|ji>
+                    t += jm[ri + spat(oj)];  // <ij|ij>
+                    if (beta(oi) == beta(oj)) hel_tmp -= km[ri + spat(oj)];  // <ij|ji>
                 }
             }
             hel_doub += t;  // the last electron adds t = 0
@@ -782,7 +785,7 @@ __device__ inline double diag_helement(const DevSys &s, const unsigned long long
         NECI_FOR_WORDS(w, s.W) n += __popcll(d[w] & (d[w] >> 1) & 0x5555555555555555ull);
         return s.uhub * n;
     }
-    return sltcnd_0(s, d, s.W) + s.ecore;
+    return sltcnd_0(d, s.W, s.nBI, s.jmat, s.kmat, s.tdiag) + s.ecore;
 }
 
 // <D_a|H|D_b> for a != b, given the excitation level.

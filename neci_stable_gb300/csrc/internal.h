@@ -31,6 +31,14 @@ enum KernelId {
     K_NUM
 };
 
+// Spawn records of a step up to which its annihilation takes the kernels of a
+// short list, measured on both sides of the lines: lookup and compression in
+// one (k_ann_gather: 19 against 33 us at 1.5e5 records, 49 against 69 at
+// 3e5, 116 against 107 at 1.4e6), decision and placement in one (k_ann_new:
+// 26 against 39 us at 1.5e5 records, 90 against 60 at 3e5).
+constexpr long long kGatherSpawns = 600000;
+constexpr long long kShortSpawns = 200000;
+
 struct Engine {
     neci_gpu_system desc{};
     DevSys sys{};
@@ -51,6 +59,9 @@ struct Engine {
     // blocks per SM (DevState::comp_shift holds the table load setting)
     int spawn_occ = 8;
     int sort_bpsm = 2;
+    // the last step's spawn list was short: lookup and compression, decision
+    // and placement in one kernel each (update_short_list)
+    bool gather = true, short_list = true;
     int merge_bpsm = 2;  // merge sweep blocks per SM beside the placement (update_merge_blocks)
     bool compact_due = false;  // the last step left more holes than occupied slots
     bool rehash_due = false;   // ... or the walker hash over its load
@@ -118,6 +129,8 @@ void launch_core(Engine &e, cudaStream_t s);
 void launch_ann_probe(Engine &e, cudaStream_t s);
 void launch_ann_compress(Engine &e, cudaStream_t s);
 void launch_ann_insert(Engine &e, cudaStream_t s, int split);
+void launch_ann_gather(Engine &e, cudaStream_t s);
+void launch_ann_new(Engine &e, cudaStream_t s, int split);
 void launch_merge_stats(Engine &e, cudaStream_t s, int with_core, int split);
 void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split);
 void launch_rdm(Engine &e, cudaStream_t s);

@@ -30,6 +30,7 @@
 //   k_final        collect estimators into the step's stats record, reset the
 //                  per-step counters, clear the walker hash if its load is
 //                  high (the next sweep refills it)
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 
@@ -781,6 +782,32 @@ __global__ void __launch_bounds__(256) k_core_sum(DevSys s, DevState st, const I
 // ===========================================================================
 // Annihilation pass 1: probe the walker hash with every spawn record.
 // ===========================================================================
+// One record: its |amplitude| to aq, the lookup, and for a determinant of the
+// list its amplitude, count and initiator bit to the slot's sums.  Returns
+// whether it was found (h: its hash).
+template <int LR>
+__device__ inline bool probe_record(const DevSys &s, const DevState &st, const long long *rec, const int32_t *rh2,
+                                    unsigned long long &h, unsigned long long (&aq)[2]) {
+    constexpr int L = LR;
+    const int W = s.W;
+    unsigned long long d[kMaxWords];
+    NECI_FOR_WORDS(w, W) d[w] = (unsigned long long)rec[w];
+    long long q[2] = {0, 0};
+    NECI_FOR_RUNS(k, L) q[k] = rec[W + k];
+    const long long fl = rec[W + L];
+    NECI_FOR_RUNS(k, L) aq[k] += (unsigned long long)(q[k] < 0 ? -q[k] : q[k]);
+    h = neci_hash(d, W, rh2);
+    const long long slot = hash_find(st, d, W, s.R, h, st.ctl);
+    if (slot < 0) return false;
+    NECI_FOR_RUNS(k, L) {
+        if (q[k] == 0) continue;
+        atomicAdd((unsigned long long *)&st.acc[slot * L + k], (unsigned long long)q[k]);
+        atomicAdd(&st.meta[slot * L + k], 1u);
+        if (test_bit(fl, init_flag_bit(k))) atomicOr(&st.meta[slot * L + k], 0x80000000u);
+    }
+    return true;
+}
+
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).
 template <int LR>
 __global__ void __launch_bounds__(256) k_ann_probe(DevSys s, DevState st) {
@@ -819,26 +846,7 @@ __global__ void __launch_bounds__(256) k_ann_probe(DevSys s, DevState st) {
         bool cand = false;
         unsigned long long h = 0;
         if (i < n) {
-            const long long *rec = st.spawn + i * R;
-            unsigned long long d[kMaxWords];
-            NECI_FOR_WORDS(w, W) d[w] = (unsigned long long)rec[w];
-            long long q[2] = {0, 0};
-            NECI_FOR_RUNS(k, L) q[k] = rec[W + k];
-            const long long fl = rec[W + L];
-            NECI_FOR_RUNS(k, L) aq[k] += (unsigned long long)(q[k] < 0 ? -q[k] : q[k]);
-            h = neci_hash(d, W, sh_rh2);
-            const long long slot = hash_find(st, d, W, R, h, c);
-            if (slot >= 0) {
-                NECI_FOR_RUNS(k, L) {
-                    if (q[k] == 0) continue;
-                    atomicAdd((unsigned long long *)&st.acc[slot * L + k], (unsigned long long)q[k]);
-                    const uint32_t add = 1u;
-                    atomicAdd(&st.meta[slot * L + k], add);
-                    if (test_bit(fl, init_flag_bit(k))) atomicOr(&st.meta[slot * L + k], 0x80000000u);
-                }
-            } else {
-                cand = true;
-            }
+            cand = !probe_record<LR>(s, st, st.spawn + i * R, sh_rh2, h, aq);
         }
         const unsigned int m = __ballot_sync(0xffffffffu, cand);
         if (cand) {
@@ -857,6 +865,23 @@ __global__ void __launch_bounds__(256) k_ann_probe(DevSys s, DevState st) {
 // ===========================================================================
 // Annihilation pass 2: merge candidates per determinant.
 // ===========================================================================
+// A record's part in the sums of its determinant's block (`owner`).
+template <int LR>
+__device__ inline void add_to_block(const DevState &st, const long long *rec, int W, long long owner) {
+    constexpr int L = LR;
+    const long long fl = rec[W + L];
+    atomicAdd(&st.rep_cnt[owner * (L + 1) + L], 1u);  // records in the block
+    NECI_FOR_RUNS(k, L) {
+        // FindResidualParticle ORs a record's initiator bit of a
+        // run into the block whatever its amplitude in that run
+        if (test_bit(fl, init_flag_bit(k))) atomicOr(&st.rep_cnt[owner * (L + 1) + k], 0x80000000u);
+        const long long q = rec[W + k];
+        if (q == 0) continue;
+        atomicAdd((unsigned long long *)&st.rep_q[owner * L + k], (unsigned long long)q);
+        atomicAdd(&st.rep_cnt[owner * (L + 1) + k], 1u);
+    }
+}
+
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).
 template <int LR>
 __global__ void __launch_bounds__(256) k_ann_compress(DevSys s, DevState st) {
@@ -916,17 +941,7 @@ __global__ void __launch_bounds__(256) k_ann_compress(DevSys s, DevState st) {
             if (owner < 0) {
                 set_err(c, NECI_GPU_ERR_HASH_FULL);
             } else {
-                const long long fl = rec[W + L];
-                atomicAdd(&st.rep_cnt[owner * (L + 1) + L], 1u);  // records in the block
-                NECI_FOR_RUNS(k, L) {
-                    // FindResidualParticle ORs a record's initiator bit of a
-                    // run into the block whatever its amplitude in that run
-                    if (test_bit(fl, init_flag_bit(k))) atomicOr(&st.rep_cnt[owner * (L + 1) + k], 0x80000000u);
-                    const long long q = rec[W + k];
-                    if (q == 0) continue;
-                    atomicAdd((unsigned long long *)&st.rep_q[owner * L + k], (unsigned long long)q);
-                    atomicAdd(&st.rep_cnt[owner * (L + 1) + k], 1u);
-                }
+                add_to_block<LR>(st, rec, W, owner);
             }
         }
         const unsigned int m = __ballot_sync(0xffffffffu, won);
@@ -959,6 +974,147 @@ __global__ void __launch_bounds__(256) k_ann_compress(DevSys s, DevState st) {
 // only, so its high half is never this.
 constexpr uint32_t kOwnFlags = 0xFFFFFFFFu;
 
+// A survivor on its way into the list.
+struct Placed {
+    unsigned long long d[kMaxWords], h;
+    double sign[2];
+    long long flags;
+};
+struct DecideSums {
+    double ab[2] = {0, 0}, rm[2] = {0, 0}, born[2] = {0, 0};
+    unsigned long long s[2] = {0, 0}, nz = 0;
+};
+struct PlaceSums {
+    double tp[2] = {0, 0}, norm[2] = {0, 0};
+    long long tomb = 0;  // tombstones taken over by the insertions (a negative count)
+    unsigned long long added = 0;
+};
+
+// The decision on one unique determinant (candidate ci, compression bucket
+// rb): whether it survives; then w holds its words, signs and the flag word
+// of a block of several records, and nrec the number of records (a block of
+// one keeps its record's flag word, which the caller reads).
+template <int LR>
+__device__ inline bool decide_one(const DevSys &s, const DevState &st, const IterParams &p, long long ci, uint32_t rb,
+                                  Placed &w, uint32_t &nrec, const long long *&rec, DecideSums &a) {
+    const int W = s.W;
+    constexpr int L = LR;
+    if (rb != kNoBucket) st.spawn_hash[rb] = kEmpty;  // leave the table clean
+    long long q[2] = {0, 0};
+    uint32_t cnt[2] = {0, 0};
+    NECI_FOR_RUNS(k, L) {
+        q[k] = st.rep_q[ci * L + k];
+        cnt[k] = st.rep_cnt[ci * (L + 1) + k];
+    }
+    nrec = st.rep_cnt[ci * (L + 1) + L];
+    w.flags = 0;
+    w.sign[0] = w.sign[1] = 0.0;
+    // compressed flags (CompressSpawnedList / FindResidualParticle): a block
+    // of one record keeps that record's flag word; its initiator bit in a
+    // run with a non-zero amplitude is the one in the run's count, so the
+    // counts decide the abort for every block without the record
+    if (p.t_trunc_initiator)
+        NECI_FOR_RUNS(k, L) {
+            const bool coh = p.t_init_coherent_rule && (cnt[k] & 0x7FFFFFFFu) >= 2u;
+            if (coh || (cnt[k] & 0x80000000u)) w.flags |= 1ll << init_flag_bit(k);
+        }
+    bool zero = true;
+    NECI_FOR_RUNS(k, L) {
+        if (q[k] != 0) zero = false;
+        a.s[k] += (unsigned long long)(q[k] < 0 ? -q[k] : q[k]);
+    }
+    a.nz += zero ? 0ull : 1ull;
+    if (zero) return false;
+    w.sign[0] = from_fixed(q[0]);
+    w.sign[1] = from_fixed(q[1]);
+    if (p.t_trunc_initiator)
+        NECI_FOR_RUNS(k, L)
+            if (!test_bit(w.flags, init_flag_bit(k))) { a.ab[k] += fabs(w.sign[k]); w.sign[k] = 0.0; }
+    bool unocc = true;
+    NECI_FOR_RUNS(k, L) if (abs_bits(w.sign[k]) >= dbl_bits(kEps12)) unocc = false;
+    if (unocc) return false;
+    rec = st.spawn + (long long)st.cand[ci] * s.R;
+    NECI_FOR_WORDS(i, W) w.d[i] = (unsigned long long)rec[i];
+    const unsigned long long dkey = det_key(w.d, W, p.seed);
+    bool want = false;
+    NECI_FOR_RUNS(k, L) {
+        // stochRoundSpawn (Annihilation.F90:1354-1418)
+        const double c = abs_dbl(w.sign[k]);
+        if (abs_bits(c) > dbl_bits(kEps12) && abs_bits(c) < dbl_bits(p.occupied_thresh)) {
+            Stream rng(dkey, p.iter, P_ANN_ROUND, k, 0);
+            const double pRemove =
+                1.0 - (dbl_bits(p.occupied_thresh) == dbl_bits(1.0) ? c : div_dbl(c, p.occupied_thresh));
+            if (bern(rng, pRemove)) { a.rm[k] += c; w.sign[k] = 0.0; }
+            else { a.born[k] += p.occupied_thresh - c; w.sign[k] = fsign(p.occupied_thresh, w.sign[k]); }
+        }
+        if (abs_bits(w.sign[k]) >= dbl_bits(kEps12)) want = true;
+    }
+    return want;
+}
+
+// AddNewHashDet for one survivor, the rank-th of a warp's batch: t0 and f0 are
+// the batch's first places on the free list's cursor and among the fresh
+// slots.  split: the merge sweep skips the new determinants (it runs beside
+// the placement), so their |C| and C^2 (TotParts, norm) and the reference's
+// sign are taken here.
+template <int LR>
+__device__ inline void place_one(const DevSys &s, const DevState &st, const Placed &w, unsigned long long t0,
+                                 unsigned long long f0, unsigned long long nfree, unsigned int rank, double dh,
+                                 double odh, bool rdm, int split, PlaceSums &a) {
+    Control *c = st.ctl;
+    const int W = s.W;
+    constexpr int L = LR;
+    const unsigned long long t = t0 + rank;
+    const unsigned long long first_fresh = t0 >= nfree ? t0 : nfree;  // the first t that gets a fresh slot
+    const long long slot = t < nfree ? (long long)st.free_list[t] : (long long)(f0 + (t - first_fresh));
+    if (slot + 1 >= st.max_walkers) {
+        set_err(c, NECI_GPU_ERR_LIST_FULL);
+        return;
+    }
+    long long *o = st.dets + slot * s.R;
+    NECI_FOR_WORDS(i, W) o[i] = (long long)w.d[i];
+    NECI_FOR_RUNS(k, L) o[W + k] = double_to_word(w.sign[k]);
+    o[W + L] = w.flags & ~1ll;
+    st.diagH[slot] = dh;
+    st.offdiagH[slot] = odh;
+    if (st.n_core > 0) st.core_of_slot[slot] = -1;
+    if (rdm) st.rdm_w[slot] = w.sign[0] * w.sign[1];
+    a.tomb -= hash_insert(st, slot, w.h, c);
+    ++a.added;
+    if (split) {
+        bool is_ref = true;
+        NECI_FOR_WORDS(i, W) if (w.d[i] != s.ilut_ref[i]) is_ref = false;
+        NECI_FOR_RUNS(k, L) {
+            const double v = w.sign[k];
+            a.tp[k] += fabs(v);
+            a.norm[k] = fma(v, v, a.norm[k]);  // a statistic: one rounding, one FP64 instruction
+            if (is_ref) c->noat_hf[k] = v;
+        }
+    }
+}
+
+template <int LR>
+__device__ inline void add_decide_sums(Control *c, const DecideSums &a) {
+    double v[6] = {a.ab[0], a.ab[1], a.rm[0], a.rm[1], a.born[0], a.born[1]};
+    double *const dst[6] = {&c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
+                            &c->nborn[0], &c->nborn[1]};
+    block_add<6>(v, dst, LR);
+    unsigned long long u[3] = {a.s[0], a.s[1], a.nz};
+    unsigned long long *const du[3] = {&c->abs_s[0], &c->abs_s[1], &c->n_reps_nz};
+    block_add_u<3>(u, du);
+}
+template <int LR>
+__device__ inline void add_place_sums(Control *c, const PlaceSums &a, int split) {
+    unsigned long long u[2] = {(unsigned long long)a.tomb, a.added};  // two's complement for -count
+    unsigned long long *const du[2] = {&c->n_tomb, &c->n_new};
+    block_add_u<2>(u, du);
+    if (split) {
+        double v[4] = {a.tp[0], a.tp[1], a.norm[0], a.norm[1]};
+        double *const dst[4] = {&c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
+        block_add<4>(v, dst, LR);
+    }
+}
+
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).
 template <int LR>
 __global__ void __launch_bounds__(256) k_ann_decide(DevSys s, DevState st, const IterParams *pp) {
@@ -968,72 +1124,19 @@ __global__ void __launch_bounds__(256) k_ann_decide(DevSys s, DevState st, const
     // the appends count past the allocation when it overflows (SPAWN_FULL is
     // reported at the end of the step): only the entries written are read
     const long long n = (long long)min(c->n_reps, (unsigned long long)st.max_spawned);
-    const int W = s.W, R = s.R;
     constexpr int L = LR;
-    double a_ab[2] = {0, 0}, a_rm[2] = {0, 0}, a_born[2] = {0, 0};
-    unsigned long long a_s[2] = {0, 0}, a_nz = 0;
+    DecideSums ds;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long nround = ((n + stride - 1) / stride) * stride;
     for (long long ri = blockIdx.x * (long long)blockDim.x + threadIdx.x; ri < nround; ri += stride) {
         bool want = false;
         long long ci = 0;
-        double ss[2] = {0.0, 0.0};
-        long long flags = 0;
-        uint32_t nrec = 0;
         if (ri < n) {
             ci = st.reps[ri];
-            const uint32_t rb = st.rep_bucket[ri];
-            if (rb != kNoBucket) st.spawn_hash[rb] = kEmpty;  // leave the table clean
-            long long q[2] = {0, 0};
-            uint32_t cnt[2] = {0, 0};
-            NECI_FOR_RUNS(k, L) {
-                q[k] = st.rep_q[ci * L + k];
-                cnt[k] = st.rep_cnt[ci * (L + 1) + k];
-            }
-            nrec = st.rep_cnt[ci * (L + 1) + L];
-            // compressed flags (CompressSpawnedList / FindResidualParticle):
-            // a block of one record keeps that record's flag word, read by
-            // k_ann_place for the survivors only; its initiator bit in a run
-            // with a non-zero amplitude is the one in the run's count, so the
-            // counts decide the abort for every block without the record
-            if (p.t_trunc_initiator)
-                NECI_FOR_RUNS(k, L) {
-                    const bool coh = p.t_init_coherent_rule && (cnt[k] & 0x7FFFFFFFu) >= 2u;
-                    if (coh || (cnt[k] & 0x80000000u)) flags |= 1ll << init_flag_bit(k);
-                }
-            bool zero = true;
-            NECI_FOR_RUNS(k, L) {
-                if (q[k] != 0) zero = false;
-                a_s[k] += (unsigned long long)(q[k] < 0 ? -q[k] : q[k]);
-            }
-            a_nz += zero ? 0ull : 1ull;
-            if (!zero) {
-                ss[0] = from_fixed(q[0]);
-                ss[1] = from_fixed(q[1]);
-                if (p.t_trunc_initiator)
-                    NECI_FOR_RUNS(k, L)
-                        if (!test_bit(flags, init_flag_bit(k))) { a_ab[k] += fabs(ss[k]); ss[k] = 0.0; }
-                bool unocc = true;
-                NECI_FOR_RUNS(k, L) if (abs_bits(ss[k]) >= dbl_bits(kEps12)) unocc = false;
-                if (!unocc) {
-                    const long long *rec = st.spawn + (long long)st.cand[ci] * R;
-                    unsigned long long d[kMaxWords];
-                    NECI_FOR_WORDS(w, W) d[w] = (unsigned long long)rec[w];
-                    const unsigned long long dkey = det_key(d, W, p.seed);
-                    NECI_FOR_RUNS(k, L) {
-                        // stochRoundSpawn (Annihilation.F90:1354-1418)
-                        const double a = abs_dbl(ss[k]);
-                        if (abs_bits(a) > dbl_bits(kEps12) && abs_bits(a) < dbl_bits(p.occupied_thresh)) {
-                            Stream rng(dkey, p.iter, P_ANN_ROUND, k, 0);
-                            const double pRemove =
-                                1.0 - (dbl_bits(p.occupied_thresh) == dbl_bits(1.0) ? a : div_dbl(a, p.occupied_thresh));
-                            if (bern(rng, pRemove)) { a_rm[k] += a; ss[k] = 0.0; }
-                            else { a_born[k] += p.occupied_thresh - a; ss[k] = fsign(p.occupied_thresh, ss[k]); }
-                        }
-                    }
-                    NECI_FOR_RUNS(k, L) if (abs_bits(ss[k]) >= dbl_bits(kEps12)) want = true;
-                }
-            }
+            Placed w;
+            uint32_t nrec;
+            const long long *rec = nullptr;
+            want = decide_one<LR>(s, st, p, ci, st.rep_bucket[ri], w, nrec, rec, ds);
             // the sums are consumed: cleared for the next step, or, for a
             // survivor, replaced by its signs (as double bits) and its flag
             // word (low half in the record count's place, high half in the
@@ -1041,11 +1144,11 @@ __global__ void __launch_bounds__(256) k_ann_decide(DevSys s, DevState st, const
             // whose own flag word k_ann_place reads) for k_ann_place, which
             // clears them
             NECI_FOR_RUNS(k, L) {
-                st.rep_q[ci * L + k] = want ? double_to_word(ss[k]) : 0ll;
+                st.rep_q[ci * L + k] = want ? double_to_word(w.sign[k]) : 0ll;
                 st.rep_cnt[ci * (L + 1) + k] = 0u;
             }
-            if (want) st.rep_cnt[ci * (L + 1)] = nrec == 1 ? kOwnFlags : (uint32_t)((unsigned long long)flags >> 32);
-            st.rep_cnt[ci * (L + 1) + L] = want ? (uint32_t)flags : 0u;
+            if (want) st.rep_cnt[ci * (L + 1)] = nrec == 1 ? kOwnFlags : (uint32_t)((unsigned long long)w.flags >> 32);
+            st.rep_cnt[ci * (L + 1) + L] = want ? (uint32_t)w.flags : 0u;
         }
         const unsigned long long pos = warp_append1(&c->n_place, want);
         if (want) {
@@ -1053,51 +1156,40 @@ __global__ void __launch_bounds__(256) k_ann_decide(DevSys s, DevState st, const
             else set_err(c, NECI_GPU_ERR_SPAWN_FULL);
         }
     }
-    double v[6] = {a_ab[0], a_ab[1], a_rm[0], a_rm[1], a_born[0], a_born[1]};
-    double *const dst[6] = {&c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
-                            &c->nborn[0], &c->nborn[1]};
-    block_add<6>(v, dst, L);
-    unsigned long long u[3] = {a_s[0], a_s[1], a_nz};
-    unsigned long long *const du[3] = {&c->abs_s[0], &c->abs_s[1], &c->n_reps_nz};
-    block_add_u<3>(u, du);
+    add_decide_sums<LR>(c, ds);
 }
 
-// split: the merge sweep skips the new determinants (it runs beside this
-// kernel), so their |C| and C^2 (TotParts, norm) and the reference's sign
-// are taken here.
 template <int LR>
 __global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, const IterParams *pp, int split) {
     if (halted(st)) return;
     const bool rdm = LR == 2 && split && s.rdm && pp->rdm_defer;
     Control *c = st.ctl;
-    double a_tp[2] = {0.0, 0.0}, a_norm[2] = {0.0, 0.0};
     const long long n = (long long)min(c->n_place, (unsigned long long)st.max_spawned);
     const int W = s.W, R = s.R;
     constexpr int L = LR;
     const int lane = threadIdx.x & 31;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long nround = ((n + stride - 1) / stride) * stride;
-    long long a_tomb = 0;  // tombstones taken over by the insertions (a negative count)
-    unsigned long long a_new = 0;
+    PlaceSums ps;
     for (long long pi = blockIdx.x * (long long)blockDim.x + threadIdx.x; pi < nround; pi += stride) {
         const bool want = pi < n;
         // the determinant, its signs and flag word (cleared from the sums'
         // slots) and its hash
-        unsigned long long d[kMaxWords], h = 0;
-        long long ws[2] = {0, 0}, flags = 0;
-        NECI_FOR_WORDS(w, W) d[w] = 0ull;
+        Placed w;
+        NECI_FOR_WORDS(i, W) w.d[i] = 0ull;
         if (want) {
             const long long ci = st.place[pi];
             const long long *rec = st.spawn + (long long)st.cand[ci] * R;
-            NECI_FOR_WORDS(w, W) d[w] = (unsigned long long)rec[w];
-            h = st.cand_h[ci];
+            NECI_FOR_WORDS(i, W) w.d[i] = (unsigned long long)rec[i];
+            w.h = st.cand_h[ci];
+            w.sign[0] = w.sign[1] = 0.0;
             NECI_FOR_RUNS(k, L) {
-                ws[k] = st.rep_q[ci * L + k];
+                w.sign[k] = word_to_double(st.rep_q[ci * L + k]);
                 st.rep_q[ci * L + k] = 0;
             }
             const uint32_t hi = st.rep_cnt[ci * (L + 1)];
-            flags = hi == kOwnFlags ? rec[W + L]
-                                    : (long long)(((unsigned long long)hi << 32) | st.rep_cnt[ci * (L + 1) + L]);
+            w.flags = hi == kOwnFlags ? rec[W + L]
+                                      : (long long)(((unsigned long long)hi << 32) | st.rep_cnt[ci * (L + 1) + L]);
             st.rep_cnt[ci * (L + 1)] = 0u;
             st.rep_cnt[ci * (L + 1) + L] = 0u;
         }
@@ -1118,51 +1210,209 @@ __global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, const 
         }
         double dh = 0.0, odh = 0.0;
         if (want) {
-            dh = diag_helement(s, d) - s.hii;
-            const int ic = excit_level(s.ilut_ref, d, W);
-            odh = (ic >= 1 && ic <= 2) ? offdiag_helement(s, s.ilut_ref, d, ic) : 0.0;
+            dh = diag_helement(s, w.d) - s.hii;
+            const int ic = excit_level(s.ilut_ref, w.d, W);
+            odh = (ic >= 1 && ic <= 2) ? offdiag_helement(s, s.ilut_ref, w.d, ic) : 0.0;
         }
         if (nwant) {
             t0 = __shfl_sync(0xffffffffu, t0, leader);
             f0 = __shfl_sync(0xffffffffu, f0, leader);
         }
-        if (!want) continue;
-        const unsigned long long t = t0 + rank;
-        const unsigned long long first_fresh = t0 >= nfree ? t0 : nfree;  // the first t that gets a fresh slot
-        const long long slot = t < nfree ? (long long)st.free_list[t] : (long long)(f0 + (t - first_fresh));
-        if (slot + 1 >= st.max_walkers) {
-            set_err(c, NECI_GPU_ERR_LIST_FULL);
-            continue;
+        if (want) place_one<LR>(s, st, w, t0, f0, nfree, rank, dh, odh, rdm, split, ps);
+    }
+    add_place_sums<LR>(c, ps, split);
+}
+
+// ===========================================================================
+// The annihilation of a short spawn list in two kernels instead of four: a
+// step of up to some 1e5 records is bound by the latency of its kernels
+// (launch, first loads, reductions: 7 to 10 us each whatever they do), not by
+// their work (kGatherSpawns, kShortSpawns).
+//   k_ann_gather  passes 1 and 2: each record is looked up in the walker hash;
+//                 the absent ones wait in shared memory until a warp has 32
+//                 (so that the merge has full lanes) and are merged per
+//                 determinant in the compression table, keyed on the record
+//                 (candidate number = record number)
+//   k_ann_new     pass 3: decision and placement, the survivors of a block's
+//                 256 decisions packed into as few warps as hold them
+// Longer lists keep the four kernels, each with its own occupancy.
+// ===========================================================================
+template <int LR>
+__global__ void __launch_bounds__(128) k_ann_gather(DevSys s, DevState st) {
+    Control *c = st.ctl;
+    const int stop = c->halted;
+    const long long n = (long long)min(c->n_spawned, (unsigned long long)st.max_spawned);
+    if (stop || n <= (long long)blockIdx.x * blockDim.x) return;
+    extern __shared__ int32_t sh_rh2[];
+    __shared__ uint32_t wait_i[4][64];
+    __shared__ unsigned long long wait_h[4][64];
+    load_rh2(s, sh_rh2);
+    const int W = s.W, R = s.R;
+    constexpr int L = LR;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long hn = 1024;
+    while (hn < ((unsigned long long)n << st.comp_shift) && hn < st.spawn_hash_n) hn <<= 1;
+    const unsigned long long mask = (hn < st.spawn_hash_n ? hn : st.spawn_hash_n) - 1;
+    unsigned long long aq[2] = {0, 0};
+    int waiting = 0;  // the same in every lane
+    // entries first .. first + m - 1 of the warp's waiting records
+    auto merge = [&](int first, int m) {
+        bool won = false;
+        uint32_t bucket = 0;
+        long long i = 0;
+        if (lane < m) {
+            i = wait_i[wid][first + lane];
+            const unsigned long long h = wait_h[wid][first + lane];
+            const long long *rec = st.spawn + i * R;
+            unsigned long long d[kMaxWords];
+            NECI_FOR_WORDS(w, W) d[w] = (unsigned long long)rec[w];
+            unsigned long long b = splitmix64(h) & mask;
+            long long owner = -1;
+            for (int p = 0; p < kProbeLimit; ++p) {
+                const uint32_t e = atomicCAS(&st.spawn_hash[b], kEmpty, (uint32_t)(i + 1));
+                if (e == kEmpty) { owner = i; won = true; bucket = (uint32_t)b; break; }
+                if (det_eq(d, st.spawn + ((long long)e - 1) * R, W)) { owner = (long long)e - 1; break; }
+                b = (b + 1) & mask;
+            }
+            if (won) {
+                st.cand[i] = (uint32_t)i;
+                st.cand_h[i] = h;
+            }
+            if (owner < 0) set_err(c, NECI_GPU_ERR_HASH_FULL);
+            else add_to_block<LR>(st, rec, W, owner);
         }
-        long long *o = st.dets + slot * R;
-        NECI_FOR_WORDS(w, W) o[w] = (long long)d[w];
-        NECI_FOR_RUNS(k, L) o[W + k] = ws[k];
-        o[W + L] = flags & ~1ll;
-        st.diagH[slot] = dh;
-        st.offdiagH[slot] = odh;
-        if (st.n_core > 0) st.core_of_slot[slot] = -1;
-        if (rdm) st.rdm_w[slot] = word_to_double(ws[0]) * word_to_double(ws[1]);
-        a_tomb -= hash_insert(st, slot, h, c);
-        ++a_new;
-        if (split) {
-            bool is_ref = true;
-            NECI_FOR_WORDS(w, W) if (d[w] != s.ilut_ref[w]) is_ref = false;
+        const unsigned long long pos = warp_append1(&c->n_reps, won);
+        if (won) {
+            st.reps[pos] = (uint32_t)i;
+            st.rep_bucket[pos] = bucket;
+        }
+    };
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long nround = ((n + stride - 1) / stride) * stride;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nround; i += stride) {
+        bool absent = false;
+        unsigned long long h = 0;
+        if (i < n) absent = !probe_record<LR>(s, st, st.spawn + i * R, sh_rh2, h, aq);
+        const unsigned int m = __ballot_sync(0xffffffffu, absent);
+        if (absent) {
+            const int k = waiting + __popc(m & ((1u << lane) - 1u));
+            wait_i[wid][k] = (uint32_t)i;
+            wait_h[wid][k] = h;
+        }
+        waiting += __popc(m);
+        __syncwarp();
+        if (waiting >= 32) {
+            waiting -= 32;
+            merge(waiting, 32);
+            __syncwarp();
+        }
+    }
+    if (waiting > 0) merge(0, waiting);
+    unsigned long long *const dst[2] = {&c->abs_q[0], &c->abs_q[1]};
+    block_add_u<2>(aq, dst);
+}
+
+// Shared memory of k_ann_new: a block's survivors, then (molecules, where it
+// fits 32 KB: up to 44 orbitals) the Coulomb, exchange and one-electron tables
+// of the diagonal element, whose loads the element's dependent FP64 additions
+// wait for.
+constexpr int kNewThreads = 256;
+__host__ __device__ inline size_t new_table_doubles(const DevSys &s) {
+    const size_t n = 2 * (size_t)s.nBI * s.nBI + s.nbasis + 1;
+    return s.system == NECI_SYS_MOLECULAR && n * sizeof(double) <= 32 * 1024 ? n : 0;
+}
+__host__ __device__ inline size_t new_shared_bytes(const DevSys &s) {
+    return kNewThreads * sizeof(Placed) + new_table_doubles(s) * sizeof(double);
+}
+
+template <int LR>
+__global__ void __launch_bounds__(kNewThreads) k_ann_new(DevSys s, DevState st, const IterParams *pp, int split) {
+    Control *c = st.ctl;
+    const int stop = c->halted;
+    const long long n = (long long)min(c->n_reps, (unsigned long long)st.max_spawned);
+    if (stop || n <= (long long)blockIdx.x * blockDim.x) return;
+    const IterParams p = *pp;
+    const bool rdm = LR == 2 && split && s.rdm && p.rdm_defer;
+    constexpr int L = LR;
+    extern __shared__ __align__(16) unsigned char new_smem[];
+    Placed *held = reinterpret_cast<Placed *>(new_smem);
+    double *tab = reinterpret_cast<double *>(new_smem + kNewThreads * sizeof(Placed));
+    __shared__ int wcount[kNewThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nn = s.nBI * s.nBI;
+    const bool in_shared = new_table_doubles(s) != 0;
+    if (in_shared) {
+        for (int i = threadIdx.x; i < nn; i += kNewThreads) {
+            tab[i] = s.jmat[i];
+            tab[nn + i] = s.kmat[i];
+        }
+        for (int i = threadIdx.x; i <= s.nbasis; i += kNewThreads) tab[2 * nn + i] = s.tdiag[i];
+    }
+    DecideSums ds;
+    PlaceSums ps;
+    const unsigned long long nfree = c->n_free;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    // a round: one decision per thread, the survivors packed (32 to a warp:
+    // an FP64 instruction takes its pipe as long for one lane as for 32),
+    // then placed
+    for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += stride) {
+        const long long ri = base + threadIdx.x;
+        Placed w;
+        bool want = false;
+        if (ri < n) {
+            const long long ci = st.reps[ri];
+            uint32_t nrec;
+            const long long *rec = nullptr;
+            want = decide_one<LR>(s, st, p, ci, st.rep_bucket[ri], w, nrec, rec, ds);
             NECI_FOR_RUNS(k, L) {
-                const double v = word_to_double(ws[k]);
-                a_tp[k] += fabs(v);
-                a_norm[k] = fma(v, v, a_norm[k]);  // a statistic: one rounding, one FP64 instruction
-                if (is_ref) c->noat_hf[k] = v;
+                st.rep_q[ci * L + k] = 0;
+                st.rep_cnt[ci * (L + 1) + k] = 0u;
+            }
+            st.rep_cnt[ci * (L + 1) + L] = 0u;
+            if (want) {
+                if (nrec == 1) w.flags = rec[s.W + LR];
+                w.h = st.cand_h[ci];
             }
         }
+        const unsigned int m = __ballot_sync(0xffffffffu, want);
+        if (lane == 0) wcount[wid] = __popc(m);
+        __syncthreads();  // (also: the last round's survivors are placed, the tables are there)
+        int before = 0, total = 0;
+        for (int k = 0; k < kNewThreads / 32; ++k) {
+            const int x = wcount[k];
+            before += k < wid ? x : 0;
+            total += x;
+        }
+        if (want) held[before + __popc(m & ((1u << lane) - 1u))] = w;
+        __syncthreads();
+        const int left = total - 32 * wid;  // this warp's part
+        if (left > 0) {
+            const int mine = left < 32 ? left : 32;
+            // their slots: the next holes of the free list, then fresh slots
+            // at the end of the list; the elements are computed meanwhile
+            unsigned long long t0 = 0, f0 = 0;
+            if (lane == 0) {
+                t0 = atomicAdd(&c->free_taken, (unsigned long long)mine);
+                const unsigned long long from_free = t0 >= nfree ? 0ull : min(nfree - t0, (unsigned long long)mine);
+                if ((unsigned long long)mine > from_free)
+                    f0 = atomicAdd(&c->tot_walkers, (unsigned long long)mine - from_free);
+            }
+            Placed v;
+            double dh = 0.0, odh = 0.0;
+            if (lane < mine) {
+                v = held[32 * wid + lane];
+                dh = in_shared ? sltcnd_0(v.d, s.W, s.nBI, tab, tab + nn, tab + 2 * nn) + s.ecore : diag_helement(s, v.d);
+                dh -= s.hii;
+                const int ic = excit_level(s.ilut_ref, v.d, s.W);
+                odh = (ic >= 1 && ic <= 2) ? offdiag_helement(s, s.ilut_ref, v.d, ic) : 0.0;
+            }
+            t0 = __shfl_sync(0xffffffffu, t0, 0);
+            f0 = __shfl_sync(0xffffffffu, f0, 0);
+            if (lane < mine) place_one<LR>(s, st, v, t0, f0, nfree, (unsigned)lane, dh, odh, rdm, split, ps);
+        }
     }
-    unsigned long long u[2] = {(unsigned long long)a_tomb, a_new};  // two's complement for -count
-    unsigned long long *const du[2] = {&c->n_tomb, &c->n_new};
-    block_add_u<2>(u, du);
-    if (split) {
-        double v[4] = {a_tp[0], a_tp[1], a_norm[0], a_norm[1]};
-        double *const dst[4] = {&c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
-        block_add<4>(v, dst, L);
-    }
+    add_decide_sums<LR>(c, ds);
+    add_place_sums<LR>(c, ps, split);
 }
 
 // ===========================================================================
@@ -1723,6 +1973,10 @@ int configure_kernels(Engine &e) {
         return 1;
     if (cudaFuncSetAttribute(k_merge_stats<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, merge_max) != cudaSuccess)
         return 1;
+    const int new_max = (int)(kNewThreads * sizeof(Placed)) + 32 * 1024;
+    if (cudaFuncSetAttribute(k_ann_new<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, new_max) != cudaSuccess ||
+        cudaFuncSetAttribute(k_ann_new<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, new_max) != cudaSuccess)
+        return 1;
     // resident blocks per SM of each instance (the smaller of the two run counts)
     auto occ = [](const void *f1, const void *f2, int threads, size_t smem) {
         int a = 0, b = 0;
@@ -1793,6 +2047,19 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split) {
         k_ann_decide<1><<<grid_spawns(e, 256, e.occ_insert), 256, 0, s>>>(e.sys, e.st, e.d_params);
         k_ann_place<1><<<gp, 128, 0, s>>>(e.sys, e.st, e.d_params, split);
     }
+}
+// The kernels of a short spawn list (Engine::short_list).
+void launch_ann_gather(Engine &e, cudaStream_t s) {
+    const size_t shm = (e.sys.nbasis + 1) * sizeof(int32_t);
+    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kGatherSpawns) / 128 + 1, e.num_sms * 8);
+    if (e.sys.L == 2) k_ann_gather<2><<<grid, 128, shm, s>>>(e.sys, e.st);
+    else k_ann_gather<1><<<grid, 128, shm, s>>>(e.sys, e.st);
+}
+void launch_ann_new(Engine &e, cudaStream_t s, int split) {
+    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kShortSpawns) / kNewThreads + 1, e.num_sms * 4);
+    const size_t shm = new_shared_bytes(e.sys);
+    if (e.sys.L == 2) k_ann_new<2><<<grid, kNewThreads, shm, s>>>(e.sys, e.st, e.d_params, split);
+    else k_ann_new<1><<<grid, kNewThreads, shm, s>>>(e.sys, e.st, e.d_params, split);
 }
 // Blocks per SM of the merge sweep when it runs beside the placement
 // (split): e.merge_bpsm, two unless the merge sweep is the longer branch, so

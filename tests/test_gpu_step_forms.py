@@ -173,3 +173,34 @@ def test_lattice_spawn_forms(kind, lenof_sign, fuse, core, real, prec, big_hash)
             same_list(spec, eng, orc, it)
     a, b = eng.tau_stats(), orc.tau_stats()
     assert a.gamma_sing == b.gamma_sing and a.cnt_sing == b.cnt_sing
+
+
+@pytest.mark.parametrize("name,lenof_sign,walkers", [("hub", 1, 300), ("mol12", 2, 200), ("mol24", 1, 400), ("mol48", 1, 300),
+                                                     ("mol40", 2, 300)])
+def test_short_and_long_spawn_lists(name, lenof_sign, walkers):
+    # both forms of the annihilation on the same list: the short form until a
+    # step writes more records than its lines, the long form after that
+    # (determinants of 1, 2 and 3 words, diagonal tables that fit shared
+    # memory and that do not)
+    spec = hubbard10(lenof_sign=lenof_sign) if name == "hub" else molecule(int(name[3:]), 8, lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 21, 1 << 22)
+    orc = Oracle(spec, 1 << 21, 1 << 22, hii=eng.hii)
+    rng = np.random.default_rng(12)
+    rows = random_walkers(spec, walkers, rng)
+    W, L = spec.W, spec.lenof_sign
+    for scale, tau, steps in ((1.0, 0.005, 3), (400.0, 0.02, 2), (1600.0, 0.02, 2)):
+        if scale > 400.0 and name not in ("mol24", "mol40"):
+            continue
+        v = rows[:, W:W + L].view(np.float64) * scale
+        r = rows.copy()
+        r[:, W:W + L] = np.ascontiguousarray(v).view(np.int64)
+        eng.upload(r)
+        orc.upload(r)
+        for it in range(1, steps + 1):
+            p = capi.default_params(tau=tau, seed=29, iter=it)
+            sg = eng.perform_fcimc_cyc_par(p)
+            sc, rc = orc.iterate(p)
+            assert rc == 0 and sg.err == 0
+            for f in ("n_attempts", "n_spawned", "n_unique", "n_new", "n_occupied"):
+                assert getattr(sg, f) == getattr(sc, f), (f, it, scale)
+            same_list(spec, eng, orc, (it, scale))
