@@ -50,38 +50,111 @@ __device__ inline float umat_r<float>(const DevSys &s, int i, int j, int k, int 
     return __ldg(&s.umat32[umat_ind(i, j, k, l) - 1]);
 }
 
+// -x on the sign bit (as an FP64 operation it would hold the FP64 pipe).
+__device__ inline double negate(double x) { return neg_dbl(x); }
+__device__ inline float negate(float x) { return -x; }
+
+// The electrons of a determinant in ascending order, one by one.
+template <int NW>
+struct Electrons {
+    unsigned long long x[NW];
+    __device__ inline int next() {  // 0-based orbital
+        int w = 0;
+        unsigned long long v = x[0];
+#pragma unroll
+        for (int k = 1; k < NW; ++k)
+            if (v == 0ull) {
+                v = x[k];
+                w = k;
+            }
+        const int b = 64 * w + __ffsll((long long)v) - 1;
+        v &= v - 1;
+#pragma unroll
+        for (int k = 0; k < NW; ++k)
+            if (w == k) x[k] = v;
+        return b;
+    }
+};
+
 // sltcnd_1_kernel (sltcnd.fpp:643-679) in precision Real, summed as the
-// FP64 form (one add per occupied k of jrow[k] or, same spin, jkrow[k]).
+// FP64 form (one add per occupied k of jrow[k] or, same spin, jkrow[k], in
+// ascending order).  Every determinant has nel - 1 such k, so with the words
+// in registers the loop's trip count is the same for all lanes and no
+// addition is predicated: GB300's FP64 pipe (about one lane per clock per SM)
+// is held as long by a predicated-off addition as by one that counts, and the
+// singles' additions bound the spawn kernel once the tau search has raised
+// pSingles (n = 24: 13 FP64 additions issued a single where 9 are needed;
+// four loads are in flight at a time).  The first term is taken as it is:
+// 0 + v is v but for the sign of a zero.
 template <typename Real, int NW = 0>
 __device__ inline Real sltcnd_1_r(const DevSys &s, const unsigned long long *d, int src, int tgt) {
     Real hel = 0;
     const int id1 = spat(src), id2 = spat(tgt);
     if (beta(src) == beta(tgt)) {
-        const size_t row = ((size_t)(id1 - 1) * s.nBI + (id2 - 1)) * s.nBI - 1;
+        const size_t row = ((size_t)(id1 - 1) * s.nBI + (id2 - 1)) * s.nBI;
         const Real *jr = (sizeof(Real) == 8 ? (const Real *)s.jrow : (const Real *)s.jrow32) + row;
         const Real *jkr = (sizeof(Real) == 8 ? (const Real *)s.jkrow : (const Real *)s.jkrow32) + row;
-        const unsigned long long same = beta(src) ? kBetaBits : kAlphaBits;
-        // The occupied k other than src in increasing order, four loads in
-        // flight at a time and added in that order.
-        NECI_FOR_WORDS(w, nwords<NW>(s)) {
-            unsigned long long x = d[w];
-            if (((src - 1) >> 6) == w) x &= ~(1ull << ((src - 1) & 63));
-            while (x) {
-                Real v[4];
-                bool have[4];
+        // (FP32 with two words: the words in registers cost more than the
+        // predicated additions, 1% at n = 64)
+        if constexpr (NW == 1 || (NW > 1 && sizeof(Real) == 8)) {
+            Electrons<NW> el;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    have[u] = x != 0ull;
-                    v[u] = 0;
-                    if (have[u]) {
-                        const int b = __ffsll((long long)x) - 1;
-                        x &= x - 1;
-                        v[u] = __ldg(((same >> b) & 1ull) ? &jkr[spat(w * 64 + b + 1)] : &jr[spat(w * 64 + b + 1)]);
+            for (int w = 0; w < NW; ++w) el.x[w] = d[w];
+            {
+                const int w0 = (src - 1) >> 6;
+#pragma unroll
+                for (int w = 0; w < NW; ++w)
+                    if (w == w0) el.x[w] &= ~(1ull << ((src - 1) & 63));
+            }
+            const int odd = (src - 1) & 1;
+            auto term = [&]() {
+                const int b = el.next();
+                return __ldg(((b ^ odd) & 1 ? jr : jkr) + (b >> 1));
+            };
+            const int m = s.nel - 1;
+            hel = term();
+            int k = 1;
+            for (; k + 4 <= m; k += 4) {
+                const Real v0 = term(), v1 = term(), v2 = term(), v3 = term();
+                hel += v0;
+                hel += v1;
+                hel += v2;
+                hel += v3;
+            }
+            if (m - k == 3) {
+                const Real v0 = term(), v1 = term(), v2 = term();
+                hel += v0;
+                hel += v1;
+                hel += v2;
+            } else if (m - k == 2) {
+                const Real v0 = term(), v1 = term();
+                hel += v0;
+                hel += v1;
+            } else if (m - k == 1) {
+                hel += term();
+            }
+        } else {
+            const unsigned long long same = beta(src) ? kBetaBits : kAlphaBits;
+            NECI_FOR_WORDS(w, nwords<NW>(s)) {
+                unsigned long long x = d[w];
+                if (((src - 1) >> 6) == w) x &= ~(1ull << ((src - 1) & 63));
+                while (x) {
+                    Real v[4];
+                    bool have[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        have[u] = x != 0ull;
+                        v[u] = 0;
+                        if (have[u]) {
+                            const int b = __ffsll((long long)x) - 1;
+                            x &= x - 1;
+                            v[u] = __ldg((((same >> b) & 1ull) ? jkr : jr) + (w * 32 + (b >> 1)));
+                        }
                     }
-                }
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (have[u]) hel += v[u];
+                    for (int u = 0; u < 4; ++u)
+                        if (have[u]) hel += v[u];
+                }
             }
         }
     }
@@ -106,7 +179,7 @@ __device__ inline void finish_single(const DevSys &s, const unsigned long long *
     const int lo = min(src, tgt), hi = max(src, tgt);
     const bool par = occ_between(d, nwords<NW>(s), lo, hi) & 1;  // make_single tParity
     const Real hel = (s.system == NECI_SYS_HUBBARD_REAL_SPACE) ? tmat_r<Real>(s, src, tgt) : sltcnd_1_r<Real, NW>(s, d, src, tgt);
-    e.hel = par ? -hel : hel;
+    e.hel = par ? negate(hel) : hel;
 }
 
 // gen_excit_rs_hubbard (real_space_hubbard.F90:1938-2030),
@@ -275,7 +348,7 @@ __device__ inline void finish_double(const DevSys &s, const unsigned long long *
     flip_orb(e.child, src1);
     flip_orb(e.child, tb);
     const Real hel = sltcnd_2_r<Real>(s, src0, src1, ta, tb);
-    e.hel = (np & 1) ? -hel : hel;
+    e.hel = (np & 1) ? negate(hel) : hel;
 }
 
 // Position among the electrons of one spin of the pair with triangular
