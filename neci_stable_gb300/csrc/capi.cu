@@ -171,7 +171,7 @@ void insert_pass(Engine &e) {
 // side by side on two streams (in the step graph, two branches), and in
 // either order give the same list and the same counts.  With profiling on
 // they run one after the other on the step's stream.
-void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
+void step_sequence(Engine &e) {
     stage(e, K_SWEEP, [&] { launch_sweep(e, e.stream); });
     // the freed slots' 2-RDM sums: beside the spawn, before the placement
     if (e.sys.rdm) {
@@ -203,7 +203,7 @@ void step_sequence(Engine &e, neci_gpu_iter_stats *out, int advance) {
         cudaStreamWaitEvent(e.stream, e.merge_ev, 0);
     }
     if (e.sys.rdm) stage(e, K_RDM, [&] { launch_rdm(e, e.stream); });
-    stage(e, K_FINAL, [&] { launch_final(e, e.stream, out, e.d_stat_pos, advance, 1); });
+    stage(e, K_FINAL, [&] { launch_final(e, e.stream, 1, 1); });
 }
 
 // Destroys the cached step graphs (after any change the kernels see by value).
@@ -238,7 +238,7 @@ int ensure_graph(Engine &e) {
     if (!e.graphs[k]) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-        step_sequence(e, e.d_stats, 1);  // each replay writes the next record (d_stat_pos)
+        step_sequence(e);  // each replay writes the next record
         CK(cudaStreamEndCapture(e.stream, &g));
         CK(cudaGraphInstantiate(&e.graphs[k], g, 0));
         cudaGraphDestroy(g);
@@ -359,8 +359,6 @@ int32_t neci_gpu_init(neci_gpu_ctx **out, const neci_gpu_system *sys, int32_t de
     A(st.ctl, 1);
     A(e.d_params, 1);
     e.max_stats = 4096;
-    A(e.d_stats, (size_t)e.max_stats + 1);
-    A(e.d_stat_pos, 1);
 #undef A
     if (rc == NECI_GPU_OK) {
         if (cudaMallocHost(&e.h_params, sizeof(IterParams)) != cudaSuccess ||
@@ -895,7 +893,9 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     c.tot_walkers = (unsigned long long)nrows;
     // the tau-search log at the end of the block outlives the walker list
     CK(cudaMemcpyAsync(e.st.ctl, &c, offsetof(Control, tau_gamma), cudaMemcpyHostToDevice, e.stream));
-    // the core space belongs to the previous list
+    // the core space belongs to the previous list (and was part of the step
+    // graphs, which otherwise stay)
+    if (e.st.n_core > 0) drop_graphs(e);
     e.st.n_core = 0;
     if (nrows > 0) launch_upload_fix(e, nrows, compute);
     CK(cudaGetLastError());
@@ -905,7 +905,6 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaMemset(&e.st.ctl->err, 0, sizeof(int)));
     e.compact_due = e.rehash_due = false;  // the list and its hash are new
     if (err) return fail(err, "upload: hash table full");
-    drop_graphs(e);
     return NECI_GPU_OK;
 }
 
@@ -918,31 +917,63 @@ int32_t neci_gpu_download_walkers(neci_gpu_ctx *ctx, int64_t *ilut, double *dh, 
     unsigned long long tw = 0;
     CK(cudaMemcpy(&tw, &e.st.ctl->tot_walkers, sizeof(tw), cudaMemcpyDeviceToHost));
     tw = std::min<unsigned long long>(tw, (unsigned long long)e.st.max_walkers);
-    const int R = e.sys.R, W = e.sys.W, L = e.sys.L;
-    std::vector<long long> rows((size_t)tw * R);
-    std::vector<double> d1(tw), d2(tw);
-    if (tw) {
-        CK(cudaMemcpy(rows.data(), e.st.dets, (size_t)tw * R * 8, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(d1.data(), e.st.diagH, (size_t)tw * 8, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(d2.data(), e.st.offdiagH, (size_t)tw * 8, cudaMemcpyDeviceToHost));
-    }
-    long long n = 0;
-    for (unsigned long long j = 0; j < tw; ++j) {
-        const long long *r = &rows[j * R];
-        bool occ = e.st.n_core > 0 && ((r[W + L] >> NECI_FLAG_DETERMINISTIC_1) & 1);
-        for (int k = 0; k < L; ++k) {
-            double v;
-            std::memcpy(&v, &r[W + k], 8);
-            if (std::fabs(v) >= 1e-12) occ = true;
+    *nrows = 0;
+    if (tw == 0) return NECI_GPU_OK;
+    // The occupied slots are packed on the device, in the spawn buffers (the
+    // records, and their hashes for the diagonal elements), which hold
+    // nothing between two calls; a list longer than they are takes several
+    // rounds of tiles.
+    const int R = e.sys.R;
+    const long long ntiles = ((long long)tw + kCompactTile - 1) / kCompactTile;
+    launch_read_scan(e, (long long)tw);
+    uint32_t total = 0;
+    CK(cudaMemcpyAsync(&total, e.st.tile_off + ntiles, sizeof(total), cudaMemcpyDeviceToHost, e.stream));
+    CK(cudaStreamSynchronize(e.stream));
+    if ((long long)total > max_rows) return fail(NECI_GPU_ERR_INVALID, "download: output too small");
+    std::vector<uint32_t> off;
+    if ((long long)total > e.st.max_spawned) {
+        off.resize((size_t)ntiles + 1);
+        CK(cudaMemcpy(off.data(), e.st.tile_off, off.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+        if (e.st.max_spawned < kCompactTile) {  // not even a tile at a time: a buffer of its own
+            long long *buf = nullptr;
+            CK(cudaMalloc((void **)&buf, (size_t)kCompactTile * (R + 2) * 8));
+            int rc = NECI_GPU_OK;
+            for (long long t = 0; t < ntiles && rc == NECI_GPU_OK; ++t) {
+                double *d = (double *)(buf + (size_t)kCompactTile * R);
+                const size_t m = off[t + 1] - off[t];
+                launch_read_pack(e, (long long)tw, t, t + 1, buf, d, d + kCompactTile);
+                if (cudaMemcpyAsync(ilut + (size_t)off[t] * R, buf, m * R * 8, cudaMemcpyDeviceToHost, e.stream) ||
+                    (dh && cudaMemcpyAsync(dh + off[t], d, m * 8, cudaMemcpyDeviceToHost, e.stream)) ||
+                    (odh && cudaMemcpyAsync(odh + off[t], d + kCompactTile, m * 8, cudaMemcpyDeviceToHost, e.stream)) ||
+                    cudaStreamSynchronize(e.stream))
+                    rc = fail(NECI_GPU_ERR_CUDA, "download: copy failed");
+            }
+            cudaFree(buf);
+            if (rc == NECI_GPU_OK) *nrows = total;
+            return rc;
         }
-        if (!occ) continue;
-        if (n >= max_rows) return fail(NECI_GPU_ERR_INVALID, "download: output too small");
-        std::memcpy(ilut + (size_t)n * R, r, (size_t)R * 8);
-        if (dh) dh[n] = d1[j];
-        if (odh) odh[n] = d2[j];
-        ++n;
     }
-    *nrows = n;
+    double *const d1 = (double *)e.st.cand_h, *const d2 = (double *)e.st.att;
+    for (long long t0 = 0; t0 < ntiles;) {
+        long long t1 = ntiles;
+        size_t first = 0, m = total;
+        if (!off.empty()) {
+            t1 = t0 + 1;
+            while (t1 < ntiles && (long long)(off[t1 + 1] - off[t0]) <= e.st.max_spawned) ++t1;
+            first = off[t0];
+            m = off[t1] - off[t0];
+        }
+        launch_read_pack(e, (long long)tw, t0, t1, e.st.spawn, dh ? d1 : nullptr, odh ? d2 : nullptr);
+        CK(cudaGetLastError());
+        if (m) {
+            CK(cudaMemcpyAsync(ilut + first * R, e.st.spawn, m * R * 8, cudaMemcpyDeviceToHost, e.stream));
+            if (dh) CK(cudaMemcpyAsync(dh + first, d1, m * 8, cudaMemcpyDeviceToHost, e.stream));
+            if (odh) CK(cudaMemcpyAsync(odh + first, d2, m * 8, cudaMemcpyDeviceToHost, e.stream));
+        }
+        CK(cudaStreamSynchronize(e.stream));
+        t0 = t1;
+    }
+    *nrows = total;
     return NECI_GPU_OK;
 }
 
@@ -1031,6 +1062,7 @@ static void take_rehash(Engine &e, neci_gpu_iter_stats *stats, int n) {
 // leaves to a later one of them (a refill of the walker hash, the diagonal of
 // the 2-RDM) is done by the last.
 static void set_span(IterParams &p, int n) {
+    p.iter_begin = p.iter;
     p.iter_end = p.iter + n;
     p.rdm_defer = n > 1;
 }
@@ -1050,15 +1082,13 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         e.h_params->iter = p->iter + done;
         set_span(*e.h_params, batch);
         CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e.stream));
-        CK(cudaMemsetAsync(e.d_stat_pos, 0, sizeof(int), e.stream));
         if (device_ms) CK(cudaEventRecord(e.ev[0], e.stream));
         if (e.profiling) {
-            for (int i = 0; i < batch; ++i) step_sequence(e, e.d_stats, 1);
+            for (int i = 0; i < batch; ++i) step_sequence(e);
         } else {
             for (int i = 0; i < batch; ++i) CK(cudaGraphLaunch(e.graph, e.stream));
         }
         if (device_ms) CK(cudaEventRecord(e.ev[1], e.stream));
-        CK(cudaMemcpyAsync(e.h_stats, e.d_stats, sizeof(neci_gpu_iter_stats) * batch, cudaMemcpyDeviceToHost, e.stream));
         CK(cudaStreamSynchronize(e.stream));
         CK(cudaGetLastError());
         if (device_ms) {
@@ -1143,7 +1173,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         cudaError_t ce = cudaEventRecord(e0.fork_ev, e0.stream);
         for (int c = 1; c < n_ctx && ce == cudaSuccess; ++c) ce = cudaStreamWaitEvent(ctxs[c]->e.stream, e0.fork_ev, 0);
         if (ce == cudaSuccess)
-            for (int c = 0; c < n_ctx; ++c) step_sequence(ctxs[c]->e, ctxs[c]->e.d_stats, 1);
+            for (int c = 0; c < n_ctx; ++c) step_sequence(ctxs[c]->e);
         for (int c = 1; c < n_ctx && ce == cudaSuccess; ++c) {
             Engine &e = ctxs[c]->e;
             ce = cudaEventRecord(e.join_ev, e.stream);
@@ -1166,17 +1196,11 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
     for (int c = 0; c < n_ctx; ++c) {
         Engine &e = ctxs[c]->e;
         CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e0.stream));
-        CK(cudaMemsetAsync(e.d_stat_pos, 0, sizeof(int), e0.stream));
         compact_if_due(e, e0.stream);
     }
     CK(cudaEventRecord(e0.ev[0], e0.stream));
     for (int i = 0; i < n_iter; ++i) CK(cudaGraphLaunch(e0.batch_graph, e0.stream));
     CK(cudaEventRecord(e0.ev[1], e0.stream));
-    for (int c = 0; c < n_ctx; ++c) {
-        Engine &e = ctxs[c]->e;
-        CK(cudaMemcpyAsync(e.h_stats, e.d_stats, sizeof(neci_gpu_iter_stats) * n_iter, cudaMemcpyDeviceToHost,
-                           e0.stream));
-    }
     CK(cudaStreamSynchronize(e0.stream));
     CK(cudaGetLastError());
     if (device_ms) {
@@ -1228,9 +1252,8 @@ int32_t neci_gpu_annihilate(neci_gpu_ctx *ctx, const neci_gpu_iter_params *p, co
     e.fuse_mode = mode;
     launch_ann_insert(e, e.stream, 0);
     launch_merge_stats(e, e.stream, 0, 0);
-    launch_final(e, e.stream, e.d_stats, nullptr, 0, 0);
+    launch_final(e, e.stream, 0, 0);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(e.h_stats, e.d_stats, sizeof(neci_gpu_iter_stats), cudaMemcpyDeviceToHost, e.stream));
     CK(cudaStreamSynchronize(e.stream));
     *stats = e.h_stats[0];
     stats->n_spawned = n;

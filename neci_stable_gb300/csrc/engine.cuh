@@ -318,6 +318,7 @@ struct IterParams {
     float f_tau, f_inv_av, f_cutoff, f_inv_cutoff;
     unsigned long long cutoff_q;  // RealSpawnCutoff in fixed point
     int av_unit;                  // AvMCExcits == 1: the spawn count is split in integers
+    long long iter_begin;         // the first iteration of these steps
     long long iter_end;           // the iteration after the last one of these steps
     int rdm_defer;                // 2-RDM: the diagonal is summed per slot (DevState::rdm_w) and added
                                   // behind the last step

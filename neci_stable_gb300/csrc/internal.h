@@ -69,10 +69,8 @@ struct Engine {
     cudaStream_t stream = nullptr;
     IterParams *d_params = nullptr;
     IterParams *h_params = nullptr;          // pinned
-    neci_gpu_iter_stats *d_stats = nullptr;  // per-step records
-    neci_gpu_iter_stats *h_stats = nullptr;  // pinned
+    neci_gpu_iter_stats *h_stats = nullptr;  // the steps' records (pinned; k_final writes them)
     int max_stats = 0;
-    int *d_stat_pos = nullptr;               // the next record a step writes (k_final)
     // changes with every drop of the step graphs (a batch graph built on them
     // is rebuilt)
     unsigned long long graph_version = 0;
@@ -132,7 +130,10 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split);
 void launch_ann_gather(Engine &e, cudaStream_t s);
 void launch_ann_new(Engine &e, cudaStream_t s, int split);
 void launch_merge_stats(Engine &e, cudaStream_t s, int with_core, int split);
-void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split);
+void launch_final(Engine &e, cudaStream_t s, int advance_iter, int split);
+// packing of the occupied slots for a read of the list
+void launch_read_scan(Engine &e, long long n);
+void launch_read_pack(Engine &e, long long n, long long t0, long long t1, long long *rows, double *dh, double *odh);
 void launch_rdm(Engine &e, cudaStream_t s);
 void launch_rdm_freed(Engine &e, cudaStream_t s);
 

@@ -240,6 +240,63 @@ __global__ void k_compact_done(DevState st) {
 }
 
 // ===========================================================================
+// Reading the list: the occupied (or core) slots packed in slot order on the
+// device, so that the host copies their rows once, straight to its caller.
+// (Copying every slot and packing on the host took 2.2 ms for 2.9e5 of 3.6e5
+// slots.)  Tiles and ranks as in the compaction; `off` gets each tile's first
+// place and, behind the last tile, their number.
+// ===========================================================================
+__global__ void __launch_bounds__(kCompactTile) k_read_count(DevSys s, DevState st, long long n) {
+    const long long ntiles = (n + kCompactTile - 1) / kCompactTile;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const long long j = t * kCompactTile + threadIdx.x;
+        unsigned int count;
+        (void)tile_rank(j < n && slot_kept(s, st, j), count);
+        if (threadIdx.x == 0) st.tile_count[t] = count;
+    }
+}
+__global__ void __launch_bounds__(kCompactTile) k_read_scan(DevState st, long long ntiles) {
+    __shared__ unsigned int warp_n[kCompactTile / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned int carry = 0;  // the same in every thread
+    for (long long base = 0; base < ntiles; base += kCompactTile) {
+        const long long t = base + threadIdx.x;
+        const unsigned int c = t < ntiles ? st.tile_count[t] : 0u;
+        unsigned int incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) warp_n[wid] = incl;
+        __syncthreads();
+        unsigned int before = 0, total = 0;
+        for (int w = 0; w < kCompactTile / 32; ++w) {
+            before += w < wid ? warp_n[w] : 0u;
+            total += warp_n[w];
+        }
+        if (t < ntiles) st.tile_off[t] = carry + before + incl - c;
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) st.tile_off[ntiles] = carry;
+}
+// The slots of tiles t0 .. t1 - 1, the first of them to row 0 of the outputs.
+__global__ void __launch_bounds__(kCompactTile) k_read_pack(DevSys s, DevState st, long long n, long long t0, long long t1,
+                                                            long long *rows, double *dh, double *odh) {
+    const unsigned int first = st.tile_off[t0];
+    for (long long t = t0 + blockIdx.x; t < t1; t += gridDim.x) {
+        const long long j = t * kCompactTile + threadIdx.x;
+        const bool keep = j < n && slot_kept(s, st, j);
+        unsigned int count;
+        const long long pos = (long long)(st.tile_off[t] - first) + tile_rank(keep, count);
+        if (!keep) continue;
+        for (int w = 0; w < s.R; ++w) rows[pos * s.R + w] = st.dets[j * s.R + w];
+        if (dh) dh[pos] = st.diagH[j];
+        if (odh) odh[pos] = st.offdiagH[j];
+    }
+}
+
+// ===========================================================================
 // k_sweep
 // ===========================================================================
 // a / b (IEEE round-to-nearest) as one inline PTX instruction, which the
@@ -1831,22 +1888,23 @@ __global__ void __launch_bounds__(256) k_rdm_freed(DevSys s, DevState st, const 
 // ===========================================================================
 // k_final: write the step's stats record.
 // ===========================================================================
-// The record goes to out[*pos] (and *pos advances, up to max_out - 1) when
-// pos is given: the step graph is the same for every step of a batch, and
-// each step's record lands in its own place.
+// The record goes straight to the host's pinned buffer (no copy behind the
+// step), at the step's place in the call: the step graph is the same for every
+// step.
 // split: the merge sweep counted the slots the step began with less the
 // freed ones; the new determinants are occupied, and the freed slots the
 // placement did not fill are holes.  A walker hash whose live entries and
 // tombstones pass 60% of the buckets is rebuilt between two calls (the host
 // is told in `reserved` of the record); within a call, past 70%, it is
 // cleared here (the return value) and the next step's sweep refills it.
-__device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int *pos, int max_out, IterParams *pp,
+__device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
                             int advance_iter, long long n_core, int split) {
+    const long long next = pp->iter + 1;
     neci_gpu_iter_stats *out = base;
-    if (pos) {
-        const int k = *pos;
+    if (advance_iter) {
+        const long long k = pp->iter - pp->iter_begin;
         out = base + (k < max_out ? k : max_out - 1);
-        *pos = k + 1;
+        pp->iter = next;
     }
     Control *c = st.ctl;
     if (c->halted) {
@@ -1889,8 +1947,6 @@ __device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int *
     r.n_new = (long long)c->n_new;
     r.n_core = n_core;
     r.err = c->err;
-    const long long next = pp->iter + 1;
-    if (advance_iter) pp->iter = next;
     const unsigned long long used = c->n_occupied + c->n_tomb;
     const bool more = advance_iter && next < pp->iter_end && !c->err;  // another step of the call follows
     const bool in_call = more && used * 10ull > st.hash_n * 7ull;
@@ -1907,10 +1963,10 @@ __device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int *
     return in_call ? 1 : 0;
 }
 
-__global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats *base, int *pos, int max_out,
-                                                IterParams *pp, int advance_iter, long long n_core, int split) {
+__global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
+                                                int advance_iter, long long n_core, int split) {
     __shared__ int clear;
-    if (threadIdx.x == 0) clear = final_record(st, base, pos, max_out, pp, advance_iter, n_core, split);
+    if (threadIdx.x == 0) clear = final_record(st, base, max_out, pp, advance_iter, n_core, split);
     __syncthreads();
     if (!clear) return;
     // one block: within a call a rebuild is due about once in hundreds of
@@ -1944,6 +2000,15 @@ void launch_compact(Engine &e, cudaStream_t s) {
     k_compact_holes<<<grid, kCompactTile, 0, s>>>(e.sys, e.st);
     k_compact_move<<<grid_slots(e), 256, 0, s>>>(e.sys, e.st);
     k_compact_done<<<1, 32, 0, s>>>(e.st);
+}
+
+void launch_read_scan(Engine &e, long long n) {
+    const long long ntiles = (n + kCompactTile - 1) / kCompactTile;
+    k_read_count<<<clamp_grid(ntiles, e.num_sms * 2), kCompactTile, 0, e.stream>>>(e.sys, e.st, n);
+    k_read_scan<<<1, kCompactTile, 0, e.stream>>>(e.st, ntiles);
+}
+void launch_read_pack(Engine &e, long long n, long long t0, long long t1, long long *rows, double *dh, double *odh) {
+    k_read_pack<<<clamp_grid(t1 - t0, e.num_sms * 2), kCompactTile, 0, e.stream>>>(e.sys, e.st, n, t0, t1, rows, dh, odh);
 }
 
 void launch_rehash(Engine &e, cudaStream_t s) {
@@ -2093,8 +2158,8 @@ void launch_rdm_freed(Engine &e, cudaStream_t s) {
     k_rdm_freed<<<clamp_grid(e.st.max_walkers / (256 * 64) + 1, 32), 256, shm, s>>>(e.sys, e.st, e.d_params, shm ? 1 : 0);
 }
 
-void launch_final(Engine &e, cudaStream_t s, neci_gpu_iter_stats *out, int *pos, int advance_iter, int split) {
-    k_final<<<1, 1024, 0, s>>>(e.st, out, pos, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
+void launch_final(Engine &e, cudaStream_t s, int advance_iter, int split) {
+    k_final<<<1, 1024, 0, s>>>(e.st, e.h_stats, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
 }
 
 }  // namespace neci

@@ -204,3 +204,35 @@ def test_short_and_long_spawn_lists(name, lenof_sign, walkers):
             for f in ("n_attempts", "n_spawned", "n_unique", "n_new", "n_occupied"):
                 assert getattr(sg, f) == getattr(sc, f), (f, it, scale)
             same_list(spec, eng, orc, (it, scale))
+
+
+@pytest.mark.parametrize("lenof_sign", [1, 2])
+@pytest.mark.parametrize("n,max_spawned", [(1, 4096), (1023, 4096), (1024, 4096), (1025, 700), (5000, 700), (5000, 1500), (5000, 5000)])
+def test_download_packs_the_occupied_slots(lenof_sign, n, max_spawned):
+    # lists of less and more than a tile and than the spawn buffer, every
+    # third slot a hole; slots in order, whatever is asked for beside the rows
+    spec = molecule(24, 10, lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 14, max_spawned)
+    rng = np.random.default_rng(n)
+    rows = random_walkers(spec, 2 * n + 50, rng)[:n]
+    assert rows.shape[0] == n
+    W, L = spec.W, spec.lenof_sign
+    rows[1::3, W:W + L] = 0
+    dh, odh = rng.normal(size=n), rng.normal(size=n)
+    eng.upload(rows, dh, odh)
+    keep = np.ones(n, dtype=bool)
+    keep[1::3] = False
+    got, gd, go = eng.download()
+    assert np.array_equal(got, rows[keep]) and np.array_equal(gd, dh[keep]) and np.array_equal(go, odh[keep])
+    out = np.full((int(keep.sum()), eng.R), -1, dtype=np.int64)
+    import ctypes as C
+    m = C.c_int64()
+    capi.check(eng.lib.neci_gpu_download_walkers(eng.ctx, capi.ptr(out), None, None, out.shape[0], C.byref(m)))
+    assert m.value == out.shape[0] and np.array_equal(out, rows[keep])
+    if out.shape[0] > 1:
+        with pytest.raises(capi.NeciGpuError):
+            eng.download(max_rows=out.shape[0] - 1)
+    eng.start_from_reference(20.0)  # the spawn buffers serve steps as before
+    st = eng.iterate_n(capi.default_params(tau=0.001, seed=1, iter=1), 3)
+    assert all(x.err == 0 and x.n_attempts > 0 for x in st)
+    eng.close()
