@@ -11,60 +11,111 @@ namespace neci {
 // ---------------------------------------------------------------------------
 // Reduction helpers.
 // ---------------------------------------------------------------------------
-__device__ inline double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
+// Modulo 2^64, as a plain sum: three 22-bit parts, whose sums over a warp fit
+// 32 bits, by the warp reduction instruction (three of them instead of ten
+// shuffles and ten additions).
 __device__ inline unsigned long long warp_sum_u(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
+    const unsigned int a = __reduce_add_sync(0xffffffffu, (unsigned int)v & 0x3FFFFFu);
+    const unsigned int b = __reduce_add_sync(0xffffffffu, (unsigned int)(v >> 22) & 0x3FFFFFu);
+    const unsigned int c = __reduce_add_sync(0xffffffffu, (unsigned int)(v >> 44));
+    return a + ((unsigned long long)b << 22) + ((unsigned long long)c << 44);
 }
 
-// Block-wide sum of NV doubles into global atomics (one atomic per value per
-// block).  The values are per run, run-minor (v[2i + run]); with one run the
-// odd entries are skipped.  Every thread's values are staged in shared
-// memory and each warp sums whole values (8 adds per lane, then 5 shuffle
-// levels), so a block issues about a quarter of the FP64 adds of a shuffle
-// tree per warp.  blockDim.x <= 256.
-template <int NV>
-__device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV], int L) {
-    __shared__ double red[NV][256];
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+// Sums of NU counts over the block, one atomic per value.
+template <int NU>
+struct BlockCounts {
+    unsigned long long red[NU][8];
+    __device__ inline void warp_part(const unsigned long long (&u)[NU]) {
 #pragma unroll
-    for (int m = 0; m < NV; ++m)
-        if ((m & 1) < L) red[m][t] = v[m];
-    __syncthreads();
-#pragma unroll
-    for (int m = 0; m < NV; ++m) {  // value m is summed by warp m mod nw
-        if (m % nw != wid || (m & 1) >= L) continue;
-        double s = 0.0;
-        for (int i = lane; i < (int)blockDim.x; i += 32) s += red[m][i];
-        s = warp_sum(s);
-        if (lane == 0 && s != 0.0) atomicAdd(dst[m], s);
+        for (int k = 0; k < NU; ++k) {
+            const unsigned long long s = warp_sum_u(u[k]);
+            if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = s;
+        }
     }
-    __syncthreads();
-}
-
-template <int NV>
-__device__ inline void block_add_u(unsigned long long (&v)[NV], unsigned long long *const (&dst)[NV]) {
-    __shared__ unsigned long long red[NV][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const unsigned long long s = warp_sum_u(v[k]);
-        if (lane == 0) red[k][wid] = s;
-    }
-    __syncthreads();
-    if (wid == 0) {
+    // behind a barrier: one thread per value
+    __device__ inline void add(unsigned long long *const (&dst)[NU]) const {
         const int nw = blockDim.x >> 5;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            unsigned long long s = lane < nw ? red[k][lane] : 0ull;
-            s = warp_sum_u(s);
-            if (lane == 0 && s != 0ull) atomicAdd(dst[k], s);
+        for (int k = 0; k < NU; ++k) {
+            if ((int)threadIdx.x != k) continue;
+            unsigned long long s = 0;
+            for (int w = 0; w < nw; ++w) s += red[k][w];
+            if (s != 0ull) atomicAdd(dst[k], s);
         }
+    }
+};
+template <int NU>
+__device__ inline void block_add_u(const unsigned long long (&u)[NU], unsigned long long *const (&dst)[NU]) {
+    __shared__ BlockCounts<NU> counts;
+    counts.warp_part(u);
+    __syncthreads();
+    counts.add(dst);
+    __syncthreads();
+}
+
+// Block-wide sums of NV doubles and NU counts into global atomics (one atomic
+// per value per block).  The doubles are per run, run-minor (v[2i + run]);
+// with one run the odd entries are skipped.  blockDim.x: a power of two from
+// 8 NV to 256.
+// The FP64 pipe of about one lane per clock per SM is what this costs: it
+// ends every block, and in a short kernel the sums of a whole step end it at
+// once.  So a value that is zero in the whole block (most are: births,
+// aborts, the reference's and its connections' sums in most blocks) takes no
+// addition; one warp per value folds the threads' values to 32 (7 full-width
+// adds of 256 values); and 8 lanes per value, four values a warp, add those
+// (6 adds for four values), instead of 5 shuffle levels each.  12 values of
+// 256 threads: 156 FP64 warp instructions before, at most 102 now, 34 with
+// four of them non-zero.
+template <int NV, int NU>
+__device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV], int L, const unsigned long long (&u)[NU],
+                                 unsigned long long *const (&du)[NU]) {
+    __shared__ double red[NV][256];
+    __shared__ double *to[NV];
+    __shared__ unsigned int row[NV];   // the non-zero values, in order
+    __shared__ unsigned int live[8];   // the warps' masks of non-zero values
+    __shared__ BlockCounts<NU> counts;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+    unsigned int mask = 0;
+#pragma unroll
+    for (int m = 0; m < NV; ++m)
+        if ((m & 1) < L) {
+            red[m][t] = v[m];
+            if ((unsigned long long)__double_as_longlong(v[m]) << 1) mask |= 1u << m;
+        }
+    if (t == 0) {
+#pragma unroll
+        for (int m = 0; m < NV; ++m) to[m] = dst[m];
+    }
+    counts.warp_part(u);
+    mask = __reduce_or_sync(0xffffffffu, mask);
+    if (lane == 0) live[wid] = mask;
+    __syncthreads();
+    counts.add(du);
+    mask = 0;
+    for (int w = 0; w < nw; ++w) mask |= live[w];
+    // the k-th non-zero value: warp k mod nw.  Not unrolled: at a short
+    // kernel's end this code runs once, its instructions fetched for it.
+    unsigned int rest = mask;
+#pragma unroll 1
+    for (int k = 0; rest; ++k, rest &= rest - 1) {
+        if ((k & (nw - 1)) != wid) continue;
+        const unsigned int m = __ffs(rest) - 1;
+        double s = red[m][lane];
+        for (int i = lane + 32; i < (int)blockDim.x; i += 32) s += red[m][i];
+        red[m][lane] = s;
+        if (lane == 0) row[k] = m;
+    }
+    __syncthreads();
+    const int n = __popc(mask);
+    if (wid * 4 < n) {  // four values a warp
+        const int k = min(t >> 3, n - 1);
+        const double *r = red[row[k]];
+        double s = r[t & 7];
+#pragma unroll
+        for (int i = 8; i < 32; i += 8) s += r[(t & 7) + i];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+        if ((t & 7) == 0 && (t >> 3) < n) atomicAdd(to[row[k]], s);
     }
     __syncthreads();
 }

@@ -699,10 +699,9 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     double *const dst[12] = {&c->tot_parts_old[0], &c->tot_parts_old[1], &c->hf_cyc[0], &c->hf_cyc[1],
                              &c->enum_cyc[0], &c->enum_cyc[1], &c->ndied[0], &c->ndied[1],
                              &c->nborn[0], &c->nborn[1], &c->naborted[0], &c->naborted[1]};
-    block_add<12>(v, dst, L);
-    unsigned long long u[2] = {acc_att, acc_tomb};
+    const unsigned long long u[2] = {acc_att, acc_tomb};
     unsigned long long *const du[2] = {&c->n_attempts, &c->n_tomb};
-    block_add_u<2>(u, du);
+    block_add<12, 2>(v, dst, L, u, du);
     if (s.tau_search) {
         // non-negative doubles order like their bit patterns
         unsigned long long b = (unsigned long long)__double_as_longlong(death_max);
@@ -1152,24 +1151,31 @@ __device__ inline void place_one(const DevSys &s, const DevState &st, const Plac
 
 template <int LR>
 __device__ inline void add_decide_sums(Control *c, const DecideSums &a) {
-    double v[6] = {a.ab[0], a.ab[1], a.rm[0], a.rm[1], a.born[0], a.born[1]};
+    const double v[6] = {a.ab[0], a.ab[1], a.rm[0], a.rm[1], a.born[0], a.born[1]};
     double *const dst[6] = {&c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
                             &c->nborn[0], &c->nborn[1]};
-    block_add<6>(v, dst, LR);
-    unsigned long long u[3] = {a.s[0], a.s[1], a.nz};
+    const unsigned long long u[3] = {a.s[0], a.s[1], a.nz};
     unsigned long long *const du[3] = {&c->abs_s[0], &c->abs_s[1], &c->n_reps_nz};
-    block_add_u<3>(u, du);
+    block_add<6, 3>(v, dst, LR, u, du);
 }
+// (the doubles are zero unless the placement accounts for its determinants)
 template <int LR>
-__device__ inline void add_place_sums(Control *c, const PlaceSums &a, int split) {
-    unsigned long long u[2] = {(unsigned long long)a.tomb, a.added};  // two's complement for -count
+__device__ inline void add_place_sums(Control *c, const PlaceSums &a) {
+    const double v[4] = {a.tp[0], a.tp[1], a.norm[0], a.norm[1]};
+    double *const dst[4] = {&c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
+    const unsigned long long u[2] = {(unsigned long long)a.tomb, a.added};  // two's complement for -count
     unsigned long long *const du[2] = {&c->n_tomb, &c->n_new};
-    block_add_u<2>(u, du);
-    if (split) {
-        double v[4] = {a.tp[0], a.tp[1], a.norm[0], a.norm[1]};
-        double *const dst[4] = {&c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
-        block_add<4>(v, dst, LR);
-    }
+    block_add<4, 2>(v, dst, LR, u, du);
+}
+// Both at the end of one kernel.
+template <int LR>
+__device__ inline void add_sums(Control *c, const DecideSums &a, const PlaceSums &b) {
+    const double v[10] = {a.ab[0], a.ab[1], a.rm[0], a.rm[1], a.born[0], a.born[1], b.tp[0], b.tp[1], b.norm[0], b.norm[1]};
+    double *const dst[10] = {&c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1], &c->nborn[0],
+                             &c->nborn[1], &c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
+    const unsigned long long u[5] = {a.s[0], a.s[1], a.nz, (unsigned long long)b.tomb, b.added};
+    unsigned long long *const du[5] = {&c->abs_s[0], &c->abs_s[1], &c->n_reps_nz, &c->n_tomb, &c->n_new};
+    block_add<10, 5>(v, dst, LR, u, du);
 }
 
 // LR: lenof_sign of the instance (1, or 2 for a replica pair).
@@ -1277,7 +1283,7 @@ __global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, const 
         }
         if (want) place_one<LR>(s, st, w, t0, f0, nfree, rank, dh, odh, rdm, split, ps);
     }
-    add_place_sums<LR>(c, ps, split);
+    add_place_sums<LR>(c, ps);
 }
 
 // ===========================================================================
@@ -1468,8 +1474,7 @@ __global__ void __launch_bounds__(kNewThreads) k_ann_new(DevSys s, DevState st, 
             if (lane < mine) place_one<LR>(s, st, v, t0, f0, nfree, (unsigned)lane, dh, odh, rdm, split, ps);
         }
     }
-    add_decide_sums<LR>(c, ds);
-    add_place_sums<LR>(c, ps, split);
+    add_sums<LR>(c, ds, ps);
 }
 
 // ===========================================================================
@@ -1670,11 +1675,10 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     double *const dst[12] = {&c->nborn[0], &c->nborn[1], &c->nannihil[0], &c->nannihil[1],
                              &c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
                              &c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
-    block_add<12>(v, dst, L);
     unsigned long long u[6] = {a_s[0], a_s[1], a_occ, a_holes, a_found, a_tomb};
     unsigned long long *const du[6] = {&c->abs_s[0], &c->abs_s[1], &c->n_occupied, &c->n_holes, &c->n_found,
                                        &c->n_tomb};
-    block_add_u<6>(u, du);
+    block_add<12, 6>(v, dst, L, u, du);
 }
 
 // ===========================================================================
