@@ -1133,6 +1133,16 @@ int32_t neci_gpu_iterate_timed(neci_gpu_ctx *ctx, const neci_gpu_iter_params *p,
     return run_steps(ctx->e, p, n_iter, stats, device_ms);
 }
 
+// How much smaller a context's grids are in a batch of n_ctx.  A block has
+// fixed costs (its tables and counters in, its sums out, at a launch rate the
+// contexts share), which a context on its own pays to fill the GPU and a
+// batch need not.  64 contexts of 5e3 to 6e5 determinants, a step in us with
+// grids 1, 2, 4, 8, 16 and 32 times smaller: 3518, 3365, 3229, 3024, 2900,
+// 3004; the 32 smallest of them 785, 674, 617, 603, 647, 767; the 16
+// smallest 278, 243, 225, 226, 259, 357; the 8 smallest 129, 125, 129, 149;
+// the 8 largest 1218, 1200, 1197, 1165, 1130, 1193; the 4 smallest 89, 84, 96.
+static int batch_share(int n_ctx) { return std::min(std::max(n_ctx / 4, 1), 16); }
+
 int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gpu_iter_params *params, int32_t n_iter,
                                neci_gpu_iter_stats *stats, double *device_ms) {
     if (!ctxs || !params || !stats || n_ctx < 1 || n_iter < 1) return fail(NECI_GPU_ERR_INVALID, "bad argument");
@@ -1173,7 +1183,12 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         cudaError_t ce = cudaEventRecord(e0.fork_ev, e0.stream);
         for (int c = 1; c < n_ctx && ce == cudaSuccess; ++c) ce = cudaStreamWaitEvent(ctxs[c]->e.stream, e0.fork_ev, 0);
         if (ce == cudaSuccess)
-            for (int c = 0; c < n_ctx; ++c) step_sequence(ctxs[c]->e);
+            for (int c = 0; c < n_ctx; ++c) {
+                Engine &e = ctxs[c]->e;
+                e.share = batch_share(n_ctx);
+                step_sequence(e);
+                e.share = 1;
+            }
         for (int c = 1; c < n_ctx && ce == cudaSuccess; ++c) {
             Engine &e = ctxs[c]->e;
             ce = cudaEventRecord(e.join_ev, e.stream);

@@ -62,6 +62,9 @@ struct Engine {
     // the last step's spawn list was short: lookup and compression, decision
     // and placement in one kernel each (update_short_list)
     bool gather = true, short_list = true;
+    // the contexts of a batch share the GPU: each one's grids are this much
+    // smaller (batch_share; 1 outside a batch's capture)
+    int share = 1;
     int merge_bpsm = 2;  // merge sweep blocks per SM beside the placement (update_merge_blocks)
     bool compact_due = false;  // the last step left more holes than occupied slots
     bool rehash_due = false;   // ... or the walker hash over its load

@@ -1984,11 +1984,12 @@ __global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats
 // Host-side launch helpers (declared in internal.h).
 // ===========================================================================
 // Grids are sized to the context's capacity, so that small contexts run
-// side by side (neci_gpu_iterate_batch) instead of each filling the GPU.
+// side by side (neci_gpu_iterate_batch) instead of each filling the GPU, and
+// in a batch are smaller by Engine::share.
 static int clamp_grid(long long want, int hi) { return (int)(want < 8 ? 8 : (want > hi ? hi : want)); }
-static int grid_slots(const Engine &e) { return clamp_grid(e.st.max_walkers / 2048 + 1, e.num_sms * 4); }
+static int grid_slots(const Engine &e) { return clamp_grid(e.st.max_walkers / (2048 * e.share) + 1, e.num_sms * 4); }
 static int grid_spawns(const Engine &e, int threads, int occ = 0) {
-    return clamp_grid(e.st.max_spawned / (threads * 4) + 1, e.num_sms * (occ > 0 ? occ : (threads == 128 ? 8 : 4)));
+    return clamp_grid(e.st.max_spawned / (threads * 4 * e.share) + 1, e.num_sms * (occ > 0 ? occ : (threads == 128 ? 8 : 4)));
 }
 static int grid_for(const Engine &e, int threads) {
     (void)threads;
@@ -2108,7 +2109,7 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split) {
     // new determinants are a small part of the spawns: the placement's grid
     // (one determinant per thread and round) is sized to a fraction of the
     // spawn capacity, so that a small instance of a batch launches few blocks
-    const int gp = clamp_grid(e.st.max_spawned / 1024 + 1, e.num_sms * e.occ_place);
+    const int gp = clamp_grid(e.st.max_spawned / (1024 * e.share) + 1, e.num_sms * e.occ_place);
     if (e.sys.L == 2) {
         k_ann_decide<2><<<grid_spawns(e, 256, e.occ_insert), 256, 0, s>>>(e.sys, e.st, e.d_params);
         k_ann_place<2><<<gp, 128, 0, s>>>(e.sys, e.st, e.d_params, split);
@@ -2120,12 +2121,12 @@ void launch_ann_insert(Engine &e, cudaStream_t s, int split) {
 // The kernels of a short spawn list (Engine::short_list).
 void launch_ann_gather(Engine &e, cudaStream_t s) {
     const size_t shm = (e.sys.nbasis + 1) * sizeof(int32_t);
-    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kGatherSpawns) / 128 + 1, e.num_sms * 8);
+    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kGatherSpawns) / (128 * e.share) + 1, e.num_sms * 8);
     if (e.sys.L == 2) k_ann_gather<2><<<grid, 128, shm, s>>>(e.sys, e.st);
     else k_ann_gather<1><<<grid, 128, shm, s>>>(e.sys, e.st);
 }
 void launch_ann_new(Engine &e, cudaStream_t s, int split) {
-    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kShortSpawns) / kNewThreads + 1, e.num_sms * 4);
+    const int grid = clamp_grid(std::min<long long>(e.st.max_spawned, kShortSpawns) / (kNewThreads * e.share) + 1, e.num_sms * 4);
     const size_t shm = new_shared_bytes(e.sys);
     if (e.sys.L == 2) k_ann_new<2><<<grid, kNewThreads, shm, s>>>(e.sys, e.st, e.d_params, split);
     else k_ann_new<1><<<grid, kNewThreads, shm, s>>>(e.sys, e.st, e.d_params, split);
@@ -2134,7 +2135,7 @@ void launch_ann_new(Engine &e, cudaStream_t s, int split) {
 // (split): e.merge_bpsm, two unless the merge sweep is the longer branch, so
 // that the placement's blocks find registers on every SM.
 void launch_merge_stats(Engine &e, cudaStream_t s, int with_core, int split) {
-    const int grid = split ? clamp_grid(e.st.max_walkers / 2048 + 1, e.num_sms * e.merge_bpsm) : grid_for(e, 256);
+    const int grid = split ? clamp_grid(e.st.max_walkers / (2048 * e.share) + 1, e.num_sms * e.merge_bpsm) : grid_for(e, 256);
     if (e.sys.L == 2)
         k_merge_stats<2><<<grid, kStageTile, merge_smem_bytes(e), s>>>(e.sys, e.st, e.d_params, with_core, split);
     else

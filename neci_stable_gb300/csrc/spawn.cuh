@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
 // Grids are sized to the context's capacity (as in kernels.cu).
 // The grid fills spawn_occ blocks per SM (8, the launch bound, unless tuned).
 inline int spawn_grid(const Engine &e, int threads) {
-    const long long want = e.st.max_spawned / (threads * 4) + 1, hi = (long long)e.num_sms * e.spawn_occ;
+    const long long want = e.st.max_spawned / (threads * 4 * e.share) + 1, hi = (long long)e.num_sms * e.spawn_occ;
     return (int)(want < 8 ? 8 : (want > hi ? hi : want));
 }
 

@@ -236,3 +236,26 @@ def test_download_packs_the_occupied_slots(lenof_sign, n, max_spawned):
     st = eng.iterate_n(capi.default_params(tau=0.001, seed=1, iter=1), 3)
     assert all(x.err == 0 and x.n_attempts > 0 for x in st)
     eng.close()
+
+
+@pytest.mark.parametrize("n_ctx", [7, 8, 33, 68])
+def test_batch_with_smaller_grids(n_ctx):
+    # the grids of a batch's contexts shrink from 8 contexts on, down to the
+    # fewest blocks (a short capacity) and to several rounds a block
+    from neci_stable_gb300.engine import iterate_batch
+    specs = [hubbard10(), molecule(12, 6), hubbard10(lenof_sign=2)]
+    walkers = [random_walkers(sp, 2000, np.random.default_rng(60 + k), scale=4.0) for k, sp in enumerate(specs)]
+    params = [capi.default_params(tau=0.004, seed=70 + i, iter=1) for i in range(n_ctx)]
+
+    def fresh(i):
+        e = Engine(specs[i % 3], 1 << (13 if i % 2 else 17), 1 << (15 if i % 2 else 18))
+        e.upload(walkers[i % 3])
+        return e
+
+    batch = [fresh(i) for i in range(n_ctx)]
+    iterate_batch(batch, params, 6)
+    for i in range(0, n_ctx, 1 if n_ctx < 10 else 5):
+        alone = fresh(i)
+        alone.iterate_n(params[i], 6)
+        W = specs[i % 3].W
+        assert np.array_equal(canonical(batch[i].download()[0], W), canonical(alone.download()[0], W)), i
