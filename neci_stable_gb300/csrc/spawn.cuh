@@ -267,6 +267,84 @@ __device__ inline void create_particle(const DevSys &s, const DevState &st, cons
     par[rwords<RW>(s)] = double_to_word(rdm_parent_weight(p, (double)e.invp, e.aq, P.neg));
 }
 
+// Children of a warp waiting for their record, in shared memory (molecular
+// systems).  The append's counter is an atomic whose result the warp waits
+// for, and the record and with 2-RDM sampling the parent's weight (an FP64
+// division) cost a warp the same for one child as for 32; so the children
+// wait until a warp has 32.  A round adds at most 32 doubles and 32 singles
+// to fewer than 32.  The kernel with records appended round by round, and so
+// (us): n = 64 with 2% of 9.8e7 attempts spawning 4745 and 4242, n = 24 with
+// 14% of 9.7e6 540 and 520 (FP32 amplitudes 509 and 481), a replica pair
+// with 2-RDM sampling at n = 32 and 5.9e5 attempts 53 and 47.
+constexpr int kHeld = 96;
+template <int NW>
+struct Held {
+    unsigned long long d[NW > 0 ? NW : kMaxWords][kHeld];
+    long long q[kHeld];
+    uint32_t mark[kHeld];  // run | initiator parent << 1 | core parent << 2 | negative parent << 3
+};
+// ... and with 2-RDM sampling, in dynamic shared memory
+struct HeldParent {
+    double invp[kHeld];
+    unsigned long long aq[kHeld];
+    uint32_t slot[kHeld];
+};
+template <typename Real, int NW>
+__device__ inline void hold(const DevSys &s, Held<NW> &h, HeldParent *hp, int &n, long long qv, unsigned long long w0,
+                            const Parent &P, const Excit<Real> &e) {
+    const unsigned int m = __ballot_sync(0xffffffffu, qv != 0);
+    if (qv != 0) {
+        const int i = n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+        NECI_FOR_WORDS(w, nwords<NW>(s)) h.d[w][i] = e.child[w];
+        h.q[i] = qv;
+        h.mark[i] = (uint32_t)P.run | (P.pinit ? 2u : 0u) | (P.core ? 4u : 0u) | (P.neg ? 8u : 0u);
+        if (hp) {
+            hp->invp[i] = (double)e.invp;
+            hp->aq[i] = e.aq;
+            hp->slot[i] = (uint32_t)w0;
+        }
+    }
+    n += __popc(m);
+}
+// create_particle for waiting children first .. first + n - 1 (n <= 32).
+template <int NW, int RW>
+__device__ inline void write_held(const DevSys &s, const DevState &st, const IterParams &p, const Held<NW> &h,
+                                  const HeldParent *hp, int first, int n) {
+    const int lane = threadIdx.x & 31, i = first + lane;
+    bool rec = lane < n;
+    unsigned long long c[kMaxWords];
+    NECI_FOR_WORDS(w, nwords<NW>(s)) c[w] = 0ull;
+    long long qv = 0;
+    uint32_t mark = 0;
+    if (rec) {
+        NECI_FOR_WORDS(w, nwords<NW>(s)) c[w] = h.d[w][i];
+        qv = h.q[i];
+        mark = h.mark[i];
+        if ((mark & 4u) && !s.tau_search && core_child<NW, RW>(s, st, c)) rec = false;
+        if (rec && qv == kOverflow) {
+            set_err(st.ctl, NECI_GPU_ERR_OVERFLOW);
+            rec = false;
+        }
+    }
+    const unsigned long long pos = warp_append1(&st.ctl->n_spawned, rec);
+    if (!rec) return;
+    if (pos >= (unsigned long long)st.max_spawned) {
+        set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        return;
+    }
+    const int run = (int)(mark & 1u);
+    long long *o = st.spawn + pos * s.R;
+    NECI_FOR_WORDS(w, rwords<RW>(s)) o[w] = w < nwords<NW>(s) ? (long long)c[w] : 0ll;
+    for (int k2 = 0; k2 < s.L; ++k2) o[rwords<RW>(s) + k2] = (k2 == run) ? qv : 0ll;
+    o[rwords<RW>(s) + s.L] = mark & 2u ? (1ll << init_flag_bit(run)) : 0ll;
+    if (!hp) return;
+    // (as in create_particle)
+    long long *par = st.spawn_par + pos * (rwords<RW>(s) + 1);
+    const long long *r = st.dets + (long long)hp->slot[i] * s.R;
+    NECI_FOR_WORDS(w, rwords<RW>(s)) par[w] = r[w];
+    par[rwords<RW>(s)] = double_to_word(rdm_parent_weight(p, hp->invp[i], hp->aq[i], (mark & 8u) != 0));
+}
+
 // Children of a warp waiting for the fused lookup, in shared memory: their
 // words, amplitude and marks.  A warp holds fewer than 32 between rounds.
 constexpr int kWaiting = 64;
@@ -349,7 +427,8 @@ __device__ inline void look_up(const DevSys &s, const DevState &st, Waiting<NW> 
 // choice), so the draws are those of the attempt processed inline.
 template <typename Real, int GEN, int CLS, int NW, int RW>
 __device__ inline void spawn_class(const DevSys &s, const DevState &st, const IterParams &p, bool valid,
-                                   const Parent &P, Stream &rng, TauAcc *tacc) {
+                                   unsigned long long w0, const Parent &P, Stream &rng, TauAcc *tacc, Held<NW> &held,
+                                   HeldParent *hp, int &n_held) {
     Excit<Real> e;
     e.ok = false;
     long long qv = 0;
@@ -359,7 +438,7 @@ __device__ inline void spawn_class(const DevSys &s, const DevState &st, const It
         else gen_pchb_double<Real, NW>(s, P.d, rng, e);
         qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, tacc);
     }
-    create_particle<Real, NW, RW>(s, st, p, qv, P, e);
+    hold<Real, NW>(s, held, hp, n_held, qv, w0, P, e);
 }
 
 // The parent and stream of a queued attempt: the stream resumes after its
@@ -414,6 +493,8 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // per warp
     __shared__ Waiting<GEN == NECI_EXGEN_RS_HUBBARD ? NW : 1> waiting[GEN == NECI_EXGEN_RS_HUBBARD ? 4 : 1];
     __shared__ unsigned long long sh_sums[GEN == NECI_EXGEN_RS_HUBBARD ? 3 : 1][128];
+    // molecular systems: the warps' children waiting for their records
+    __shared__ Held<GEN == NECI_EXGEN_RS_HUBBARD ? 1 : NW> held_all[GEN == NECI_EXGEN_RS_HUBBARD ? 1 : 4];
     __shared__ long long sh_n[2];
     // the lattice instance for one coupling: the pick's bounds, the step's
     // amplitude magnitudes, the sites' neighbours
@@ -544,12 +625,14 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // less than 512 entries past the head, never on an entry being read.
     if constexpr (GEN != NECI_EXGEN_RS_HUBBARD && !QD) {
         unsigned long long *ring = &sq[0][0], *ring_r1 = &sr1[0][0];  // 512 entries each
+        Held<NW> &held = held_all[wid];
+        HeldParent *hp = s.rdm ? reinterpret_cast<HeldParent *>(sh) + wid : nullptr;
+        int n_held = 0;  // the same in every lane of the warp
         unsigned int head = 0;
         int cnt = 0;
         long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
         for (;; q += stride) {
             const bool more = q - threadIdx.x < nround;  // the same in the whole block
-            if (!more && cnt == 0) break;
             bool single = false;
             unsigned long long w0 = 0, r1 = 0;
             if (more) {
@@ -573,7 +656,7 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                         qv = attempt_create<Real, NW, RW>(s, st, p, P, e, rng, &tacc);
                     }
                 }
-                create_particle<Real, NW, RW>(s, st, p, qv, P, e);
+                hold<Real, NW>(s, held, hp, n_held, qv, w0, P, e);
             }
             if (single) {
                 const unsigned int t = atomicAdd(&ring_tail, 1u) & 511u;
@@ -590,8 +673,17 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                 cnt -= take;
                 Parent P;
                 Stream rng = load_queued<NW, RW>(s, st, p, v, a, b, P);
-                spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v, P, rng, &tacc);
+                spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v, a, P, rng, &tacc, held, hp, n_held);
             }
+            // 32 records at once; after the last attempt what is left
+            __syncwarp();
+            while (n_held >= (more ? 32 : 1)) {
+                const int n = min(n_held, 32);
+                n_held -= n;
+                write_held<NW, RW>(s, st, p, held, hp, n_held, n);
+                __syncwarp();
+            }
+            if (!more && cnt == 0) break;
         }
     }
     // Molecular systems with QD (both classes common): a round classifies
@@ -608,10 +700,12 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // entries at once; the next round writes only after its own first
     // barrier, by which time every thread has read them.
     if constexpr (GEN != NECI_EXGEN_RS_HUBBARD && QD) {
+        Held<NW> &held = held_all[wid];
+        HeldParent *hp = s.rdm ? reinterpret_cast<HeldParent *>(sh) + wid : nullptr;
+        int n_held = 0;  // the same in every lane of the warp
         long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
         for (int round = 0;; ++round, q += stride) {
             const bool more = q - threadIdx.x < nround;  // the same in the whole block
-            if (!more && qn[0] == 0 && qn[1] == 0) break;
             const bool valid = more && q < nat;
             int cls = 0;
             unsigned long long w0 = 0, r1 = 0;
@@ -672,14 +766,23 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
                 if (t0) {
                     Parent P;
                     Stream rng = load_queued<NW, RW>(s, st, p, v0, a0, b0, P);
-                    spawn_class<Real, GEN, 0, NW, RW>(s, st, p, v0, P, rng, &tacc);
+                    spawn_class<Real, GEN, 0, NW, RW>(s, st, p, v0, a0, P, rng, &tacc, held, hp, n_held);
                 }
                 if (t1) {
                     Parent P;
                     Stream rng = load_queued<NW, RW>(s, st, p, v1, a1, b1, P);
-                    spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v1, P, rng, &tacc);
+                    spawn_class<Real, GEN, 1, NW, RW>(s, st, p, v1, a1, P, rng, &tacc, held, hp, n_held);
                 }
             }
+            // 32 records at once; after the last attempt what is left
+            __syncwarp();
+            while (n_held >= (more ? 32 : 1)) {
+                const int n = min(n_held, 32);
+                n_held -= n;
+                write_held<NW, RW>(s, st, p, held, hp, n_held, n);
+                __syncwarp();
+            }
+            if (!more && qn[0] == 0 && qn[1] == 0) break;
         }
     }
     // n_spawned and abs_q of the spawns created here (otherwise pass 1 counts
@@ -741,7 +844,7 @@ void launch_spawn_real(Engine &e, cudaStream_t s) {
     const size_t shm = e.sys.excitgen == NECI_EXGEN_RS_HUBBARD
                            ? (size_t)hash_tab_len(e.sys.nbasis) * sizeof(ulonglong2) +
                                  (size_t)(e.sys.nsites * e.sys.max_neigh) * sizeof(int32_t)
-                           : 0;
+                           : (e.sys.rdm ? 4 * sizeof(HeldParent) : 0);
     const int grid = spawn_grid(e, 128);
     if (e.sys.excitgen == NECI_EXGEN_RS_HUBBARD) launch_spawn_gen<Real, NECI_EXGEN_RS_HUBBARD>(e, s, grid, shm);
     else if (e.sys.excitgen == NECI_EXGEN_UNIFORM) launch_spawn_gen<Real, NECI_EXGEN_UNIFORM>(e, s, grid, shm);
