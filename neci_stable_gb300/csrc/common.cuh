@@ -53,6 +53,76 @@ __device__ inline void block_add_u(const unsigned long long (&u)[NU], unsigned l
     __syncthreads();
 }
 
+// A sum of doubles in fixed point, 96 bits in units of 2^-Q: an FP64 addition
+// holds its pipe (about one lane per clock per SM) for as long as the SM's
+// schedulers issue a hundred integer instructions, and this takes a dozen.  A
+// term is rounded to the nearest unit, so the sum is off by at most a half
+// unit per term, less than an FP64 running sum of such terms; the terms the
+// units are too fine for, 2^(63 - Q) and more (and infinities and NaN), go to
+// the target by themselves.
+template <int Q>
+struct FixedSum {
+    unsigned long long lo = 0;
+    int hi = 0;
+    __device__ inline void add(double a, double *target) {
+        const long long b = __double_as_longlong(a);
+        const int e = (int)(b >> 52) & 0x7FF;
+        if (e >= 1086 - Q) {
+            atomicAdd(target, a);
+            return;
+        }
+        // the significand's 64 bits (its leading one at bit 63), shifted to units
+        const int sh = 1085 - Q - e;
+        const unsigned long long m = ((unsigned long long)b << 11) | 0x8000000000000000ull;
+        unsigned long long x = sh > 63 ? 0ull : ((m >> sh) + 1) >> 1;
+        if (b < 0) x = 0ull - x;
+        lo += x;
+        hi += (lo < x ? 1 : 0) + (int)((long long)x >> 63);
+    }
+};
+struct PlainSum {
+    double v = 0.0;
+    __device__ inline void add(double a, double *) { v += a; }
+};
+// The sums every slot adds to, by instance: with one run in fixed point (the
+// sweeps held the FP64 pipe for 65% of their cycles: sweep 1902 to 1825 us and
+// step 8238 to 8076 us at n = 64, step 404 to 394 us at n = 39, 6945 to 6880
+// us on the 6x6 lattice), with a replica pair as they were (twice the
+// accumulators do not fit the registers: merge sweep 37 to 43 us at n = 32).
+template <int LR, int Q>
+using SlotSum = typename std::conditional<LR == 1, FixedSum<Q>, PlainSum>::type;
+
+// NF of them over the block, one FP64 atomic per sum (k: its place among the
+// block's; unit: 2^-Q).
+template <int NF>
+struct BlockFixed {
+    unsigned long long lo[NF][8];
+    long long hi[NF][8];
+    template <int Q>
+    __device__ inline void warp_part(int k, const FixedSum<Q> &f) {
+        const unsigned int a = __reduce_add_sync(0xffffffffu, (unsigned int)f.lo & 0x3FFFFFu);
+        const unsigned int b = __reduce_add_sync(0xffffffffu, (unsigned int)(f.lo >> 22) & 0x3FFFFFu);
+        const unsigned int c = __reduce_add_sync(0xffffffffu, (unsigned int)(f.lo >> 44));
+        const int h = (int)__reduce_add_sync(0xffffffffu, (unsigned int)f.hi);
+        if ((threadIdx.x & 31) == 0) {
+            const __int128 t = (__int128)(a + ((unsigned long long)b << 22)) + ((__int128)c << 44) + ((__int128)h << 64);
+            lo[k][threadIdx.x >> 5] = (unsigned long long)t;
+            hi[k][threadIdx.x >> 5] = (long long)(t >> 64);
+        }
+    }
+    // behind a barrier: thread `by` adds sum k
+    __device__ inline void add(int k, unsigned int by, double unit, double *target) const {
+        if (threadIdx.x != by) return;
+        __int128 t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ((__int128)hi[k][w] << 64) + (__int128)lo[k][w];
+        if (t == 0) return;
+        const bool neg = t < 0;
+        const unsigned __int128 u = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
+        const double v = ((double)(unsigned long long)(u >> 64) * 18446744073709551616.0 + (double)(unsigned long long)u) * unit;
+        atomicAdd(target, neg ? -v : v);
+    }
+};
+
 // Block-wide sums of NV doubles and NU counts into global atomics (one atomic
 // per value per block).  The doubles are per run, run-minor (v[2i + run]);
 // with one run the odd entries are skipped.  blockDim.x: a power of two from

@@ -387,8 +387,9 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     if (c->rehash_fill) sweep_refill(s, st, n);  // the walker hash is empty
     const int W = s.W, R = s.R;
     constexpr int L = LR;
-    double acc_old[2] = {0.0, 0.0}, acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0};
-    double acc_died[2] = {0.0, 0.0}, acc_born[2] = {0.0, 0.0}, acc_ab[2] = {0.0, 0.0};
+    SlotSum<LR, 52> acc_old[L];
+    SlotSum<LR, 56> acc_died[L];
+    double acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0}, acc_born[2] = {0.0, 0.0}, acc_ab[2] = {0.0, 0.0};
     double death_max = 0.0;  // max_death_cpt of this thread's determinants (tau search)
     unsigned long long acc_att = 0, acc_tomb = 0;
     // Tiles of kStageTile slots (one per block and round) are staged into
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             flags = sr[W + L];
             core = st.n_core > 0 && is_core_flags(flags);
             NECI_FOR_RUNS(k, L) {
-                acc_old[k] += abs_dbl(C[k]);
+                acc_old[L == 1 ? 0 : k].add(abs_dbl(C[k]), &c->tot_parts_old[k]);
                 if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
             }
             if (core) {
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                 // there were) is handled below
                 const double aC = abs_dbl(C[k]);
                 const bool le = le_nonneg(idie, aC);
-                acc_died[k] += le ? idie : aC;
+                acc_died[L == 1 ? 0 : k].add(le ? idie : aC, &c->ndied[k]);
                 if (!le) over = true;
                 // C - idie * sign(1, C) with Fortran's sign (+1 for C = -0.0); both products are exact
                 const bool nonneg = !(dbl_bits(C[k]) >> 63) || abs_bits(C[k]) == 0;
@@ -694,14 +695,25 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             }
         }
     }
-    const double v[12] = {acc_old[0], acc_old[1], acc_hf[0], acc_hf[1], acc_en[0], acc_en[1], acc_died[0],
-                          acc_died[1], acc_born[0], acc_born[1], acc_ab[0], acc_ab[1]};
-    double *const dst[12] = {&c->tot_parts_old[0], &c->tot_parts_old[1], &c->hf_cyc[0], &c->hf_cyc[1],
-                             &c->enum_cyc[0], &c->enum_cyc[1], &c->ndied[0], &c->ndied[1],
-                             &c->nborn[0], &c->nborn[1], &c->naborted[0], &c->naborted[1]};
     const unsigned long long u[2] = {acc_att, acc_tomb};
     unsigned long long *const du[2] = {&c->n_attempts, &c->n_tomb};
-    block_add<12, 2>(v, dst, L, u, du);
+    if constexpr (LR == 1) {
+        __shared__ BlockFixed<2> fixed;
+        fixed.warp_part(0, acc_old[0]);
+        fixed.warp_part(1, acc_died[0]);
+        const double v[8] = {acc_hf[0], 0.0, acc_en[0], 0.0, acc_born[0], 0.0, acc_ab[0], 0.0};
+        double *const dst[8] = {&c->hf_cyc[0], nullptr, &c->enum_cyc[0], nullptr, &c->nborn[0], nullptr, &c->naborted[0], nullptr};
+        block_add<8, 2>(v, dst, L, u, du);  // (its barriers are between the parts and the sums)
+        fixed.add(0, 32, 0x1.0p-52, &c->tot_parts_old[0]);
+        fixed.add(1, 64, 0x1.0p-56, &c->ndied[0]);
+    } else {
+        const double v[12] = {acc_old[0].v, acc_old[L - 1].v, acc_hf[0], acc_hf[1], acc_en[0], acc_en[1], acc_died[0].v,
+                              acc_died[L - 1].v, acc_born[0], acc_born[1], acc_ab[0], acc_ab[1]};
+        double *const dst[12] = {&c->tot_parts_old[0], &c->tot_parts_old[1], &c->hf_cyc[0], &c->hf_cyc[1],
+                                 &c->enum_cyc[0], &c->enum_cyc[1], &c->ndied[0], &c->ndied[1],
+                                 &c->nborn[0], &c->nborn[1], &c->naborted[0], &c->naborted[1]};
+        block_add<12, 2>(v, dst, L, u, du);
+    }
     if (s.tau_search) {
         // non-negative doubles order like their bit patterns
         unsigned long long b = (unsigned long long)__double_as_longlong(death_max);
@@ -1495,8 +1507,9 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     const int W = s.W, R = s.R;
     constexpr int L = LR;
     const bool rdm = LR == 2 && split && s.rdm && p.rdm_defer;
-    double a_born[2] = {0, 0}, a_ann[2] = {0, 0}, a_ab[2] = {0, 0}, a_rm[2] = {0, 0};
-    double a_tp[2] = {0, 0}, a_norm[2] = {0, 0};
+    SlotSum<LR, 56> a_born[L], a_rm[L];
+    SlotSum<LR, 52> a_tp[L];
+    double a_norm[2] = {0, 0}, a_ann[2] = {0, 0}, a_ab[2] = {0, 0};
     unsigned long long a_s[2] = {0, 0}, a_occ = 0, a_holes = 0, a_found = 0, a_tomb = 0;
     // Tiles staged into shared memory by TMA bulk copies as in k_sweep: the
     // rows, the per-slot spawn counts (meta) and the per-slot spawn sums
@@ -1543,7 +1556,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
             const int ci = st.core_of_slot[j];
             NECI_FOR_RUNS(k, L) {
                 const double y = st.core_y[(long long)ci * L + k];
-                a_born[k] += fabs(y);
+                a_born[L == 1 ? 0 : k].add(abs_dbl(y), &c->nborn[k]);
                 if (prod_negative(C[k], y)) a_ann[k] += 2.0 * min_abs(C[k], y);
                 C[k] = y + C[k];
             }
@@ -1572,7 +1585,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                 if (abs_bits(C[k]) < dbl_bits(kEps12) && p.t_trunc_initiator) {
                     const bool sp_init = (m[k] & 0x80000000u) ||
                                          (p.t_init_coherent_rule && (m[k] & 0x7FFFFFFFu) >= 2u);
-                    if (!sp_init && !core) { a_ab[k] += fabs(S[k]); S[k] = 0.0; }
+                    if (!sp_init && !core) { a_ab[k] += abs_dbl(S[k]); S[k] = 0.0; }
                 }
                 if (prod_negative(C[k], S[k])) a_ann[k] += 2.0 * min_abs(C[k], S[k]);
             }
@@ -1608,7 +1621,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                     const double pRemove =
                         dbl_bits(p.occupied_thresh) == dbl_bits(1.0) ? tma : div_dbl(tma, p.occupied_thresh);
                     if (bern(rng, pRemove)) {
-                        a_rm[k] += a;
+                        a_rm[L == 1 ? 0 : k].add(a, &c->nremoved[k]);
                         C[k] = 0.0;
                         bool unocc = true;
                         NECI_FOR_RUNS(k2, L) if (abs_bits(C[k2]) >= dbl_bits(kEps12)) unocc = false;
@@ -1618,7 +1631,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                             r[W + L] = flags | 1ll;
                         }
                     } else {
-                        a_born[k] += tma;
+                        a_born[L == 1 ? 0 : k].add(tma, &c->nborn[k]);
                         C[k] = fsign(p.occupied_thresh, C[k]);
                     }
                     changed = true;
@@ -1628,7 +1641,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
         if (changed) NECI_FOR_RUNS(k, L) r[W + k] = double_to_word(C[k]);
         occ = false;
         NECI_FOR_RUNS(k, L) {
-            a_tp[k] += abs_dbl(C[k]);
+            a_tp[L == 1 ? 0 : k].add(abs_dbl(C[k]), &c->tot_parts[k]);
             a_norm[k] = fma(C[k], C[k], a_norm[k]);  // a statistic: one rounding, one FP64 instruction
             if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
         }
@@ -1670,15 +1683,28 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                  (const uint32_t *)(sbase + (size_t)kStageTile * R * 8) + (size_t)threadIdx.x * L,
                  (const long long *)(sbase + (size_t)kStageTile * (R * 8 + L * 4)) + (size_t)threadIdx.x * L);
     }
-    double v[12] = {a_born[0], a_born[1], a_ann[0], a_ann[1], a_ab[0], a_ab[1], a_rm[0], a_rm[1],
-                    a_tp[0], a_tp[1], a_norm[0], a_norm[1]};
-    double *const dst[12] = {&c->nborn[0], &c->nborn[1], &c->nannihil[0], &c->nannihil[1],
-                             &c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
-                             &c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
-    unsigned long long u[6] = {a_s[0], a_s[1], a_occ, a_holes, a_found, a_tomb};
+    const unsigned long long u[6] = {a_s[0], a_s[1], a_occ, a_holes, a_found, a_tomb};
     unsigned long long *const du[6] = {&c->abs_s[0], &c->abs_s[1], &c->n_occupied, &c->n_holes, &c->n_found,
                                        &c->n_tomb};
-    block_add<12, 6>(v, dst, L, u, du);
+    if constexpr (LR == 1) {
+        __shared__ BlockFixed<3> fixed;
+        fixed.warp_part(0, a_born[0]);
+        fixed.warp_part(1, a_rm[0]);
+        fixed.warp_part(2, a_tp[0]);
+        const double v[6] = {a_norm[0], 0.0, a_ann[0], 0.0, a_ab[0], 0.0};
+        double *const dst[6] = {&c->norm[0], nullptr, &c->nannihil[0], nullptr, &c->naborted[0], nullptr};
+        block_add<6, 6>(v, dst, L, u, du);  // (its barriers are between the parts and the sums)
+        fixed.add(0, 32, 0x1.0p-56, &c->nborn[0]);
+        fixed.add(1, 64, 0x1.0p-56, &c->nremoved[0]);
+        fixed.add(2, 96, 0x1.0p-52, &c->tot_parts[0]);
+    } else {
+        const double v[12] = {a_born[0].v, a_born[L - 1].v, a_ann[0], a_ann[1], a_ab[0], a_ab[1], a_rm[0].v, a_rm[L - 1].v,
+                              a_tp[0].v, a_tp[L - 1].v, a_norm[0], a_norm[1]};
+        double *const dst[12] = {&c->nborn[0], &c->nborn[1], &c->nannihil[0], &c->nannihil[1],
+                                 &c->naborted[0], &c->naborted[1], &c->nremoved[0], &c->nremoved[1],
+                                 &c->tot_parts[0], &c->tot_parts[1], &c->norm[0], &c->norm[1]};
+        block_add<12, 6>(v, dst, L, u, du);
+    }
 }
 
 // ===========================================================================

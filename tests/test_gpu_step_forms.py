@@ -259,3 +259,37 @@ def test_batch_with_smaller_grids(n_ctx):
         alone.iterate_n(params[i], 6)
         W = specs[i % 3].W
         assert np.array_equal(canonical(batch[i].download()[0], W), canonical(alone.download()[0], W)), i
+
+
+@pytest.mark.parametrize("n", [1, 31, 257, 1500])
+def test_sums_of_the_sweeps(n):
+    # the sweeps' sums in fixed point: amplitudes around its limits (2048 for
+    # the population, 128 for the deaths, which the shift makes large, small
+    # and negative), against sums without rounding.  A term is off by at most
+    # 2^-53 (population) or 2^-57 (deaths), the FP64 sum of the blocks' sums
+    # by a few units in its last place.
+    import math
+    spec = hubbard10()
+    rng = np.random.default_rng(90 + n)
+    rows = random_walkers(spec, n, rng)
+    W = spec.W
+    edge = np.array([2047.9999999999998, 2048.0, 2048.0000000000005, 1.0, 1.0000000000000002, 0.7, 3.3e5, 1e-3, 2.0 ** -40])
+    amp = np.where(np.arange(len(rows)) % 3 == 0, rng.choice(edge, len(rows)), rng.lognormal(0.0, 2.0, len(rows)))
+    amp *= rng.choice([-1.0, 1.0], len(rows))
+    rows[:, W] = amp.view(np.int64)
+    eng = Engine(spec, 1 << 17, 1 << 25)  # up to 2e7 attempts
+    for shift in (-2.0, 0.0, 9.0):
+        eng.upload(rows)
+        held, dh, _ = eng.download()
+        c = np.ascontiguousarray(held[:, W]).view(np.float64)
+        fac = 0.01 * (dh - shift)
+        died = [min(f * abs(x), abs(x)) for f, x in zip(fac, c)]
+        p = capi.default_params(tau=0.01, diag_sft=[shift, shift], seed=4, iter=1)
+        st = eng.perform_fcimc_cyc_par(p)
+        assert st.err == 0
+        for got, terms, unit in ((st.tot_parts_old[0], np.abs(c).tolist(), 2.0 ** -53), (st.ndied[0], died, 2.0 ** -57)):
+            size = math.fsum(abs(t) for t in terms)
+            assert abs(got - math.fsum(terms)) <= len(terms) * unit + 16 * 2.0 ** -53 * size, (shift, got)
+        after = np.ascontiguousarray(eng.download()[0][:, W]).view(np.float64)
+        total = math.fsum(np.abs(after))
+        assert abs(st.tot_parts[0] - total) <= len(after) * 2.0 ** -53 + 16 * 2.0 ** -53 * total
