@@ -1,5 +1,5 @@
 // common.cuh -- device helpers shared by the step kernels (kernels.cu) and
-// the spawn kernel (spawn.cu): block reductions into the step's counters,
+// the spawn kernel (spawn.cuh): block reductions into the step's counters,
 // warp-aggregated appends, and the walker hash (hash_table_lookup,
 // AddNewHashDet, RemoveHashDet).
 #pragma once

@@ -10,7 +10,7 @@
 //                  core vector gather, and the death step
 //                  (perform_death_all_walkers / walker_death)
 //   k_spawn        the spawn attempts (generate_excitation, attempt_create,
-//                  create_particle): in spawn.cu
+//                  create_particle): in spawn.cuh
 //   k_core         determ_projection_no_death (semi_stoch_procs.F90:290)
 //   k_ann_probe    annihilation pass 1: look every spawn up in the walker
 //                  hash (hash_table_lookup, hash.F90:294); spawns onto
@@ -24,6 +24,8 @@
 //                  survivors are listed for
 //   k_ann_place    AddNewHashDet: slots, rows, hash buckets, diagonal
 //                  elements, one new determinant per thread
+//   k_ann_gather, k_ann_new  the same for a short spawn list: lookup and
+//                  compression in one kernel, decision and placement in one
 //   k_merge_stats  deterministic_annihilation + AnnihilateSpawnedParts
 //                  found branch + CalcHashTableStats (load_balancer.fpp:646)
 //                  in one sweep over the slots
