@@ -48,11 +48,11 @@ BLOOM = 3.0
 # kernel -> (bytes per unit, step count that is the unit).
 # The spawn kernel is bound by instruction issue, not by HBM: its issue
 # figures from the same capture are reported beside its HBM roofline.
-NCU_SPAWN_ISSUE = {"issue_active": 0.586, "alu_pipe": 0.541, "fp64_pipe": 0.372, "warps_active": 0.451,
-                   "lanes_per_instruction": 25.2, "dram_bytes_per_attempt": 15.8}
+NCU_SPAWN_ISSUE = {"issue_active": 0.586, "alu_pipe": 0.566, "fp64_pipe": 0.327, "warps_active": 0.442,
+                   "lanes_per_instruction": 27.3, "dram_bytes_per_attempt": 9.5}
 
 NCU_DRAM_BYTES_PER_UNIT = {
-    "spawn": (15.8, "n_attempts"),
+    "spawn": (9.5, "n_attempts"),
 }
 
 
@@ -782,8 +782,9 @@ def main():
     sort_ms = sum(v["ms"] for v in sort_stages.values())
     sort_bytes = sum(v["algorithmic_bytes"] for v in sort_stages.values())
     ktm = {k: v for k, v in r["ktimes_mixed"].items() if v[1] > 0}
-    # sweep, spawn, compress, decide, place, merge, final; the probe
-    # unless the spawn kernel does it; the core projection and the sum of its
+    # sweep, spawn, compress, decide, place, merge, final (a short spawn list,
+    # not this workload's, takes two fewer); the probe unless the spawn kernel
+    # does it; the core projection and the sum of its
     # long rows (a compaction, when a step leaves more holes than walkers, and
     # a rebuild of the walker hash run between calls)
     launches_per_step = 7 + (2 if r["last"]["n_core"] > 0 else 0) + (0 if fused else 1)
