@@ -1240,8 +1240,12 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
     return NECI_GPU_OK;
 }
 
+// A caller's spawn list.  Its length is checked, and what the call allocates
+// is allocated, before the first kernel that counts: a step finds the
+// counters as the call before it left them (reset_counters).
+static bool spawns_fit(const Engine &e, int64_t n) { return n >= 0 && n <= e.st.max_spawned; }
+static const char *const kSpawnsTooLong = "spawn list longer than MaxSpawned";
 static int upload_spawns(Engine &e, const int64_t *sp, int64_t n) {
-    if (n < 0 || n > e.st.max_spawned) return fail(NECI_GPU_ERR_SPAWN_FULL, "spawn list longer than MaxSpawned");
     if (n > 0) CK(cudaMemcpyAsync(e.st.spawn, sp, (size_t)n * e.sys.R * 8, cudaMemcpyHostToDevice, e.stream));
     launch_convert_spawns(e, n);
     return NECI_GPU_OK;
@@ -1252,6 +1256,7 @@ int32_t neci_gpu_annihilate(neci_gpu_ctx *ctx, const neci_gpu_iter_params *p, co
     if (int r = check_ctx(ctx)) return r;
     Engine &e = ctx->e;
     if (!p || !stats || (!spawned && n > 0)) return fail(NECI_GPU_ERR_INVALID, "null argument");
+    if (!spawns_fit(e, n)) return fail(NECI_GPU_ERR_SPAWN_FULL, kSpawnsTooLong);
     copy_params(*e.h_params, *p);
     CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e.stream));
     launch_rehash(e, e.stream);
@@ -1282,10 +1287,8 @@ int32_t neci_gpu_compress_spawns(neci_gpu_ctx *ctx, const int64_t *spawned, int6
     if (int r = check_ctx(ctx)) return r;
     Engine &e = ctx->e;
     if ((!spawned && n > 0) || !out || !n_out) return fail(NECI_GPU_ERR_INVALID, "null argument");
+    if (!spawns_fit(e, n)) return fail(NECI_GPU_ERR_SPAWN_FULL, kSpawnsTooLong);
     const int R = e.sys.R, W = e.sys.W, L = e.sys.L;
-    launch_begin(e, e.stream);
-    if (int r = upload_spawns(e, spawned, n)) return r;
-    annihilation_passes(e, 0);
     // the output buffers come from the stream's pool and go back to it on
     // every exit, the early returns of a failed call included
     struct StreamBuffers {
@@ -1302,6 +1305,9 @@ int32_t neci_gpu_compress_spawns(neci_gpu_ctx *ctx, const int64_t *spawned, int6
     long long *const d_out = buf.out;
     unsigned long long *const d_n = buf.n;
     CK(cudaMemsetAsync(d_n, 0, sizeof(unsigned long long), e.stream));
+    launch_begin(e, e.stream);
+    if (int r = upload_spawns(e, spawned, n)) return r;
+    annihilation_passes(e, 0);
     launch_compress_out(e, d_out, d_n);
     CK(cudaGetLastError());
     unsigned long long hn = 0;

@@ -3,6 +3,7 @@ the CPU oracle, bit for bit:
 * the walker hash kept at a high load, where its tombstones pile up and it is
   rebuilt inside a call (cleared behind one step, refilled by the next sweep)
   and between calls;
+* a spawn list refused for its length between two steps;
 * heavy parents, whose spawn attempts are numbered by the spawn kernel instead
   of written as entries: around the limit, around the granules, alone and
   many side by side;
@@ -87,6 +88,34 @@ def test_hash_after_entry_points_between_steps():
     if gone.size:
         with pytest.raises(capi.NeciGpuError):
             eng.set_core_space(gone[:1, None])
+
+
+@pytest.mark.parametrize("ann", [capi.ANN_HASH, capi.ANN_SORT])
+def test_steps_after_a_refused_spawn_list(ann):
+    # a spawn list longer than the capacity is refused before anything is
+    # counted: the next steps' free list holds every hole once
+    spec = molecule(12, 6)
+    eng = Engine(spec, 1 << 13, 1 << 13)
+    orc = Oracle(spec, 1 << 13, 1 << 13, hii=eng.hii)
+    eng.set_option(capi.OPT_ANNIHILATION, ann)
+    eng.start_from_reference(initial_part=600.0)
+    orc.upload(eng.download()[0])
+    run_both(spec, eng, orc, (40,), tau=0.01, seed=13)
+    long_list = np.repeat(eng.download()[0][:1], (1 << 13) + 1, axis=0)
+    it = 41
+    for _ in range(3):
+        with pytest.raises(capi.NeciGpuError) as ei:
+            eng.annihilate(capi.default_params(tau=0.01, seed=13, iter=it), long_list)
+        assert ei.value.code == capi.ERR_SPAWN_FULL
+        with pytest.raises(capi.NeciGpuError) as ei:
+            eng.compress_spawns(long_list)
+        assert ei.value.code == capi.ERR_SPAWN_FULL
+        p = capi.default_params(tau=0.01, seed=13, iter=it)
+        sg, (sc, rc) = eng.perform_fcimc_cyc_par(p), orc.iterate(p)
+        assert rc == 0 and sg.err == 0 and sg.holes_in_list > 0
+        assert abs(sg.tot_parts_old[0] - sc.tot_parts_old[0]) <= 1e-12 * sc.tot_parts_old[0]
+        same_list(spec, eng, orc, it)
+        it += 1
 
 
 @pytest.mark.parametrize("name,lenof_sign", [("hub", 1), ("hub", 2), ("mol", 1), ("mol", 2)])
