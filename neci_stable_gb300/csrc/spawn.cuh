@@ -507,10 +507,14 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     if (threadIdx.x == 0) {
         const unsigned long long na = st.ctl->n_att, cap = (unsigned long long)st.max_att;
         const unsigned long long nh = st.ctl->n_big & ((1ull << kBigShift) - 1);
-        const bool stop = halted(st);
-        if (!stop && na + nh > cap) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
-        sh_n[0] = (long long)min(na, cap);
-        sh_n[1] = stop ? 0 : sh_n[0] + (long long)min(nh, cap);
+        const bool over = na + nh > cap;
+        if (over && !halted(st)) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        // a step with more attempts than the list holds fails and makes none:
+        // the sweep leaves out entries that do not fit, and what lies in
+        // their places need not be an entry (a list read packs diagonal
+        // elements there)
+        sh_n[0] = (long long)na;
+        sh_n[1] = over || halted(st) ? 0 : (long long)(na + nh);
     }
     __syncthreads();
     // a block with no attempts leaves (the grid is sized to the capacity)

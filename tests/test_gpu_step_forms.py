@@ -3,7 +3,8 @@ the CPU oracle, bit for bit:
 * the walker hash kept at a high load, where its tombstones pile up and it is
   rebuilt inside a call (cleared behind one step, refilled by the next sweep)
   and between calls;
-* a spawn list refused for its length between two steps;
+* a spawn list refused for its length between two steps, and a step with more
+  attempts than its list holds;
 * heavy parents, whose spawn attempts are numbered by the spawn kernel instead
   of written as entries: around the limit, around the granules, alone and
   many side by side;
@@ -11,6 +12,8 @@ the CPU oracle, bit for bit:
   in the spawn kernel or behind it, core parents, and walker hashes the
   spawn kernel's table cannot hold."""
 from __future__ import annotations
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -116,6 +119,37 @@ def test_steps_after_a_refused_spawn_list(ann):
         assert abs(sg.tot_parts_old[0] - sc.tot_parts_old[0]) <= 1e-12 * sc.tot_parts_old[0]
         same_list(spec, eng, orc, it)
         it += 1
+
+
+@pytest.mark.parametrize("name,lenof_sign", [("hub", 1), ("mol", 1), ("mol", 2)])
+@pytest.mark.parametrize("big", [0.0, 30.0, 2500.0])
+def test_more_attempts_than_the_list_holds(name, lenof_sign, big):
+    # entries, heavy parents or both pass the 3072 attempts of the list, in a
+    # step behind a list read: the step fails without an attempt, and a list
+    # that fits runs again
+    spec = hubbard10(lenof_sign=lenof_sign) if name == "hub" else molecule(12, 6, lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 12, 1 << 10)
+    orc = Oracle(spec, 1 << 12, 1 << 12, hii=eng.hii)
+    rows = random_walkers(spec, 700, np.random.default_rng(41))
+    W, L = spec.W, spec.lenof_sign
+    v = rows[:, W:W + L].view(np.float64).copy()
+    v[:, :] = 6.0 if big == 0.0 else 1.0
+    if big:
+        v[: 120 if big < 100.0 else 2, 0] = big
+    rows[:, W:W + L] = v.view(np.int64)
+    few = rows.copy()
+    few[:, W:W + L] = np.ones_like(v).view(np.int64)
+    for it in (1, 2):
+        eng.upload(rows)
+        eng.download()
+        st = capi.IterStats()
+        p = capi.default_params(tau=0.002, seed=3, iter=it)
+        assert eng.lib.neci_gpu_iterate(eng.ctx, ctypes.byref(p), ctypes.byref(st)) == capi.ERR_SPAWN_FULL
+        assert st.err == capi.ERR_SPAWN_FULL and st.n_attempts == int(v.sum()) > 3072 and st.n_spawned == 0
+        eng.upload(few)
+        orc.upload(few)
+        eng.download()
+        run_both(spec, eng, orc, (2,), tau=0.002, seed=17)
 
 
 @pytest.mark.parametrize("name,lenof_sign", [("hub", 1), ("hub", 2), ("mol", 1), ("mol", 2)])
