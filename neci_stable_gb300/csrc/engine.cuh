@@ -31,7 +31,8 @@ constexpr int kMaxNeigh = 8;
 #endif
 constexpr int kBigAttempts = NECI_BIG_ATTEMPTS;
 constexpr int kBigGranule = 128;  // attempts of heavy parents per entry of DevState::big_at
-constexpr int kBigShift = 36;     // Control::n_big: parents << kBigShift | their attempts
+constexpr int kBigShift = 36;     // Control::n_big: parents << kBigShift | their attempts (modulo 2^36: a step
+                                  // whose n_attempts pass max_att, below 2^33, is refused before they are read)
 constexpr int kHugeAttempts = 1 << 16;  // at most kMaxHuge parents may have more attempts than this
 constexpr int kMaxHuge = 4096;
 constexpr int kCompactTile = 1024;        // slots per block of the compaction scans

@@ -152,6 +152,31 @@ def test_more_attempts_than_the_list_holds(name, lenof_sign, big):
         run_both(spec, eng, orc, (2,), tau=0.002, seed=17)
 
 
+@pytest.mark.parametrize("lenof_sign", [1, 2])
+@pytest.mark.parametrize("n,rest", [(31, 31.0), (32, 1.0), (32, 40.0), (33, 1.0), (64, 2.0)])
+def test_attempts_past_36_bits(lenof_sign, n, rest):
+    # n amplitudes of 2^31 (2^31 attempts each): around and past the 2^36
+    # attempts that the heavy parents' packed count holds, the step is refused
+    # as any other that passes its list
+    spec = hubbard10(lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 12, 1 << 14)
+    rows = random_walkers(spec, 300, np.random.default_rng(43))
+    W, L = spec.W, spec.lenof_sign
+    v = np.ones((len(rows), L))
+    v[:20] = rest
+    v.ravel()[60:60 + n] = -2.0 ** 31
+    rows[:, W:W + L] = v.view(np.int64)
+    eng.upload(rows)
+    st = capi.IterStats()
+    p = capi.default_params(tau=1e-6, seed=3, iter=1)
+    assert eng.lib.neci_gpu_iterate(eng.ctx, ctypes.byref(p), ctypes.byref(st)) == capi.ERR_SPAWN_FULL
+    assert st.n_attempts == int(np.abs(v).sum()) and st.n_spawned == 0
+    v[:] = 1.0
+    rows[:, W:W + L] = v.view(np.int64)
+    eng.upload(rows)
+    assert eng.perform_fcimc_cyc_par(p).n_attempts == v.size
+
+
 @pytest.mark.parametrize("name,lenof_sign", [("hub", 1), ("hub", 2), ("mol", 1), ("mol", 2)])
 @pytest.mark.parametrize("signs", [(32.0, 33.0), (33.0,) * 40, (127.5, 128.0, 129.0, 31.0, 1.0), (40.0, 5000.0, 1.5, 70000.0),
                                    (1.0, 2.0, 31.0)])
