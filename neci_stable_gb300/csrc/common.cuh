@@ -53,59 +53,69 @@ __device__ inline void block_add_u(const unsigned long long (&u)[NU], unsigned l
     __syncthreads();
 }
 
-// A sum of doubles in fixed point, 96 bits in units of 2^-Q: an FP64 addition
-// holds its pipe (about one lane per clock per SM) for as long as the SM's
-// schedulers issue a hundred integer instructions, and this takes a dozen.  A
-// term is rounded to the nearest unit, so the sum is off by at most a half
-// unit per term, less than an FP64 running sum of such terms; the terms the
-// units are too fine for, 2^(63 - Q) and more (and infinities and NaN), go to
-// the target by themselves.
+// A sum of doubles that is exact: terms of 2^(52 - Q) up to 2^(80 - Q), all of
+// whose bits are units of 2^-Q, are added as 96-bit integers; any other term
+// goes to an FP64 sum of the thread's own.  An FP64 addition holds its pipe
+// (about one lane per clock per SM) for as long as the SM's schedulers issue
+// a hundred integer instructions, and this takes some fifteen.  No bit of a
+// term is lost at any size, and a thread's share of 2^31 slots (27 594 terms
+// below 2^80 units) stays below 2^95.  (`own` is the thread's place in shared memory, not a
+// register: the sweeps are short of them, and the atomic is a loop, which the
+// compiler cannot turn into a predicated FP64 addition for every term.)
 template <int Q>
-struct FixedSum {
+struct ExactSum {
     unsigned long long lo = 0;
-    int hi = 0;
-    __device__ inline void add(double a, double *target) {
+    unsigned int hi = 0;
+    __device__ inline void add(double a, double *own) {
         const long long b = __double_as_longlong(a);
-        const int e = (int)(b >> 52) & 0x7FF;
-        if (e >= 1086 - Q) {
-            atomicAdd(target, a);
+        const unsigned int s = ((unsigned int)(b >> 52) & 0x7FFu) - (unsigned int)(1075 - Q);
+        if (s > 27u) {
+            if (b << 1) atomicAdd(own, a);
             return;
         }
-        // the significand's 64 bits (its leading one at bit 63), shifted to units
-        const int sh = 1085 - Q - e;
-        const unsigned long long m = ((unsigned long long)b << 11) | 0x8000000000000000ull;
-        unsigned long long x = sh > 63 ? 0ull : ((m >> sh) + 1) >> 1;
-        if (b < 0) x = 0ull - x;
+        const unsigned long long m = ((unsigned long long)b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+        unsigned long long x = m << s;
+        unsigned int xh = (unsigned int)((m >> 32) >> (32u - s));
+        if (b < 0) {
+            x = 0ull - x;
+            xh = ~xh + (x == 0ull ? 1u : 0u);
+        }
         lo += x;
-        hi += (lo < x ? 1 : 0) + (int)((long long)x >> 63);
+        hi += xh + (lo < x ? 1u : 0u);
     }
 };
 struct PlainSum {
     double v = 0.0;
     __device__ inline void add(double a, double *) { v += a; }
 };
-// The sums every slot adds to, by instance: with one run in fixed point (the
-// sweeps held the FP64 pipe for 65% of their cycles: sweep 1902 to 1825 us and
-// step 8238 to 8076 us at n = 64, step 404 to 394 us at n = 39, 6945 to 6880
-// us on the 6x6 lattice), with a replica pair as they were (twice the
-// accumulators do not fit the registers: merge sweep 37 to 43 us at n = 32).
+// The sums every slot adds to, by instance: exact with one run, FP64 with a
+// replica pair (twice the accumulators do not fit the registers: merge sweep
+// 37 to 43 us at n = 32).  Steps with FP64 sums, and so (us): n = 64 8238 and
+// 8117, 6x6 lattice 6945 and 6917, n = 24 793 and 781, n = 39 404 and 399; the
+// sweep of 63504 determinants with 3000 walkers each 51 and 40.
 template <int LR, int Q>
-using SlotSum = typename std::conditional<LR == 1, FixedSum<Q>, PlainSum>::type;
+using SlotSum = typename std::conditional<LR == 1, ExactSum<Q>, PlainSum>::type;
+// An amplitude (2^-8 to 2^20) and what a step takes from one or adds to it:
+// a death, a rounding, a projected amplitude (2^-24 to 16).
+constexpr int kUnitAmplitude = 60, kUnitChange = 76;
 
 // NF of them over the block, one FP64 atomic per sum (k: its place among the
-// block's; unit: 2^-Q).
+// block's; unit: 2^-Q).  The total is rounded at the conversion only.
 template <int NF>
-struct BlockFixed {
+struct BlockExact {
     unsigned long long lo[NF][8];
     long long hi[NF][8];
     template <int Q>
-    __device__ inline void warp_part(int k, const FixedSum<Q> &f) {
+    __device__ inline void warp_part(int k, const ExactSum<Q> &f) {
+        // parts whose sums over a warp fit 32 bits
         const unsigned int a = __reduce_add_sync(0xffffffffu, (unsigned int)f.lo & 0x3FFFFFu);
         const unsigned int b = __reduce_add_sync(0xffffffffu, (unsigned int)(f.lo >> 22) & 0x3FFFFFu);
         const unsigned int c = __reduce_add_sync(0xffffffffu, (unsigned int)(f.lo >> 44));
-        const int h = (int)__reduce_add_sync(0xffffffffu, (unsigned int)f.hi);
+        const unsigned int d = __reduce_add_sync(0xffffffffu, f.hi & 0xFFFFu);
+        const int e = __reduce_add_sync(0xffffffffu, (int)f.hi >> 16);
         if ((threadIdx.x & 31) == 0) {
-            const __int128 t = (__int128)(a + ((unsigned long long)b << 22)) + ((__int128)c << 44) + ((__int128)h << 64);
+            const __int128 t = (__int128)(a + ((unsigned long long)b << 22)) + ((__int128)c << 44) +
+                               ((__int128)((long long)d + (long long)e * 65536) << 64);
             lo[k][threadIdx.x >> 5] = (unsigned long long)t;
             hi[k][threadIdx.x >> 5] = (long long)(t >> 64);
         }

@@ -389,8 +389,10 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     if (c->rehash_fill) sweep_refill(s, st, n);  // the walker hash is empty
     const int W = s.W, R = s.R;
     constexpr int L = LR;
-    SlotSum<LR, 52> acc_old[L];
-    SlotSum<LR, 56> acc_died[L];
+    SlotSum<LR, kUnitAmplitude> acc_old[L];
+    SlotSum<LR, kUnitChange> acc_died[L];
+    __shared__ double own[LR == 1 ? 2 : 1][kStageTile];  // their terms out of the units' range, by thread
+    if (LR == 1) own[0][threadIdx.x] = own[LR == 1 ? 1 : 0][threadIdx.x] = 0.0;
     double acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0}, acc_born[2] = {0.0, 0.0}, acc_ab[2] = {0.0, 0.0};
     double death_max = 0.0;  // max_death_cpt of this thread's determinants (tau search)
     unsigned long long acc_att = 0, acc_tomb = 0;
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             flags = sr[W + L];
             core = st.n_core > 0 && is_core_flags(flags);
             NECI_FOR_RUNS(k, L) {
-                acc_old[L == 1 ? 0 : k].add(abs_dbl(C[k]), &c->tot_parts_old[k]);
+                acc_old[L == 1 ? 0 : k].add(abs_dbl(C[k]), &own[0][threadIdx.x]);
                 if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
             }
             if (core) {
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                 // there were) is handled below
                 const double aC = abs_dbl(C[k]);
                 const bool le = le_nonneg(idie, aC);
-                acc_died[L == 1 ? 0 : k].add(le ? idie : aC, &c->ndied[k]);
+                acc_died[L == 1 ? 0 : k].add(le ? idie : aC, &own[LR == 1 ? 1 : 0][threadIdx.x]);
                 if (!le) over = true;
                 // C - idie * sign(1, C) with Fortran's sign (+1 for C = -0.0); both products are exact
                 const bool nonneg = !(dbl_bits(C[k]) >> 63) || abs_bits(C[k]) == 0;
@@ -700,14 +702,14 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     const unsigned long long u[2] = {acc_att, acc_tomb};
     unsigned long long *const du[2] = {&c->n_attempts, &c->n_tomb};
     if constexpr (LR == 1) {
-        __shared__ BlockFixed<2> fixed;
-        fixed.warp_part(0, acc_old[0]);
-        fixed.warp_part(1, acc_died[0]);
-        const double v[8] = {acc_hf[0], 0.0, acc_en[0], 0.0, acc_born[0], 0.0, acc_ab[0], 0.0};
-        double *const dst[8] = {&c->hf_cyc[0], nullptr, &c->enum_cyc[0], nullptr, &c->nborn[0], nullptr, &c->naborted[0], nullptr};
-        block_add<8, 2>(v, dst, L, u, du);  // (its barriers are between the parts and the sums)
-        fixed.add(0, 32, 0x1.0p-52, &c->tot_parts_old[0]);
-        fixed.add(1, 64, 0x1.0p-56, &c->ndied[0]);
+        __shared__ BlockExact<2> exact;
+        exact.warp_part(0, acc_old[0]);
+        exact.warp_part(1, acc_died[0]);
+        const double v[6] = {acc_hf[0], acc_en[0], acc_born[0], acc_ab[0], own[0][threadIdx.x], own[LR == 1 ? 1 : 0][threadIdx.x]};
+        double *const dst[6] = {&c->hf_cyc[0], &c->enum_cyc[0], &c->nborn[0], &c->naborted[0], &c->tot_parts_old[0], &c->ndied[0]};
+        block_add<6, 2>(v, dst, 2, u, du);  // (every place taken; its barriers are between the parts and the sums)
+        exact.add(0, 32, 0x1.0p-60, &c->tot_parts_old[0]);
+        exact.add(1, 64, 0x1.0p-76, &c->ndied[0]);
     } else {
         const double v[12] = {acc_old[0].v, acc_old[L - 1].v, acc_hf[0], acc_hf[1], acc_en[0], acc_en[1], acc_died[0].v,
                               acc_died[L - 1].v, acc_born[0], acc_born[1], acc_ab[0], acc_ab[1]};
@@ -1509,8 +1511,12 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     const int W = s.W, R = s.R;
     constexpr int L = LR;
     const bool rdm = LR == 2 && split && s.rdm && p.rdm_defer;
-    SlotSum<LR, 56> a_born[L], a_rm[L];
-    SlotSum<LR, 52> a_tp[L];
+    SlotSum<LR, kUnitChange> a_born[L], a_rm[L];
+    SlotSum<LR, kUnitAmplitude> a_tp[L];
+    __shared__ double own[LR == 1 ? 3 : 1][kStageTile];  // as in k_sweep
+    for (int i = 0; i < (LR == 1 ? 3 : 0); ++i) own[i][threadIdx.x] = 0.0;
+    double *const own_born = &own[0][threadIdx.x], *const own_rm = &own[LR == 1 ? 1 : 0][threadIdx.x],
+                 *const own_tp = &own[LR == 1 ? 2 : 0][threadIdx.x];
     double a_norm[2] = {0, 0}, a_ann[2] = {0, 0}, a_ab[2] = {0, 0};
     unsigned long long a_s[2] = {0, 0}, a_occ = 0, a_holes = 0, a_found = 0, a_tomb = 0;
     // Tiles staged into shared memory by TMA bulk copies as in k_sweep: the
@@ -1558,7 +1564,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
             const int ci = st.core_of_slot[j];
             NECI_FOR_RUNS(k, L) {
                 const double y = st.core_y[(long long)ci * L + k];
-                a_born[L == 1 ? 0 : k].add(abs_dbl(y), &c->nborn[k]);
+                a_born[L == 1 ? 0 : k].add(abs_dbl(y), own_born);
                 if (prod_negative(C[k], y)) a_ann[k] += 2.0 * min_abs(C[k], y);
                 C[k] = y + C[k];
             }
@@ -1623,7 +1629,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                     const double pRemove =
                         dbl_bits(p.occupied_thresh) == dbl_bits(1.0) ? tma : div_dbl(tma, p.occupied_thresh);
                     if (bern(rng, pRemove)) {
-                        a_rm[L == 1 ? 0 : k].add(a, &c->nremoved[k]);
+                        a_rm[L == 1 ? 0 : k].add(a, own_rm);
                         C[k] = 0.0;
                         bool unocc = true;
                         NECI_FOR_RUNS(k2, L) if (abs_bits(C[k2]) >= dbl_bits(kEps12)) unocc = false;
@@ -1633,7 +1639,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
                             r[W + L] = flags | 1ll;
                         }
                     } else {
-                        a_born[L == 1 ? 0 : k].add(tma, &c->nborn[k]);
+                        a_born[L == 1 ? 0 : k].add(tma, own_born);
                         C[k] = fsign(p.occupied_thresh, C[k]);
                     }
                     changed = true;
@@ -1643,7 +1649,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
         if (changed) NECI_FOR_RUNS(k, L) r[W + k] = double_to_word(C[k]);
         occ = false;
         NECI_FOR_RUNS(k, L) {
-            a_tp[L == 1 ? 0 : k].add(abs_dbl(C[k]), &c->tot_parts[k]);
+            a_tp[L == 1 ? 0 : k].add(abs_dbl(C[k]), own_tp);
             a_norm[k] = fma(C[k], C[k], a_norm[k]);  // a statistic: one rounding, one FP64 instruction
             if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
         }
@@ -1689,16 +1695,16 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     unsigned long long *const du[6] = {&c->abs_s[0], &c->abs_s[1], &c->n_occupied, &c->n_holes, &c->n_found,
                                        &c->n_tomb};
     if constexpr (LR == 1) {
-        __shared__ BlockFixed<3> fixed;
-        fixed.warp_part(0, a_born[0]);
-        fixed.warp_part(1, a_rm[0]);
-        fixed.warp_part(2, a_tp[0]);
-        const double v[6] = {a_norm[0], 0.0, a_ann[0], 0.0, a_ab[0], 0.0};
-        double *const dst[6] = {&c->norm[0], nullptr, &c->nannihil[0], nullptr, &c->naborted[0], nullptr};
-        block_add<6, 6>(v, dst, L, u, du);  // (its barriers are between the parts and the sums)
-        fixed.add(0, 32, 0x1.0p-56, &c->nborn[0]);
-        fixed.add(1, 64, 0x1.0p-56, &c->nremoved[0]);
-        fixed.add(2, 96, 0x1.0p-52, &c->tot_parts[0]);
+        __shared__ BlockExact<3> exact;
+        exact.warp_part(0, a_born[0]);
+        exact.warp_part(1, a_rm[0]);
+        exact.warp_part(2, a_tp[0]);
+        const double v[6] = {a_norm[0], a_ann[0], a_ab[0], *own_born, *own_rm, *own_tp};
+        double *const dst[6] = {&c->norm[0], &c->nannihil[0], &c->naborted[0], &c->nborn[0], &c->nremoved[0], &c->tot_parts[0]};
+        block_add<6, 6>(v, dst, 2, u, du);  // (every place taken; its barriers are between the parts and the sums)
+        exact.add(0, 32, 0x1.0p-76, &c->nborn[0]);
+        exact.add(1, 64, 0x1.0p-76, &c->nremoved[0]);
+        exact.add(2, 96, 0x1.0p-60, &c->tot_parts[0]);
     } else {
         const double v[12] = {a_born[0].v, a_born[L - 1].v, a_ann[0], a_ann[1], a_ab[0], a_ab[1], a_rm[0].v, a_rm[L - 1].v,
                               a_tp[0].v, a_tp[L - 1].v, a_norm[0], a_norm[1]};

@@ -381,3 +381,52 @@ def test_sums_of_the_sweeps(n):
         after = np.ascontiguousarray(eng.download()[0][:, W]).view(np.float64)
         total = math.fsum(np.abs(after))
         assert abs(st.tot_parts[0] - total) <= len(after) * 2.0 ** -53 + 16 * 2.0 ** -53 * total
+
+
+@pytest.mark.parametrize("n", [30, 3000])
+@pytest.mark.parametrize("tau,low,high", [(1e-7, -6.0, 0.0), (1e-4, -9.0, -6.0), (1e-4, -1.0, 4.0), (1e-9, 3.0, 9.0)])
+def test_sums_of_the_sweeps_relative(n, tau, low, high):
+    # the sweeps' sums of amplitudes of any size keep the precision of FP64
+    # sums: a sum of terms t is off by at most 40 roundings of its partial
+    # sums (two terms a thread, sixteen additions over a block, an addition
+    # for each of a dozen blocks), 40 x 2^-53 sum |t|
+    import math
+    spec = hubbard10()
+    rng = np.random.default_rng(n)
+    rows = random_walkers(spec, n, rng)
+    W = spec.W
+    amp = 10.0 ** rng.uniform(low, high, len(rows)) * rng.choice([-1.0, 1.0], len(rows))
+    if high > 8.0:
+        amp[3:] = 1.0 + rng.uniform(0.0, 1.0, len(rows) - 3)  # few large ones: their attempts fit
+        amp[:3] *= 1e-3
+    rows[:, W] = amp.view(np.int64)
+    eng = Engine(spec, 1 << 14, 1 << 23)
+
+    def near(got, terms):
+        terms = [float(t) for t in terms]
+        assert abs(got - math.fsum(terms)) <= 40 * 2.0 ** -53 * math.fsum(abs(t) for t in terms), got
+
+    def signs():
+        held, dh, _ = eng.download()
+        o = np.argsort(held[:, 0])
+        return held[o, 0], np.ascontiguousarray(held[o, W]).view(np.float64), dh[o]
+
+    for core in (False, True):
+        for shift in (-3.0, 6.0):
+            eng.upload(rows)
+            if core:
+                eng.set_core_space(rows[:, :W])
+            dets, c, dh = signs()
+            fac = tau * (dh - shift)
+            died = np.minimum(fac * np.abs(c), np.abs(c))
+            st = eng.perform_fcimc_cyc_par(capi.default_params(tau=tau, diag_sft=[shift, shift], seed=4, iter=1))
+            near(st.tot_parts_old[0], np.abs(c))
+            near(st.ndied[0], died)
+            dets1, c1, _ = signs()
+            near(st.tot_parts[0], np.abs(c1))
+            if not core and st.n_spawned == 0:
+                left = np.abs(c - died * np.sign(c))
+                rounded = left < 1.0
+                stays = np.isin(dets, dets1)
+                near(st.nremoved[0], left[rounded & ~stays])
+                near(st.nborn[0], 1.0 - left[rounded & stays])
