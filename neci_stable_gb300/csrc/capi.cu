@@ -881,7 +881,6 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaMemsetAsync(e.st.hash, 0, (size_t)e.st.hash_n * 4, e.stream));
     CK(cudaMemsetAsync(e.st.acc, 0, (size_t)e.st.max_walkers * e.sys.L * 8, e.stream));
     CK(cudaMemsetAsync(e.st.meta, 0, (size_t)e.st.max_walkers * e.sys.L * 4, e.stream));
-    // (not zero only behind a failed step)
     if (e.st.rdm_w) CK(cudaMemsetAsync(e.st.rdm_w, 0, (size_t)e.st.max_walkers * 8, e.stream));
     if (nrows > 0) CK(cudaMemcpyAsync(e.st.dets, ilut, (size_t)nrows * R * 8, cudaMemcpyHostToDevice, e.stream));
     const int compute = (dh && odh) ? 0 : 1;

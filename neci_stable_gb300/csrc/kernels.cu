@@ -1885,10 +1885,12 @@ __device__ inline void diag_end(const DevSys &s, const DevState &st, const DiagS
 // lane per clock per SM: 110 of the 286 us of a step at n = 32 with 2.5e5
 // determinants of 12 electrons.  A determinant that stays for the whole call
 // takes the walk once, and one multiply-add a step in the merge sweep.
+// A step that fails halts those behind it, but the sums are added all the same
+// behind the last of them: the weights of the steps before the failure and of
+// the failed one, whose off-diagonal terms are in the 2-RDM already.
 __global__ void __launch_bounds__(256) k_rdm_diag(DevSys s, DevState st, const IterParams *pp, int use_shared) {
-    if (halted(st)) return;
     const bool defer = pp->rdm_defer != 0;
-    if (defer && pp->iter + 1 < pp->iter_end) return;
+    if (defer ? pp->iter + 1 < pp->iter_end : halted(st)) return;
     extern __shared__ double sh_diag[];
     __shared__ uint16_t pairs[kMaxNel * (kMaxNel - 1) / 2];
     const DiagSums ds = diag_begin(s, use_shared ? sh_diag : nullptr, pairs);

@@ -430,3 +430,52 @@ def test_sums_of_the_sweeps_relative(n, tau, low, high):
                 stays = np.isin(dets, dets1)
                 near(st.nremoved[0], left[rounded & ~stays])
                 near(st.nborn[0], 1.0 - left[rounded & stays])
+
+
+def same_rdm(eng, orc, tag):
+    # atomic FP64 sums on both sides of the comparison: their order is free
+    a, b = eng.rdm2(), orc.rdm2()
+    np.testing.assert_allclose(a, b, rtol=1e-9, atol=1e-12 * max(np.abs(b).max(), 1.0), err_msg=str(tag))
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_rdm_of_a_call_that_fails(batch):
+    # a call of many steps whose eleventh has more attempts than the list
+    # holds: the steps up to it leave both parts of their 2-RDM, as one-step
+    # calls do, and so does the call after the next upload
+    from neci_stable_gb300.engine import iterate_batch
+    spec = molecule(12, 6, lenof_sign=2)
+
+    def fresh(max_spawned):
+        e = Engine(spec, 1 << 14, max_spawned)
+        e.start_from_reference(initial_part=3000.0)
+        e.set_rdm_sampling(True)
+        e.rdm2(reset=True)
+        return e
+
+    def params(it):
+        return capi.default_params(tau=0.01, diag_sft=[2.0, 2.0], seed=8, iter=it)
+
+    free = fresh(1 << 16)
+    start = free.download()[0]
+    attempts = [free.perform_fcimc_cyc_par(params(it)).n_attempts for it in range(1, 21)]
+    fail = next(k for k in range(10, 20) if attempts[k] > max(attempts[:k]) + 2)
+    room = (max(attempts[:fail]) - 1024) // 2 + 1
+    one, many = fresh(room), fresh(room)
+    with pytest.raises(capi.NeciGpuError):
+        for it in range(1, 21):
+            one.perform_fcimc_cyc_par(params(it))
+    assert it == fail + 1
+    with pytest.raises(capi.NeciGpuError) as ei:
+        if batch:
+            iterate_batch([many, free], [params(1), params(21)], 20)
+        else:
+            many.iterate_n(params(1), 20)
+    assert ei.value.code == capi.ERR_SPAWN_FULL
+    same_rdm(many, one, "after the failed call")
+    for e in (one, many):
+        e.upload(start)
+    many.iterate_n(params(1), 5)
+    for it in range(1, 6):
+        one.perform_fcimc_cyc_par(params(it))
+    same_rdm(many, one, "after the next call")
