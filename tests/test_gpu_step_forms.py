@@ -479,3 +479,53 @@ def test_rdm_of_a_call_that_fails(batch):
     for it in range(1, 6):
         one.perform_fcimc_cyc_par(params(it))
     same_rdm(many, one, "after the next call")
+
+
+@pytest.mark.parametrize("name,pop,core,batch,calls", [("hub", 300.0, 0, False, (2, 7, 30)), ("hub", 300.0, 30, True, (7, 1, 12)),
+                                                       ("mol12", 400.0, 0, True, (2, 7, 30)), ("mol12", 400.0, 40, False, (2, 7, 30)),
+                                                       ("mol33", 400.0, 0, False, (3, 9)), ("mol24", 0.0, 0, False, (2, 3))])
+def test_rdm_of_calls_of_several_steps(name, pop, core, batch, calls):
+    # the diagonal summed per slot over a call: slots freed and filled again,
+    # emptied by the annihilation, core slots, both forms of the annihilation
+    # (mol24 passes the lines of the short one), one and two words
+    from neci_stable_gb300.engine import iterate_batch
+    big = name == "mol24"
+    shift = [-5.4] * 2 if name == "hub" else [0.0] * 2  # the ring's population would outgrow its list
+    spec = hubbard10(lenof_sign=2) if name == "hub" else molecule(int(name[3:]), 8 if big else 6, lenof_sign=2)
+    cap = (1 << 21, 1 << 22) if big else (1 << 15, 1 << 17)
+    eng, other, orc = Engine(spec, *cap), Engine(spec, *cap), None
+    orc = Oracle(spec, *cap, hii=eng.hii)
+    if big:
+        rows = random_walkers(spec, 300, np.random.default_rng(5))
+        rows[:, spec.W:spec.W + 2] = (rows[:, spec.W:spec.W + 2].view(np.float64) * 1000.0).view(np.int64)
+        eng.upload(rows)
+    else:
+        eng.start_from_reference(initial_part=pop)
+        eng.iterate_n(capi.default_params(tau=0.02, diag_sft=shift, seed=2, iter=1), 20)
+    rows = eng.download()[0]
+    for e in (eng, other, orc):
+        e.upload(rows)
+        if core:
+            o = np.argsort(-np.abs(rows[:, spec.W:spec.W + 2].view(np.float64)).sum(axis=1), kind="stable")
+            e.set_core_space(rows[o[:core], :spec.W])
+        e.set_rdm_sampling(True)
+        e.rdm2(reset=True)
+    it, removed, placed, spawned = 1, 0.0, 0, 0
+    for n in calls:
+        p = capi.default_params(tau=0.02, diag_sft=shift, seed=6, iter=it)
+        if batch:
+            stats = iterate_batch([other, eng], [p, p], n)[0][1]
+        else:
+            stats = eng.iterate_n(p, n)
+        for k in range(n):
+            sc, rc = orc.iterate(capi.default_params(tau=0.02, diag_sft=shift, seed=6, iter=it + k))
+            assert rc == 0 and stats[k].err == 0 and stats[k].n_occupied == sc.n_occupied
+            removed += stats[k].nremoved[0] + stats[k].nremoved[1]
+            placed += stats[k].n_new
+            spawned = max(spawned, stats[k].n_spawned)
+        it += n
+        same_list(spec, eng, orc, it)
+        same_rdm(eng, orc, it)
+        if batch:
+            same_rdm(other, orc, it)
+    assert removed > 0.0 and placed > 0 and (spawned > 600000) == big
