@@ -898,10 +898,12 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     e.st.n_core = 0;
     if (nrows > 0) launch_upload_fix(e, nrows, compute);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(e.stream));
+    // the status read and reset in the order of the steps' stream: nothing
+    // orders the default stream before the next step
     int err = 0;
-    CK(cudaMemcpy(&err, &e.st.ctl->err, sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemset(&e.st.ctl->err, 0, sizeof(int)));
+    CK(cudaMemcpyAsync(&err, &e.st.ctl->err, sizeof(int), cudaMemcpyDeviceToHost, e.stream));
+    CK(cudaMemsetAsync(&e.st.ctl->err, 0, sizeof(int), e.stream));
+    CK(cudaStreamSynchronize(e.stream));
     e.compact_due = e.rehash_due = false;  // the list and its hash are new
     if (err) return fail(err, "upload: hash table full");
     return NECI_GPU_OK;

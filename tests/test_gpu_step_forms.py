@@ -152,6 +152,20 @@ def test_more_attempts_than_the_list_holds(name, lenof_sign, big):
         run_both(spec, eng, orc, (2,), tau=0.002, seed=17)
 
 
+def test_error_of_the_step_behind_an_upload():
+    # the upload's reset of the status comes before the step's first kernel
+    spec = hubbard10()
+    eng = Engine(spec, 1 << 12, 1 << 10)
+    rows = random_walkers(spec, 700, np.random.default_rng(44))
+    rows[:, spec.W] = np.float64(6.0).view(np.int64)
+    p = capi.default_params(tau=0.002, seed=3, iter=1)
+    st = capi.IterStats()
+    for _ in range(100):
+        eng.upload(rows)
+        assert eng.lib.neci_gpu_iterate(eng.ctx, ctypes.byref(p), ctypes.byref(st)) == capi.ERR_SPAWN_FULL
+        assert st.err == capi.ERR_SPAWN_FULL
+
+
 @pytest.mark.parametrize("lenof_sign", [1, 2])
 @pytest.mark.parametrize("n,rest", [(31, 31.0), (32, 1.0), (32, 40.0), (33, 1.0), (64, 2.0)])
 def test_attempts_past_36_bits(lenof_sign, n, rest):
