@@ -843,6 +843,22 @@ int32_t neci_gpu_init_pchb(neci_gpu_ctx *ctx) {
     return NECI_GPU_OK;
 }
 
+// The most a batch may shrink a context's grids, a power of two up to 16, from
+// the last step: a block of the sweeps keeps to ten tiles of the list in use,
+// a block of the spawn kernel to 24 rounds, or a full context among small
+// ones would hold up the batch with a sixteenth of its blocks: 8.5e5
+// determinants in 2e6 slots beside 63 contexts of 3e3, a step in us with its
+// grids 16 times smaller and so (twice) 1340 and 905, beside 63 of 2e4
+// determinants 1730 and 1370.  (The contexts batch_share's figures are of use
+// a tenth of their capacity.)
+static void update_live_share(Engine &e, long long slots, long long attempts) {
+    const double most = std::min(1.25 * (double)e.st.max_walkers / (double)std::max(slots, 1ll),
+                                 6.0 * (double)e.st.max_spawned / (double)std::max(attempts, 1ll));
+    auto power = [](double x) { return x >= 16.0 ? 16 : x >= 8.0 ? 8 : x >= 4.0 ? 4 : x >= 2.0 ? 2 : 1; };
+    // (up again with a margin, so that the batch graph is not rebuilt to and fro)
+    e.live_share = std::min(std::max(e.live_share, power(most / 1.5)), power(most));
+}
+
 int64_t neci_gpu_check_rows(const int64_t *ilut, int64_t nrows, int32_t nifd, int32_t lenof_sign, int32_t nel,
                             int32_t nbasis) {
     if (nrows < 0 || (nrows > 0 && !ilut) || nifd < 0 || nifd + 1 > kMaxWords || lenof_sign < 1 || lenof_sign > 2)
@@ -905,6 +921,7 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaMemsetAsync(&e.st.ctl->err, 0, sizeof(int), e.stream));
     CK(cudaStreamSynchronize(e.stream));
     e.compact_due = e.rehash_due = false;  // the list and its hash are new
+    update_live_share(e, nrows, 0);
     if (err) return fail(err, "upload: hash table full");
     return NECI_GPU_OK;
 }
@@ -1108,6 +1125,7 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         update_fuse_probe(e, stats[done - 1]);
         update_merge_blocks(e, stats[done - 1]);
         update_short_list(e, stats[done - 1]);
+        update_live_share(e, stats[done - 1].tot_walkers, stats[done - 1].n_attempts);
         update_compact_due(e, stats[done - 1]);
         if (done < n_iter) compact_if_due(e, e.stream);
     }
@@ -1134,15 +1152,16 @@ int32_t neci_gpu_iterate_timed(neci_gpu_ctx *ctx, const neci_gpu_iter_params *p,
     return run_steps(ctx->e, p, n_iter, stats, device_ms);
 }
 
-// How much smaller a context's grids are in a batch of n_ctx.  A block has
-// fixed costs (its tables and counters in, its sums out, at a launch rate the
-// contexts share), which a context on its own pays to fill the GPU and a
-// batch need not.  64 contexts of 5e3 to 6e5 determinants, a step in us with
-// grids 1, 2, 4, 8, 16 and 32 times smaller: 3518, 3365, 3229, 3024, 2900,
-// 3004; the 32 smallest of them 785, 674, 617, 603, 647, 767; the 16
-// smallest 278, 243, 225, 226, 259, 357; the 8 smallest 129, 125, 129, 149;
+// How much smaller a context's grids are in a batch.  A block has fixed costs
+// (its tables and counters in, its sums out, at a launch rate the contexts
+// share), which a context on its own pays to fill the GPU and a batch need
+// not: n_ctx / 4 times smaller, at most 16, and no more than the context's
+// list allows (update_live_share).  64 contexts of 5e3 to 6e5 determinants, a
+// step in us with grids 1, 2, 4, 8, 16 and 32 times smaller: 3518, 3365, 3229,
+// 3024, 2900, 3004; the 32 smallest of them 785, 674, 617, 603, 647, 767; the
+// 16 smallest 278, 243, 225, 226, 259, 357; the 8 smallest 129, 125, 129, 149;
 // the 8 largest 1218, 1200, 1197, 1165, 1130, 1193; the 4 smallest 89, 84, 96.
-static int batch_share(int n_ctx) { return std::min(std::max(n_ctx / 4, 1), 16); }
+static int batch_share(const Engine &e, int n_ctx) { return std::min(std::max(n_ctx / 4, 1), e.live_share); }
 
 int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gpu_iter_params *params, int32_t n_iter,
                                neci_gpu_iter_stats *stats, double *device_ms) {
@@ -1168,7 +1187,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         set_span(*e.h_params, n_iter);
         const unsigned long long v = e.graph_version * 8 + (e.h_params->precision == NECI_PREC_MIXED ? 4 : 0) +
                                      (sweep_fast(*e.h_params) ? 2 : 0) + (e.st.n_core > 0 ? 1 : 0);
-        key.push_back({(const void *)ctxs[c], v});
+        key.push_back({(const void *)ctxs[c], v * 32 + (unsigned long long)batch_share(e, n_ctx)});
     }
     if (!e0.batch_graph || e0.batch_key != key) {
         // One graph for a step of the whole batch: the first context's stream
@@ -1186,7 +1205,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         if (ce == cudaSuccess)
             for (int c = 0; c < n_ctx; ++c) {
                 Engine &e = ctxs[c]->e;
-                e.share = batch_share(n_ctx);
+                e.share = batch_share(e, n_ctx);
                 step_sequence(e);
                 e.share = 1;
             }
@@ -1234,6 +1253,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
             update_fuse_probe(e, e.h_stats[n_iter - 1]);
             update_merge_blocks(e, e.h_stats[n_iter - 1]);
             update_short_list(e, e.h_stats[n_iter - 1]);
+            update_live_share(e, e.h_stats[n_iter - 1].tot_walkers, e.h_stats[n_iter - 1].n_attempts);
             update_compact_due(e, e.h_stats[n_iter - 1]);
         }
     }

@@ -65,6 +65,7 @@ struct Engine {
     // the contexts of a batch share the GPU: each one's grids are this much
     // smaller (batch_share; 1 outside a batch's capture)
     int share = 1;
+    int live_share = 16;  // ... and this much at most (update_live_share)
     int merge_bpsm = 2;  // merge sweep blocks per SM beside the placement (update_merge_blocks)
     bool compact_due = false;  // the last step left more holes than occupied slots
     bool rehash_due = false;   // ... or the walker hash over its load

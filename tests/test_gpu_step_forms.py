@@ -363,6 +363,30 @@ def test_batch_with_smaller_grids(n_ctx):
         assert np.array_equal(canonical(batch[i].download()[0], W), canonical(alone.download()[0], W)), i
 
 
+@pytest.mark.parametrize("n_ctx,sizes", [(16, (17, 12, 12)), (33, (18, 12, 15)), (64, (17, 13, 13))])
+def test_batch_of_uneven_contexts(n_ctx, sizes):
+    # the first context's capacity is 4 to 64 times the others': its grids
+    # shrink by its part of the batch, theirs by their number
+    from neci_stable_gb300.engine import iterate_batch
+    specs = [molecule(14, 8), hubbard10(lenof_sign=2), molecule(12, 6)]
+    walkers = [random_walkers(specs[0], 20000, np.random.default_rng(80), scale=2.0)]
+    walkers += [random_walkers(sp, 900, np.random.default_rng(81 + k), scale=4.0) for k, sp in enumerate(specs[1:])]
+    params = [capi.default_params(tau=0.004, seed=170 + i, iter=1) for i in range(n_ctx)]
+
+    def fresh(i):
+        k = 0 if i == 0 else 1 + i % 2
+        e = Engine(specs[k], 1 << sizes[k], 1 << sizes[k] + 1)
+        e.upload(walkers[k])
+        return e, specs[k].W
+
+    batch = [fresh(i)[0] for i in range(n_ctx)]
+    iterate_batch(batch, params, 5)
+    for i in (0, 1, 2, n_ctx - 1):
+        alone, W = fresh(i)
+        alone.iterate_n(params[i], 5)
+        assert np.array_equal(canonical(batch[i].download()[0], W), canonical(alone.download()[0], W)), i
+
+
 @pytest.mark.parametrize("n", [1, 31, 257, 1500])
 def test_sums_of_the_sweeps(n):
     # the sweeps' sums in fixed point: amplitudes around its limits (2048 for
