@@ -761,9 +761,14 @@ def main():
         traffic = per_unit * r["last"][unit]
     # achieved GB/s of every kernel (algorithmic bytes of the last profiled step)
     kernel_gbs = {}
+    # (a short spawn list is compressed by the lookup's kernel, which then holds
+    # the time of both stages)
+    gathered = "ann_compress" in kt and kt["ann_compress"][0] == 0.0
     for k, (ms, cnt) in kt.items():
         b = algorithmic_bytes(k, r["last"], W, L, nnz, fused)
-        if b > 0:
+        if gathered and k == "ann_probe":
+            b += algorithmic_bytes("ann_compress", r["last"], W, L, nnz, fused)
+        if b > 0 and ms > 0.0:
             kernel_gbs[k] = b / (ms / cnt / 1e3) / 1e9
     ann = tuple(k for k in ("ann_probe", "ann_compress", "ann_insert") if k in kt)
     ann_ms = sum(kt[k][0] / kt[k][1] for k in ann)
@@ -782,12 +787,13 @@ def main():
     sort_ms = sum(v["ms"] for v in sort_stages.values())
     sort_bytes = sum(v["algorithmic_bytes"] for v in sort_stages.values())
     ktm = {k: v for k, v in r["ktimes_mixed"].items() if v[1] > 0}
-    # sweep, spawn, compress, decide, place, merge, final (a short spawn list,
-    # not this workload's, takes two fewer); the probe unless the spawn kernel
-    # does it; the core projection and the sum of its
-    # long rows (a compaction, when a step leaves more holes than walkers, and
-    # a rebuild of the walker hash run between calls)
+    # sweep, spawn, compress, decide, place, merge, final; the probe unless the
+    # spawn kernel does it; the core projection and the sum of its long rows;
+    # for a short spawn list one kernel looks up and compresses and, up to 2e5
+    # records, one decides and places (a compaction, when a step leaves more
+    # holes than walkers, and a rebuild of the walker hash run between calls)
     launches_per_step = 7 + (2 if r["last"]["n_core"] > 0 else 0) + (0 if fused else 1)
+    launches_per_step -= (1 if gathered else 0) + (1 if r["last"]["n_spawned"] <= 200_000 else 0)
     line = {
         "metric": METRIC, "value": updates / dev_s, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": 1000.0 * dev_s / args.steps, "higher_is_better": True,

@@ -144,14 +144,13 @@ void lookup_passes(Engine &e) {
     else stage(e, K_ANN_PROBE, [&] { launch_ann_probe(e, e.stream); });
 }
 
-// The compression of the hash form (the sort form has none left; for a short
-// list the lookup's kernel does it, and the stage is counted with no time of
-// its own).
+// The compression of the hash form (the sort form has none left).  For a short
+// list the lookup's kernel does it: the stage is counted, as the step has it,
+// with no time, and its time is the lookup's.
 void compress_pass(Engine &e) {
     if (e.ann_mode == NECI_ANN_SORT) return;
-    stage(e, K_ANN_COMPRESS, [&] {
-        if (!e.gather || fused_lookup(e)) launch_ann_compress(e, e.stream);
-    });
+    if (!e.gather || fused_lookup(e)) stage(e, K_ANN_COMPRESS, [&] { launch_ann_compress(e, e.stream); });
+    else if (e.profiling) e.kernel_launches[K_ANN_COMPRESS] += 1;
 }
 
 // The new determinants of a step.

@@ -308,6 +308,33 @@ def test_short_and_long_spawn_lists(name, lenof_sign, walkers):
             same_list(spec, eng, orc, (it, scale))
 
 
+def form_of_a_step(eng, p):
+    """Whether the lookup's kernel compressed the spawns of one step (the
+    compression is counted, with no time of its own)."""
+    eng.set_profiling(True)
+    eng.kernel_times()
+    st = eng.perform_fcimc_cyc_par(p)
+    kt = eng.kernel_times()
+    eng.set_profiling(False)
+    assert st.err == 0 and kt["ann_compress"][1] == 1 and kt["ann_probe"][1] == 1 and kt["ann_probe"][0] > 0.0
+    return kt["ann_compress"][0] == 0.0
+
+
+def test_times_of_a_short_spawn_list():
+    spec = molecule(24, 8)
+    eng = Engine(spec, 1 << 21, 1 << 22)
+    rows = random_walkers(spec, 300, np.random.default_rng(12))
+    for scale, short in ((1.0, True), (4000.0, False)):
+        r = rows.copy()
+        r[:, spec.W] = (rows[:, spec.W].view(np.float64) * scale).view(np.int64)
+        eng.upload(r)
+        p = capi.default_params(tau=0.02, seed=29, iter=1)
+        st = eng.perform_fcimc_cyc_par(p)  # chooses the form of the next step
+        assert st.n_spawned < 400000 if short else st.n_spawned > 600000, st.n_spawned
+        p.iter = 2
+        assert form_of_a_step(eng, p) == short
+
+
 @pytest.mark.parametrize("lenof_sign", [1, 2])
 @pytest.mark.parametrize("n,max_spawned", [(1, 4096), (1023, 4096), (1024, 4096), (1025, 700), (5000, 700), (5000, 1500), (5000, 5000)])
 def test_download_packs_the_occupied_slots(lenof_sign, n, max_spawned):
