@@ -842,6 +842,20 @@ int32_t neci_gpu_init_pchb(neci_gpu_ctx *ctx) {
     return NECI_GPU_OK;
 }
 
+// Whether the next steps take the annihilation's kernels of a short spawn list,
+// from the records of the last step, with a margin so that the choice does not
+// flap; before a context's first step, from its list: a step spawns about a
+// record for every second determinant (0.05 to 1 of them at n = 24 to 64).
+static void update_short_list(Engine &e, long long records) {
+    auto below = [&](bool now, long long line) { return records <= (now ? line : line - line / 4); };
+    const bool gather = below(e.gather, kGatherSpawns), small = below(e.short_list, kShortSpawns);
+    if (gather != e.gather || small != e.short_list) {
+        e.gather = gather;
+        e.short_list = small;
+        drop_graphs(e);
+    }
+}
+
 // The most a batch may shrink a context's grids, a power of two up to 16, from
 // the last step: a block of the sweeps keeps to ten tiles of the list in use,
 // a block of the spawn kernel to 24 rounds, or a full context among small
@@ -921,6 +935,7 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaStreamSynchronize(e.stream));
     e.compact_due = e.rehash_due = false;  // the list and its hash are new
     update_live_share(e, nrows, 0);
+    if (!e.stepped) update_short_list(e, nrows / 2);
     if (err) return fail(err, "upload: hash table full");
     return NECI_GPU_OK;
 }
@@ -1039,19 +1054,6 @@ static void update_merge_blocks(Engine &e, const neci_gpu_iter_stats &last) {
     }
 }
 
-// Whether the next steps take the annihilation's kernels of a short spawn list,
-// from the last step's records, with a margin so that the choice does not
-// flap.
-static void update_short_list(Engine &e, const neci_gpu_iter_stats &last) {
-    auto below = [&](bool now, long long line) { return last.n_spawned <= (now ? line : line - line / 4); };
-    const bool gather = below(e.gather, kGatherSpawns), small = below(e.short_list, kShortSpawns);
-    if (gather != e.gather || small != e.short_list) {
-        e.gather = gather;
-        e.short_list = small;
-        drop_graphs(e);
-    }
-}
-
 // Compaction of the walker list runs between calls, before the first step
 // of a call whose last step left more holes than occupied slots (the rule
 // k_final applies to Control::compact; the compaction kernels check that
@@ -1123,7 +1125,8 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         done += batch;
         update_fuse_probe(e, stats[done - 1]);
         update_merge_blocks(e, stats[done - 1]);
-        update_short_list(e, stats[done - 1]);
+        update_short_list(e, stats[done - 1].n_spawned);
+        e.stepped = true;
         update_live_share(e, stats[done - 1].tot_walkers, stats[done - 1].n_attempts);
         update_compact_due(e, stats[done - 1]);
         if (done < n_iter) compact_if_due(e, e.stream);
@@ -1251,7 +1254,8 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         if (!first_err) {
             update_fuse_probe(e, e.h_stats[n_iter - 1]);
             update_merge_blocks(e, e.h_stats[n_iter - 1]);
-            update_short_list(e, e.h_stats[n_iter - 1]);
+            update_short_list(e, e.h_stats[n_iter - 1].n_spawned);
+            e.stepped = true;
             update_live_share(e, e.h_stats[n_iter - 1].tot_walkers, e.h_stats[n_iter - 1].n_attempts);
             update_compact_due(e, e.h_stats[n_iter - 1]);
         }

@@ -62,6 +62,7 @@ struct Engine {
     // the last step's spawn list was short: lookup and compression, decision
     // and placement in one kernel each (update_short_list)
     bool gather = true, short_list = true;
+    bool stepped = false;  // the context has made a step
     // the contexts of a batch share the GPU: each one's grids are this much
     // smaller (batch_share; 1 outside a batch's capture)
     int share = 1;

@@ -14,12 +14,14 @@ the CPU oracle, bit for bit:
 from __future__ import annotations
 
 import ctypes
+import itertools
 
 import numpy as np
 import pytest
 
 from neci_stable_gb300 import capi
 from neci_stable_gb300.engine import Engine
+from neci_stable_gb300.systems import make_rows
 from oracle.oracle import Oracle
 
 from helpers import canonical, hubbard10, hubbard_square, molecule, random_walkers
@@ -333,6 +335,20 @@ def test_times_of_a_short_spawn_list():
         assert st.n_spawned < 400000 if short else st.n_spawned > 600000, st.n_spawned
         p.iter = 2
         assert form_of_a_step(eng, p) == short
+
+
+def test_form_of_the_first_step():
+    # a context that has not stepped yet takes the form of its list's length
+    spec = molecule(24, 8)
+    half = [sum(1 << 2 * o for o in c) for c in itertools.combinations(range(24), 4)][:1200]
+    dets = (np.array(half)[:, None] | (np.array(half)[None, :] << 1)).reshape(-1, 1)  # 1.44e6
+    p = capi.default_params(tau=0.001, seed=29, iter=1)
+    for lengths in ((1000, dets.size), (dets.size, 1000)):
+        eng = Engine(spec, 1 << 21, 1 << 22)
+        for n in lengths:
+            eng.upload(make_rows(dets[:n], np.ones(n), np.zeros(n, dtype=np.int64)))
+        assert form_of_a_step(eng, p) == (n == 1000)
+        eng.close()
 
 
 @pytest.mark.parametrize("lenof_sign", [1, 2])
