@@ -75,7 +75,9 @@ struct Control {
                                         // the walker list is uploaded again
     int rehash;                         // rebuild the walker hash before the next step (k_hash_clear,
                                         // k_hash_fill)
-    int rehash_fill;                    // k_final cleared the walker hash: this step's sweep refills it
+    int clear_next;                     // the next step's k_final clears the walker hash
+    int hash_clear;                     // ... this step's does (set by its sweep)
+    int rehash_fill;                    // the last step's k_final cleared it: this step's sweep refills it
     int compact;                        // compact the walker list at the next step
     unsigned long long compact_k;       // occupied slots kept by the compaction
     unsigned long long compact_pos_k;   // occupied slots below compact_k

@@ -97,12 +97,10 @@ __global__ void k_hash_fill(DevSys s, DevState st) {
         hash_insert(st, j, neci_hash(d, s.W, sh_rh2), st.ctl);
     }
 }
-// Ends a rebuild (the flag stays up until both kernels have seen it); a
-// refill left to the next sweep is done with it.
+// Ends a rebuild (the flag stays up until both kernels have seen it).
 __global__ void k_hash_done(DevState st) {
     if (threadIdx.x != 0 || halted(st) || !st.ctl->rehash) return;
     st.ctl->rehash = 0;
-    st.ctl->rehash_fill = 0;
 }
 
 // ===========================================================================
@@ -385,7 +383,10 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     const IterParams p = *pp;
     Control *c = st.ctl;
     const long long n = slots_in_use(st);
-    if (blockIdx.x == 0 && threadIdx.x == 0) c->n_pre = (unsigned long long)n;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c->n_pre = (unsigned long long)n;
+        c->hash_clear = c->clear_next;
+    }
     if (c->rehash_fill) sweep_refill(s, st, n);  // the walker hash is empty
     const int W = s.W, R = s.R;
     constexpr int L = LR;
@@ -1935,24 +1936,29 @@ __global__ void __launch_bounds__(256) k_rdm_freed(DevSys s, DevState st, const 
 // freed ones; the new determinants are occupied, and the freed slots the
 // placement did not fill are holes.  A walker hash whose live entries and
 // tombstones pass 60% of the buckets is rebuilt between two calls (the host
-// is told in `reserved` of the record); within a call, past 70%, it is
-// cleared here (the return value) and the next step's sweep refills it.
-__device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
+// is told in `reserved` of the record); within a call, past 65%, the next
+// step's k_final clears it and the sweep behind that refills it, when the call
+// has both.
+__device__ void final_record(const DevState &st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
                             int advance_iter, long long n_core, int split) {
-    const long long next = pp->iter + 1;
+    Control *c = st.ctl;
+    // (read together, before the first store)
+    const long long next = pp->iter + 1, begin = pp->iter_begin, end = pp->iter_end;
+    const int stop = c->halted, err = c->err;
+    const bool cleared = advance_iter && c->hash_clear;  // the walker hash, by this kernel
+    const unsigned long long tomb = cleared ? 0ull : c->n_tomb;
     neci_gpu_iter_stats *out = base;
     if (advance_iter) {
-        const long long k = pp->iter - pp->iter_begin;
+        const long long k = next - 1 - begin;
         out = base + (k < max_out ? k : max_out - 1);
         pp->iter = next;
     }
-    Control *c = st.ctl;
-    if (c->halted) {
+    if (stop) {
         // a previous step failed: report its status again, change nothing
         neci_gpu_iter_stats r{};
-        r.err = c->halted;
+        r.err = stop;
         *out = r;
-        return 0;
+        return;
     }
     if (c->tot_walkers > (unsigned long long)st.max_walkers) c->tot_walkers = (unsigned long long)st.max_walkers;
     if (split) {
@@ -1986,33 +1992,36 @@ __device__ int final_record(const DevState &st, neci_gpu_iter_stats *base, int m
     r.n_unique = (long long)(c->n_reps_nz + c->n_found);
     r.n_new = (long long)c->n_new;
     r.n_core = n_core;
-    r.err = c->err;
-    const unsigned long long used = c->n_occupied + c->n_tomb;
-    const bool more = advance_iter && next < pp->iter_end && !c->err;  // another step of the call follows
-    const bool in_call = more && used * 10ull > st.hash_n * 7ull;
-    c->rehash_fill = in_call ? 1 : 0;
-    c->rehash = !more && used * 10ull > st.hash_n * 6ull ? 1 : 0;
-    if (in_call) c->n_tomb = 0;
-    r.reserved = c->rehash;
+    r.err = err;
+    const unsigned long long used = (unsigned long long)r.n_occupied + tomb;
+    const long long left = advance_iter && !err ? end - next : 0;  // steps of the call that follow
+    const int rebuild = left == 0 && used * 10ull > st.hash_n * 6ull ? 1 : 0;
+    if (cleared) c->n_tomb = 0;
+    c->rehash_fill = cleared ? 1 : 0;
+    c->clear_next = left >= 2 && used * 20ull > st.hash_n * 13ull ? 1 : 0;
+    c->rehash = rebuild;
+    r.reserved = rebuild;
     *out = r;
     // compact the list before the next call when holes outnumber occupied slots
     c->compact = (c->tot_walkers > (unsigned long long)(4 * kCompactTile) && c->n_holes * 2ull > c->tot_walkers) ? 1 : 0;
     // a failed step halts the ones after it (in the same graph batch)
-    if (c->err) c->halted = c->err;
+    if (err) c->halted = err;
     reset_counters(c);
-    return in_call ? 1 : 0;
 }
 
+// The blocks behind the first only clear: hash_clear is set by this step's
+// sweep and not changed here, so they need not wait for the record.  One block
+// alone takes about 2.5 ms for a table of 2^27 buckets, a third of a step of
+// the 6x6 lattice (calls of 90 steps with two to three rebuilds: 7.70 and 7.60
+// ms a step); a kernel of its own behind every step would cost each of them an
+// idle launch.
 __global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
                                                 int advance_iter, long long n_core, int split) {
-    __shared__ int clear;
-    if (threadIdx.x == 0) clear = final_record(st, base, max_out, pp, advance_iter, n_core, split);
-    __syncthreads();
-    if (!clear) return;
-    // one block: within a call a rebuild is due about once in hundreds of
-    // steps, and a grid-wide kernel would cost an idle launch in each of them
+    if (blockIdx.x == 0 && threadIdx.x == 0) final_record(st, base, max_out, pp, advance_iter, n_core, split);
+    if (!advance_iter || !st.ctl->hash_clear) return;
     uint4 *t = reinterpret_cast<uint4 *>(st.hash);
-    for (unsigned long long b = threadIdx.x; b < st.hash_n / 4; b += blockDim.x)
+    for (unsigned long long b = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; b < st.hash_n / 4;
+         b += (unsigned long long)gridDim.x * blockDim.x)
         t[b] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
 }
 
@@ -2200,7 +2209,9 @@ void launch_rdm_freed(Engine &e, cudaStream_t s) {
 }
 
 void launch_final(Engine &e, cudaStream_t s, int advance_iter, int split) {
-    k_final<<<1, 1024, 0, s>>>(e.st, e.h_stats, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
+    // a block per 64 MB of the walker hash
+    const int grid = (int)std::min<unsigned long long>(std::max(e.st.hash_n >> 24, 1ull), (unsigned long long)e.num_sms);
+    k_final<<<grid, 1024, 0, s>>>(e.st, e.h_stats, e.max_stats, e.d_params, advance_iter, e.st.n_core, split);
 }
 
 }  // namespace neci

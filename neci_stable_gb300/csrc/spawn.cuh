@@ -505,16 +505,16 @@ __global__ void __launch_bounds__(128, NECI_SPAWN_BLOCKS_PER_SM)
     // attempts in all; sh_n[0] of them have entries (kept in shared memory:
     // the loops below are short of registers)
     if (threadIdx.x == 0) {
-        // (the sweep's 64-bit count: the heavy parents' part of n_big wraps at
-        // 2^36 attempts)
-        const bool over = st.ctl->n_attempts > (unsigned long long)st.max_att;
-        if (over && !halted(st)) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
-        // a step with more attempts than the list holds fails and makes none:
-        // the sweep leaves out entries that do not fit, and what lies in
-        // their places need not be an entry (a list read packs diagonal
-        // elements there)
-        sh_n[0] = (long long)st.ctl->n_att;
-        sh_n[1] = over || halted(st) ? 0 : (long long)st.ctl->n_attempts;
+        // a step with more attempts than the list holds (by the sweep's 64-bit
+        // count: the heavy parents' part of n_big wraps at 2^36) fails and
+        // makes none: the sweep leaves out entries that do not fit, and what
+        // lies in their places need not be an entry (a list read packs
+        // diagonal elements there)
+        const unsigned long long total = st.ctl->n_attempts, entries = st.ctl->n_att;
+        const bool stop = halted(st), over = total > (unsigned long long)st.max_att;
+        if (over && !stop) set_err(st.ctl, NECI_GPU_ERR_SPAWN_FULL);
+        sh_n[0] = (long long)entries;
+        sh_n[1] = over || stop ? 0 : (long long)total;
     }
     __syncthreads();
     // a block with no attempts leaves (the grid is sized to the capacity)

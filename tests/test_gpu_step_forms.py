@@ -69,6 +69,28 @@ def test_walker_hash_at_high_load(lenof_sign, calls):
     eng.close()
 
 
+def test_large_walker_hash_rebuilt_inside_a_call():
+    # a table that several blocks clear (2^25 buckets): one call of 60 steps,
+    # whose determinants take more places of the table than it may hold,
+    # against calls of one step, which rebuild it between them.  A determinant
+    # missing from the table would be counted as a new one.
+    spec = hubbard_square(4, 4, 16)
+    half = [sum(1 << 2 * o for o in c) for c in itertools.combinations(range(16), 8)][::12][:1000]
+    dets = (np.array(half)[:, None] | (np.array(half)[None, :] << 1)).reshape(-1, 1)
+    counts = []
+    for last in ((60,), (1,) * 60):
+        eng = Engine(spec, 1 << 24, 1 << 24)
+        eng.upload(make_rows(dets, np.full(dets.size, 2.0), np.full(dets.size, 1 << 13)))
+        stats = []
+        for n, shift in [(10, 6.0)] * 6 + [(n, -9.0) for n in last]:
+            stats += eng.iterate_n(capi.default_params(tau=0.01, diag_sft=[shift] * 2, seed=6, iter=1 + len(stats)), n)
+        assert all(s.err == 0 and s.reserved == 0 for s in stats)
+        counts.append([(s.n_occupied, s.n_new, s.n_unique, s.n_spawned, s.n_attempts) for s in stats])
+        eng.close()
+    assert sum(c[1] for c in counts[0]) > 0.65 * 2 ** 25
+    assert counts[0] == counts[1]
+
+
 def test_hash_after_entry_points_between_steps():
     # the counters and the walker hash an entry point finds between two steps
     spec = molecule(12, 6)
