@@ -176,6 +176,7 @@ void step_sequence(Engine &e) {
     if (e.sys.rdm) {
         if (e.profiling) {
             stage(e, K_RDM, [&] { launch_rdm_freed(e, e.stream); });
+            e.kernel_launches[K_RDM] -= 1;  // the first part of the step's one stage
         } else {
             cudaEventRecord(e.sweep_ev, e.stream);
             cudaStreamWaitEvent(e.side, e.sweep_ev, 0);

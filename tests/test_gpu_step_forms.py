@@ -359,6 +359,20 @@ def test_times_of_a_short_spawn_list():
         assert form_of_a_step(eng, p) == short
 
 
+def test_stages_are_counted_once_a_step():
+    spec = molecule(12, 6, lenof_sign=2)
+    eng = Engine(spec, 1 << 14, 1 << 16)
+    eng.start_from_reference(initial_part=300.0)
+    eng.set_rdm_sampling(True)
+    eng.set_profiling(True)
+    eng.kernel_times()
+    eng.iterate_n(capi.default_params(tau=0.01, seed=29, iter=1), 7)
+    kt = eng.kernel_times()
+    for stage in ("sweep", "spawn", "ann_probe", "ann_compress", "ann_insert", "merge_stats", "rdm", "final"):
+        assert kt[stage][1] == 7, (stage, kt[stage])
+    assert kt["rdm"][0] > 0.0
+
+
 def test_form_of_the_first_step():
     # a context that has not stepped yet takes the form of its list's length
     spec = molecule(24, 8)
