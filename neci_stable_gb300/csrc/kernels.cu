@@ -243,15 +243,23 @@ __global__ void k_compact_done(DevState st) {
 // Reading the list: the occupied (or core) slots packed in slot order on the
 // device, so that the host copies their rows once, straight to its caller.
 // (Copying every slot and packing on the host took 2.2 ms for 2.9e5 of 3.6e5
-// slots.)  Tiles and ranks as in the compaction; `off` gets each tile's first
-// place and, behind the last tile, their number.
+// slots.)  Tiles and ranks as in the compaction; tile_off gets each tile's
+// first place and, behind the last tile, their number.
 // ===========================================================================
+// A slot whose amplitude is not a number is no walker of the list that is read.
+__device__ inline bool slot_listed(const DevSys &s, const DevState &st, long long j) {
+    const long long *r = st.dets + j * s.R;
+    if (st.n_core > 0 && is_core_flags(r[s.W + s.L])) return true;
+    NECI_FOR_RUNS(k, s.L)
+        if (fabs(word_to_double(r[s.W + k])) >= kEps12) return true;
+    return false;
+}
 __global__ void __launch_bounds__(kCompactTile) k_read_count(DevSys s, DevState st, long long n) {
     const long long ntiles = (n + kCompactTile - 1) / kCompactTile;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long j = t * kCompactTile + threadIdx.x;
         unsigned int count;
-        (void)tile_rank(j < n && slot_kept(s, st, j), count);
+        (void)tile_rank(j < n && slot_listed(s, st, j), count);
         if (threadIdx.x == 0) st.tile_count[t] = count;
     }
 }
@@ -286,7 +294,7 @@ __global__ void __launch_bounds__(kCompactTile) k_read_pack(DevSys s, DevState s
     const unsigned int first = st.tile_off[t0];
     for (long long t = t0 + blockIdx.x; t < t1; t += gridDim.x) {
         const long long j = t * kCompactTile + threadIdx.x;
-        const bool keep = j < n && slot_kept(s, st, j);
+        const bool keep = j < n && slot_listed(s, st, j);
         unsigned int count;
         const long long pos = (long long)(st.tile_off[t] - first) + tile_rank(keep, count);
         if (!keep) continue;

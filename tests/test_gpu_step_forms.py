@@ -419,6 +419,27 @@ def test_download_packs_the_occupied_slots(lenof_sign, n, max_spawned):
     eng.close()
 
 
+@pytest.mark.parametrize("lenof_sign", [1, 2])
+def test_download_of_amplitudes_at_the_edges(lenof_sign):
+    # listed: |C| >= 1e-12 in some run, infinities among them; not: smaller
+    # ones, zeros of either sign, NaN
+    spec = molecule(12, 6, lenof_sign=lenof_sign)
+    eng = Engine(spec, 1 << 12, 1 << 12)
+    rows = random_walkers(spec, 200, np.random.default_rng(3))
+    W, L = spec.W, spec.lenof_sign
+    edge = np.array([1.0, 1e-12, np.nextafter(1e-12, 0.0), -1e-12, 0.0, -0.0, np.nan, -np.nan, np.inf, -np.inf, 5e-324])
+    v = np.zeros((len(rows), L))
+    v[:, 0] = edge[np.arange(len(rows)) % edge.size]
+    v[:, L - 1] = edge[np.arange(len(rows)) % edge.size if L == 1 else np.arange(len(rows)) // edge.size % edge.size]
+    rows[:, W:W + L] = v.view(np.int64)
+    eng.upload(rows)
+    with np.errstate(invalid="ignore"):
+        listed = (np.abs(v) >= 1e-12).any(axis=1)
+    assert np.array_equal(eng.download()[0][:, :W + L], rows[listed][:, :W + L])
+    eng.set_core_space(rows[listed][:30, :W])
+    assert np.array_equal(eng.download()[0][:, :W + L], rows[listed][:, :W + L])
+
+
 @pytest.mark.parametrize("n_ctx", [7, 8, 33, 68])
 def test_batch_with_smaller_grids(n_ctx):
     # the grids of a batch's contexts shrink from 8 contexts on, down to the
