@@ -59,9 +59,10 @@ __device__ inline void block_add_u(const unsigned long long (&u)[NU], unsigned l
 // (about one lane per clock per SM) for as long as the SM's schedulers issue
 // a hundred integer instructions, and this takes some fifteen.  No bit of a
 // term is lost at any size, and a thread's share of 2^31 slots (27 594 terms
-// below 2^80 units) stays below 2^95.  (`own` is the thread's place in shared memory, not a
-// register: the sweeps are short of them, and the atomic is a loop, which the
-// compiler cannot turn into a predicated FP64 addition for every term.)
+// below 2^80 units) stays below 2^95.  `own` is the thread's place in shared
+// memory, not a register: the sweeps are short of them, and the atomic is a
+// loop, which the compiler cannot turn into a predicated FP64 addition for
+// every term.
 template <int Q>
 struct ExactSum {
     unsigned long long lo = 0;
@@ -91,13 +92,15 @@ struct PlainSum {
 // The sums every slot adds to, by instance: exact with one run, FP64 with a
 // replica pair (twice the accumulators do not fit the registers: merge sweep
 // 37 to 43 us at n = 32).  Steps with FP64 sums, and so (us): n = 64 8238 and
-// 8117, 6x6 lattice 6945 and 6917, n = 24 793 and 781, n = 39 404 and 399; the
+// 8134, 6x6 lattice 6945 and 6917, n = 24 793 and 782, n = 39 404 and 396; the
 // sweep of 63504 determinants with 3000 walkers each 51 and 40.
 template <int LR, int Q>
 using SlotSum = typename std::conditional<LR == 1, ExactSum<Q>, PlainSum>::type;
-// An amplitude (2^-8 to 2^20) and what a step takes from one or adds to it:
-// a death, a rounding, a projected amplitude (2^-24 to 16).
-constexpr int kUnitAmplitude = 60, kUnitChange = 76;
+// An amplitude (2^-18 to 2^10) and what a step takes from one or adds to it:
+// a death, a rounding, a projected amplitude (2^-26 to 4).  (Units of 2^-64
+// and 2^-76 left the core amplitudes of a decaying projection out: 45.2 and
+// 44.6 us a step on the 10-site ring.)
+constexpr int kUnitAmplitude = 70, kUnitChange = 78;
 
 // NF of them over the block, one FP64 atomic per sum (k: its place among the
 // block's; unit: 2^-Q).  The total is rounded at the conversion only.
@@ -146,12 +149,13 @@ struct BlockExact {
 // (6 adds for four values), instead of 5 shuffle levels each.  12 values of
 // 256 threads: 156 FP64 warp instructions before, at most 102 now, 34 with
 // four of them non-zero.
-template <int NV, int NU>
-__device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV], int L, const unsigned long long (&u)[NU],
-                                 unsigned long long *const (&du)[NU]) {
-    __shared__ double red[NV][256];
-    __shared__ double *to[NV];
-    __shared__ unsigned int row[NV];   // the non-zero values, in order
+// NO more doubles are in the last rows of `red` already (the sweeps' threads
+// add to their places there).
+template <int NV, int NO, int NU>
+__device__ inline void block_add_rows(double (*red)[256], const double (&v)[NV], double *const (&dst)[NV + NO], int L,
+                                      const unsigned long long (&u)[NU], unsigned long long *const (&du)[NU]) {
+    __shared__ double *to[NV + NO];
+    __shared__ unsigned int row[NV + NO];  // the non-zero values, in order
     __shared__ unsigned int live[8];   // the warps' masks of non-zero values
     __shared__ BlockCounts<NU> counts;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
@@ -162,9 +166,12 @@ __device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV]
             red[m][t] = v[m];
             if ((unsigned long long)__double_as_longlong(v[m]) << 1) mask |= 1u << m;
         }
+#pragma unroll
+    for (int m = NV; m < NV + NO; ++m)
+        if ((unsigned long long)__double_as_longlong(red[m][t]) << 1) mask |= 1u << m;
     if (t == 0) {
 #pragma unroll
-        for (int m = 0; m < NV; ++m) to[m] = dst[m];
+        for (int m = 0; m < NV + NO; ++m) to[m] = dst[m];
     }
     counts.warp_part(u);
     mask = __reduce_or_sync(0xffffffffu, mask);
@@ -198,6 +205,12 @@ __device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV]
         if ((t & 7) == 0 && (t >> 3) < n) atomicAdd(to[row[k]], s);
     }
     __syncthreads();
+}
+template <int NV, int NU>
+__device__ inline void block_add(const double (&v)[NV], double *const (&dst)[NV], int L, const unsigned long long (&u)[NU],
+                                 unsigned long long *const (&du)[NU]) {
+    __shared__ double red[NV][256];
+    block_add_rows<NV, 0, NU>(red, v, dst, L, u, du);
 }
 
 // Warp-aggregated append of `want` items: returns this lane's first index.

@@ -400,8 +400,11 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
     constexpr int L = LR;
     SlotSum<LR, kUnitAmplitude> acc_old[L];
     SlotSum<LR, kUnitChange> acc_died[L];
-    __shared__ double own[LR == 1 ? 2 : 1][kStageTile];  // their terms out of the units' range, by thread
-    if (LR == 1) own[0][threadIdx.x] = own[LR == 1 ? 1 : 0][threadIdx.x] = 0.0;
+    // one run: the block's rows of block_add_rows; the last two take the sums'
+    // terms out of the units' range, by thread
+    __shared__ double red[LR == 1 ? 6 : 1][kStageTile];
+    double *const own_old = &red[LR == 1 ? 4 : 0][threadIdx.x], *const own_died = &red[LR == 1 ? 5 : 0][threadIdx.x];
+    *own_old = *own_died = 0.0;
     double acc_hf[2] = {0.0, 0.0}, acc_en[2] = {0.0, 0.0}, acc_born[2] = {0.0, 0.0}, acc_ab[2] = {0.0, 0.0};
     double death_max = 0.0;  // max_death_cpt of this thread's determinants (tau search)
     unsigned long long acc_att = 0, acc_tomb = 0;
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
             flags = sr[W + L];
             core = st.n_core > 0 && is_core_flags(flags);
             NECI_FOR_RUNS(k, L) {
-                acc_old[L == 1 ? 0 : k].add(abs_dbl(C[k]), &own[0][threadIdx.x]);
+                acc_old[L == 1 ? 0 : k].add(abs_dbl(C[k]), own_old);
                 if (abs_bits(C[k]) >= dbl_bits(kEps12)) occ = true;
             }
             if (core) {
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
                 // there were) is handled below
                 const double aC = abs_dbl(C[k]);
                 const bool le = le_nonneg(idie, aC);
-                acc_died[L == 1 ? 0 : k].add(le ? idie : aC, &own[LR == 1 ? 1 : 0][threadIdx.x]);
+                acc_died[L == 1 ? 0 : k].add(le ? idie : aC, own_died);
                 if (!le) over = true;
                 // C - idie * sign(1, C) with Fortran's sign (+1 for C = -0.0); both products are exact
                 const bool nonneg = !(dbl_bits(C[k]) >> 63) || abs_bits(C[k]) == 0;
@@ -714,11 +717,11 @@ __global__ void __launch_bounds__(256, 4) k_sweep(DevSys s, DevState st, const I
         __shared__ BlockExact<2> exact;
         exact.warp_part(0, acc_old[0]);
         exact.warp_part(1, acc_died[0]);
-        const double v[6] = {acc_hf[0], acc_en[0], acc_born[0], acc_ab[0], own[0][threadIdx.x], own[LR == 1 ? 1 : 0][threadIdx.x]};
+        const double v[4] = {acc_hf[0], acc_en[0], acc_born[0], acc_ab[0]};
         double *const dst[6] = {&c->hf_cyc[0], &c->enum_cyc[0], &c->nborn[0], &c->naborted[0], &c->tot_parts_old[0], &c->ndied[0]};
-        block_add<6, 2>(v, dst, 2, u, du);  // (every place taken; its barriers are between the parts and the sums)
-        exact.add(0, 32, 0x1.0p-60, &c->tot_parts_old[0]);
-        exact.add(1, 64, 0x1.0p-76, &c->ndied[0]);
+        block_add_rows<4, 2, 2>(red, v, dst, 2, u, du);  // (every row taken; its barriers are between the parts and the sums)
+        exact.add(0, 32, 0x1.0p-70, &c->tot_parts_old[0]);
+        exact.add(1, 64, 0x1.0p-78, &c->ndied[0]);
     } else {
         const double v[12] = {acc_old[0].v, acc_old[L - 1].v, acc_hf[0], acc_hf[1], acc_en[0], acc_en[1], acc_died[0].v,
                               acc_died[L - 1].v, acc_born[0], acc_born[1], acc_ab[0], acc_ab[1]};
@@ -1522,10 +1525,10 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
     const bool rdm = LR == 2 && split && s.rdm && p.rdm_defer;
     SlotSum<LR, kUnitChange> a_born[L], a_rm[L];
     SlotSum<LR, kUnitAmplitude> a_tp[L];
-    __shared__ double own[LR == 1 ? 3 : 1][kStageTile];  // as in k_sweep
-    for (int i = 0; i < (LR == 1 ? 3 : 0); ++i) own[i][threadIdx.x] = 0.0;
-    double *const own_born = &own[0][threadIdx.x], *const own_rm = &own[LR == 1 ? 1 : 0][threadIdx.x],
-                 *const own_tp = &own[LR == 1 ? 2 : 0][threadIdx.x];
+    __shared__ double red[LR == 1 ? 6 : 1][kStageTile];  // as in k_sweep
+    double *const own_born = &red[LR == 1 ? 3 : 0][threadIdx.x], *const own_rm = &red[LR == 1 ? 4 : 0][threadIdx.x],
+                 *const own_tp = &red[LR == 1 ? 5 : 0][threadIdx.x];
+    *own_born = *own_rm = *own_tp = 0.0;
     double a_norm[2] = {0, 0}, a_ann[2] = {0, 0}, a_ab[2] = {0, 0};
     unsigned long long a_s[2] = {0, 0}, a_occ = 0, a_holes = 0, a_found = 0, a_tomb = 0;
     // Tiles staged into shared memory by TMA bulk copies as in k_sweep: the
@@ -1708,12 +1711,12 @@ __global__ void __launch_bounds__(256, 4) k_merge_stats(DevSys s, DevState st, c
         exact.warp_part(0, a_born[0]);
         exact.warp_part(1, a_rm[0]);
         exact.warp_part(2, a_tp[0]);
-        const double v[6] = {a_norm[0], a_ann[0], a_ab[0], *own_born, *own_rm, *own_tp};
+        const double v[3] = {a_norm[0], a_ann[0], a_ab[0]};
         double *const dst[6] = {&c->norm[0], &c->nannihil[0], &c->naborted[0], &c->nborn[0], &c->nremoved[0], &c->tot_parts[0]};
-        block_add<6, 6>(v, dst, 2, u, du);  // (every place taken; its barriers are between the parts and the sums)
-        exact.add(0, 32, 0x1.0p-76, &c->nborn[0]);
-        exact.add(1, 64, 0x1.0p-76, &c->nremoved[0]);
-        exact.add(2, 96, 0x1.0p-60, &c->tot_parts[0]);
+        block_add_rows<3, 3, 6>(red, v, dst, 2, u, du);  // (as in k_sweep)
+        exact.add(0, 32, 0x1.0p-78, &c->nborn[0]);
+        exact.add(1, 64, 0x1.0p-78, &c->nremoved[0]);
+        exact.add(2, 96, 0x1.0p-70, &c->tot_parts[0]);
     } else {
         const double v[12] = {a_born[0].v, a_born[L - 1].v, a_ann[0], a_ann[1], a_ab[0], a_ab[1], a_rm[0].v, a_rm[L - 1].v,
                               a_tp[0].v, a_tp[L - 1].v, a_norm[0], a_norm[1]};
@@ -1945,15 +1948,14 @@ __global__ void __launch_bounds__(256) k_rdm_freed(DevSys s, DevState st, const 
 // placement did not fill are holes.  A walker hash whose live entries and
 // tombstones pass 60% of the buckets is rebuilt between two calls (the host
 // is told in `reserved` of the record); within a call, past 65%, the next
-// step's k_final clears it and the sweep behind that refills it, when the call
-// has both.
-__device__ void final_record(const DevState &st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
-                            int advance_iter, long long n_core, int split) {
+// step's k_final clears it (cleared) and the sweep behind that refills it, when
+// the call has both.
+__device__ inline void final_record(const DevState &st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
+                                    int advance_iter, int cleared, long long n_core, int split) {
     Control *c = st.ctl;
     // (read together, before the first store)
     const long long next = pp->iter + 1, begin = pp->iter_begin, end = pp->iter_end;
     const int stop = c->halted, err = c->err;
-    const bool cleared = advance_iter && c->hash_clear;  // the walker hash, by this kernel
     const unsigned long long tomb = cleared ? 0ull : c->n_tomb;
     neci_gpu_iter_stats *out = base;
     if (advance_iter) {
@@ -2025,8 +2027,9 @@ __device__ void final_record(const DevState &st, neci_gpu_iter_stats *base, int 
 // idle launch.
 __global__ void __launch_bounds__(1024) k_final(DevState st, neci_gpu_iter_stats *base, int max_out, IterParams *pp,
                                                 int advance_iter, long long n_core, int split) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) final_record(st, base, max_out, pp, advance_iter, n_core, split);
-    if (!advance_iter || !st.ctl->hash_clear) return;
+    const int clear = advance_iter ? st.ctl->hash_clear : 0;  // (read before the record's stores)
+    if (blockIdx.x == 0 && threadIdx.x == 0) final_record(st, base, max_out, pp, advance_iter, clear, n_core, split);
+    if (!clear) return;
     uint4 *t = reinterpret_cast<uint4 *>(st.hash);
     for (unsigned long long b = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; b < st.hash_n / 4;
          b += (unsigned long long)gridDim.x * blockDim.x)
