@@ -790,10 +790,12 @@ def main():
     # sweep, spawn, compress, decide, place, merge, final; the probe unless the
     # spawn kernel does it; the core projection and the sum of its long rows;
     # for a short spawn list one kernel looks up and compresses and, up to 2e5
-    # records, one decides and places (a compaction, when a step leaves more
-    # holes than walkers, and a rebuild of the walker hash run between calls)
+    # records and 1.2e4 new determinants, one decides and places (a compaction,
+    # when a step leaves more holes than walkers, and a rebuild of the walker
+    # hash run between calls)
     launches_per_step = 7 + (2 if r["last"]["n_core"] > 0 else 0) + (0 if fused else 1)
-    launches_per_step -= (1 if gathered else 0) + (1 if r["last"]["n_spawned"] <= 200_000 else 0)
+    launches_per_step -= (1 if gathered else 0)
+    launches_per_step -= 1 if r["last"]["n_spawned"] <= 200_000 and r["last"]["n_new"] <= 12_000 else 0
     line = {
         "metric": METRIC, "value": updates / dev_s, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": 1000.0 * dev_s / args.steps, "higher_is_better": True,

@@ -844,12 +844,14 @@ int32_t neci_gpu_init_pchb(neci_gpu_ctx *ctx) {
 }
 
 // Whether the next steps take the annihilation's kernels of a short spawn list,
-// from the records of the last step, with a margin so that the choice does not
-// flap; before a context's first step, from its list: a step spawns about a
-// record for every second determinant (0.05 to 1 of them at n = 24 to 64).
-static void update_short_list(Engine &e, long long records) {
-    auto below = [&](bool now, long long line) { return records <= (now ? line : line - line / 4); };
-    const bool gather = below(e.gather, kGatherSpawns), small = below(e.short_list, kShortSpawns);
+// from the last step's records and new determinants, with a margin so that
+// the choice does not flap; before a context's first step, from its list: a
+// step spawns about a record for every second determinant (0.05 to 1 of them
+// at n = 24 to 64), and an eighth of the records make a new one (0.03 to 0.2).
+static void update_short_list(Engine &e, long long records, long long added) {
+    auto below = [](bool now, long long x, long long line) { return x <= (now ? line : line - line / 4); };
+    const bool gather = below(e.gather, records, kGatherSpawns);
+    const bool small = below(e.short_list, records, kShortSpawns) && below(e.short_list, added, kShortNew);
     if (gather != e.gather || small != e.short_list) {
         e.gather = gather;
         e.short_list = small;
@@ -936,7 +938,7 @@ int32_t neci_gpu_upload_walkers(neci_gpu_ctx *ctx, const int64_t *ilut, int64_t 
     CK(cudaStreamSynchronize(e.stream));
     e.compact_due = e.rehash_due = false;  // the list and its hash are new
     update_live_share(e, nrows, 0);
-    if (!e.stepped) update_short_list(e, nrows / 2);
+    if (!e.stepped) update_short_list(e, nrows / 2, nrows / 16);
     if (err) return fail(err, "upload: hash table full");
     return NECI_GPU_OK;
 }
@@ -1126,7 +1128,7 @@ static int run_steps(Engine &e, const neci_gpu_iter_params *p, int n_iter, neci_
         done += batch;
         update_fuse_probe(e, stats[done - 1]);
         update_merge_blocks(e, stats[done - 1]);
-        update_short_list(e, stats[done - 1].n_spawned);
+        update_short_list(e, stats[done - 1].n_spawned, stats[done - 1].n_new);
         e.stepped = true;
         update_live_share(e, stats[done - 1].tot_walkers, stats[done - 1].n_attempts);
         update_compact_due(e, stats[done - 1]);
@@ -1255,7 +1257,7 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         if (!first_err) {
             update_fuse_probe(e, e.h_stats[n_iter - 1]);
             update_merge_blocks(e, e.h_stats[n_iter - 1]);
-            update_short_list(e, e.h_stats[n_iter - 1].n_spawned);
+            update_short_list(e, e.h_stats[n_iter - 1].n_spawned, e.h_stats[n_iter - 1].n_new);
             e.stepped = true;
             update_live_share(e, e.h_stats[n_iter - 1].tot_walkers, e.h_stats[n_iter - 1].n_attempts);
             update_compact_due(e, e.h_stats[n_iter - 1]);

@@ -31,13 +31,23 @@ enum KernelId {
     K_NUM
 };
 
-// Spawn records of a step up to which its annihilation takes the kernels of a
-// short list, measured on both sides of the lines: lookup and compression in
-// one (k_ann_gather: 19 against 33 us at 1.5e5 records, 49 against 69 at
-// 3e5, 116 against 107 at 1.4e6), decision and placement in one (k_ann_new:
-// 26 against 39 us at 1.5e5 records, 90 against 60 at 3e5).
-constexpr long long kGatherSpawns = 600000;
+// Spawn records of a step, and of its new determinants, up to which its
+// annihilation takes the kernels of a short list.  Both save launches and
+// waits, and both put work into one kernel that the split form has beside the
+// merge sweep (compression) or at a better occupancy (placement), so the lines
+// are those of the step, in us with the split form and so:
+// lookup and compression in one (k_ann_gather): lattice with several couplings
+// 1.0e5 records 133 and 118, 2.6e5 266 and 258, 5.2e5 458 and 477; n = 39
+// 2.1e5 309 and 290, 4.2e5 496 and 502; n = 24 2.8e5 224 and 216, 5.5e5 365
+// and 374; 12-site ring 3.5e5 148 and 144, 6.8e5 235 and 234;
+// decision and placement in one (k_ann_new), beside k_ann_gather: ring 1.8e5
+// records and 5.9e3 new determinants 97.9 and 93.3; n = 32 replica pair 8.3e4
+// and 7.4e3 146 and 142; n = 39 1.0e5 and 1.2e4 177 and 179; n = 24 1.5e5 and
+// 1.6e4 135 and 136; n = 64 1.7e5 and 3.6e4 822 and 846; n = 39 2.1e5 and
+// 2.4e4 290 and 321.
+constexpr long long kGatherSpawns = 350000;
 constexpr long long kShortSpawns = 200000;
+constexpr long long kShortNew = 12000;
 
 struct Engine {
     neci_gpu_system desc{};

@@ -1318,7 +1318,7 @@ __global__ void __launch_bounds__(128) k_ann_place(DevSys s, DevState st, const 
 // The annihilation of a short spawn list in two kernels instead of four: a
 // step of up to some 1e5 records is bound by the latency of its kernels
 // (launch, first loads, reductions: 7 to 10 us each whatever they do), not by
-// their work (kGatherSpawns, kShortSpawns).
+// their work (kGatherSpawns, kShortSpawns, kShortNew).
 //   k_ann_gather  passes 1 and 2: each record is looked up in the walker hash;
 //                 the absent ones wait in shared memory until a warp has 32
 //                 (so that the merge has full lanes) and are merged per
