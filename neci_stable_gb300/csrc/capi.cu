@@ -1060,8 +1060,8 @@ static void update_merge_blocks(Engine &e, const neci_gpu_iter_stats &last) {
 // Compaction of the walker list runs between calls, before the first step
 // of a call whose last step left more holes than occupied slots (the rule
 // k_final applies to Control::compact; the compaction kernels check that
-// flag and ask for the rebuild of the walker hash, which the next step
-// does).  It is not part of the step graph: holes cost only sweep work, and
+// flag and ask for the rebuild of the walker hash, which is launched behind
+// them).  It is not part of the step graph: holes cost only sweep work, and
 // the five launches would do nothing in almost every step.
 static void update_compact_due(Engine &e, const neci_gpu_iter_stats &last) {
     e.compact_due = last.tot_walkers > 4ll * kCompactTile && 2 * last.holes_in_list > last.tot_walkers;
@@ -1231,8 +1231,8 @@ int32_t neci_gpu_iterate_batch(neci_gpu_ctx **ctxs, int32_t n_ctx, const neci_gp
         }
         e0.batch_key = key;
     }
-    // parameters in, record counters reset, then one launch per step; the
-    // whole batch runs in the first context's stream order
+    // parameters in, then one launch per step; the whole batch runs in the
+    // first context's stream order
     for (int c = 0; c < n_ctx; ++c) {
         Engine &e = ctxs[c]->e;
         CK(cudaMemcpyAsync(e.d_params, e.h_params, sizeof(IterParams), cudaMemcpyHostToDevice, e0.stream));

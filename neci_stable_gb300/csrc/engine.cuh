@@ -33,7 +33,9 @@ constexpr int kBigAttempts = NECI_BIG_ATTEMPTS;
 constexpr int kBigGranule = 128;  // attempts of heavy parents per entry of DevState::big_at
 constexpr int kBigShift = 36;     // Control::n_big: parents << kBigShift | their attempts (modulo 2^36: a step
                                   // whose n_attempts pass max_att, below 2^33, is refused before they are read)
-constexpr int kHugeAttempts = 1 << 16;  // at most kMaxHuge parents may have more attempts than this
+// A step with more than kMaxHuge parents past kHugeAttempts is refused
+// (SPAWN_FULL): a limit of the call, which nothing here is sized by.
+constexpr int kHugeAttempts = 1 << 16;
 constexpr int kMaxHuge = 4096;
 constexpr int kCompactTile = 1024;        // slots per block of the compaction scans
 constexpr int kProbeLimit = 1 << 16;
@@ -78,7 +80,7 @@ struct Control {
     int clear_next;                     // the next step's k_final clears the walker hash
     int hash_clear;                     // ... this step's does (set by its sweep)
     int rehash_fill;                    // the last step's k_final cleared it: this step's sweep refills it
-    int compact;                        // compact the walker list at the next step
+    int compact;                        // compact the walker list before the next call's first step
     unsigned long long compact_k;       // occupied slots kept by the compaction
     unsigned long long compact_pos_k;   // occupied slots below compact_k
     double nborn[2], ndied[2], nannihil[2], naborted[2], nremoved[2];

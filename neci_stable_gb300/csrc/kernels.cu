@@ -30,8 +30,8 @@
 //                  found branch + CalcHashTableStats (load_balancer.fpp:646)
 //                  in one sweep over the slots
 //   k_final        collect estimators into the step's stats record, reset the
-//                  per-step counters, clear the walker hash if its load is
-//                  high (the next sweep refills it)
+//                  per-step counters, clear the walker hash if its load was
+//                  high a step ago (the next sweep refills it)
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -104,8 +104,8 @@ __global__ void k_hash_done(DevState st) {
 }
 
 // ===========================================================================
-// Compaction of the walker list (run at the start of a step when the
-// previous one left more holes than occupied slots).  The K occupied slots
+// Compaction of the walker list (run between two calls when the last step
+// left more holes than occupied slots).  The K occupied slots
 // (or core slots) keep their order; those at or above K move into the holes
 // below K, the r-th of them into the r-th hole, so that slots 0..K-1 hold the
 // whole list.  TotWalkers becomes K and the walker hash is rebuilt.  Results
