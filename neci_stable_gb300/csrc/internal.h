@@ -31,8 +31,8 @@ enum KernelId {
     K_NUM
 };
 
-// Spawn records of a step, and of its new determinants, up to which its
-// annihilation takes the kernels of a short list.  Both save launches and
+// Spawn records and new determinants of a step up to which its annihilation
+// takes the kernels of a short list.  Both save launches and
 // waits, and both put work into one kernel that the split form has beside the
 // merge sweep (compression) or at a better occupancy (placement), so the lines
 // are those of the step, in us with the split form and so:
